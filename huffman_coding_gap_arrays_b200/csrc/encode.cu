@@ -3,46 +3,57 @@
 // Replaces cuencoder + cu_get_gaparray (encoder/src/encoder.cu:142-379) and
 // produces the same bitstream and gap array bit for bit.
 //
-// Work unit: a region (super-tile) of st_chunks x 8 KiB input bytes of one
-// job, taken by global id by persistent CTAs of 512 threads; the single-buffer
-// entry points run one job, the batched ones thousands, each with its own
-// codebook (the CTA reloads its code tables when the job changes).  Its bit count is one dot product of
-// its histogram (recorded by hist_st_kernel in the same pass that builds the
-// global histogram) with the code lengths, so a single bounded look-back over
-// super-tiles gives its first output bit G; no per-chunk look-back and no
-// waiting on neighbours afterwards.  A CTA claims its next super-tile one
-// ahead and publishes that one's bit count at once, so no look-back ever
-// waits on a claimed super-tile, and the input stream never drains between
-// super-tiles.
+// Work unit: a region (super-tile) of st_bytes input bytes of one job, taken
+// by global id by persistent CTAs of 16 warps; the single-buffer entry points
+// run one job, the batched ones thousands, each with its own codebook (the
+// CTA reloads its code table when the job changes).  A region's bit count is
+// one dot product of its histogram (recorded by hist_st_kernel in the same
+// pass that builds the global histogram) with the code lengths, so a single
+// bounded look-back over regions gives its first output bit G.  A CTA claims
+// its next region one ahead and publishes that one's bit count at once, so no
+// look-back ever waits on a claimed region.
 //
-// Input: chunks are staged in a ring of kRing shared-memory buffers by 1-D
-// bulk copies (TMA engine, completion on an mbarrier), issued by one thread
-// kRing chunks ahead of the one being encoded: 48 KiB per SM in flight, which
-// a one-load-per-thread register prefetch cannot reach.
+// Input: steps of 16 KiB are staged in a ring of shared-memory buffers by 1-D
+// bulk copies (completion on an mbarrier), one step ahead of the one being
+// encoded.  In a step every warp owns 1 KiB and every lane 32 consecutive
+// bytes.
 //
-// Per chunk:
-//   * lookups in a 32-way lane-replicated codeword table ([byte][lane]: each
-//     lane reads its own bank, never a conflict);
-//   * one block scan of per-thread bit counts (warp scan + 16 warp totals);
-//   * packing two codes at a time (<= 32 bits) into a shared image of the
-//     output words, indexed from the segment-aligned word below the chunk's
-//     first bit, so the image's 16-byte groups are the output's 16-byte
-//     groups; every completed word is OR-ed in with a shared atomic (the
-//     image is clear when a chunk starts, so for a word no neighbour shares
-//     the OR is a store, and one path without a first-word flag measured 7 %
-//     faster than plain stores plus an atomic for the shared word);
-//   * a gap entry falls out of word completion: the code completing global
-//     word w with w % 4 == 3 ends segment w/4 and its spill into the next
-//     word is that segment's entry (encoder/src/encoder.cu:307-312); each
-//     segment has exactly one such code, so entries are plain byte stores;
-//   * complete words go out with 16-byte coalesced stores, and each group of
-//     the image is cleared right after it is read; the partial last word and
-//     gap word are carried to the next chunk.  Two barriers per chunk.
-// The super-tile's first partial word and gap word also hold bits of the
-// previous super-tile; one warp rebuilds those by re-encoding at most 1023
-// bits backwards from G (the predecessor's last bytes), so neighbouring
-// super-tiles never wait on each other.  The output needs no pre-zeroing (the
-// reference memsets it, encoder.cu:412-414) and no global atomics.
+// The kernel is bound by instruction issue (8-bit symbols, integer work only),
+// so the loop is built to spend few instructions per byte:
+//   * one 8-byte lookup per byte, {left-aligned code, length}, from a table
+//     replicated over 16 lanes ([byte][lane & 15]: a half-warp's 8-byte reads
+//     each have their own bank pair);
+//   * codes are joined without branches, two to a word and four to a 64-bit
+//     piece, before their place in the output is known; the running lengths of
+//     the piece's four codes ride in one register, a byte each (multiply-adds,
+//     on the pipe that the shifts leave idle);
+//   * one barrier per step: each warp publishes its bit count and its last 32
+//     code bits, and then knows where its own bits start and what the word it
+//     starts in holds already, so it packs, and writes, its words alone: no
+//     word is shared between warps;
+//   * in the warp, a lane stores the words it completes with plain shared
+//     stores (32 bytes are at least 32 bits: no word sees three lanes) and
+//     ORs its unfinished last word into the next lane's first;
+//   * a piece that reaches a segment's end leaves its four running lengths,
+//     minus the distance to that end, in a ring of records indexed by segment:
+//     the first byte with its top bit set is the spill of the code that ends
+//     or crosses there, which is the segment's gap entry
+//     (encoder/src/encoder.cu:307-312).  One step later the records become gap
+//     words, one thread to a word of eight entries.
+// Bytes outside the job in a warp at one of its ends are encoded with the rest
+// and masked off again, so there is one packing loop; a warp whose bits do not
+// fit its image (over 10 bits a byte) packs its two halves one after the other.
+// Nothing is pre-zeroed (the reference memsets its outputs, encoder.cu:412-414)
+// and there are no global atomics: a region's first word is completed by
+// re-encoding the bits before G, and its first gap byte likewise, so
+// neighbouring regions never wait on each other.
+//
+// Measured (B200, kernel alone), against a loop that packed two codes at a time
+// into one image of the CTA with two barriers per 8 KiB: 256 MiB of Zipf(1.2)
+// 344 -> 237 us, of the mixed stream 409 -> 243, of BF16 sign|mantissa bytes
+// 353 -> 282, of BF16 exponents 335 -> 234; 1024 buffers of 4 KiB - 4 MiB
+// (593 MB) in 64 KiB regions 879 -> 654 us, in 256 KiB regions 791 -> 568.
+// 0.73 warp instructions per byte (1.12 before) at 71 % of the issue slots.
 #include <cuda_runtime.h>
 
 #include "device_util.cuh"
@@ -51,16 +62,45 @@
 namespace hgap {
 
 constexpr int kEncThreads = 512;
-constexpr int kEncBpt = 16;
 constexpr int kEncWarps = kEncThreads / 32;
-static_assert(kEncThreads * kEncBpt == kEncChunkBytes, "chunk = threads x bytes per thread");
-constexpr int kRing = 3;                                  // input chunks staged ahead
-constexpr int kImgWords = kEncChunkBytes * 16 / 32 + 16;  // <= 16 bits per byte, + carry/alignment
-constexpr int kLutWords = 256 * 32;
-// two lane-replicated tables (left-aligned codes, lengths), the input ring,
-// the output image and one spill byte per image word
-constexpr size_t kEncSmem =
-    (size_t)2 * kLutWords * 4 + (size_t)kRing * kEncChunkBytes + (size_t)kImgWords * 4 + kImgWords;
+constexpr int kLaneBytes = 32;                        // input bytes per lane and step
+constexpr int kPieces = kLaneBytes / 4;               // 64-bit pieces of four codes per lane
+constexpr int kWarpBytes = 32 * kLaneBytes;
+constexpr int kStepBytes = kEncWarps * kWarpBytes;    // 16 KiB
+static_assert(kEncChunkBytes % kWarpBytes == 0, "a region ends on a warp's boundary");
+constexpr int kRing = 2;                              // input steps staged
+constexpr int kLutRep = 16;                           // table copies: one per lane of a half-warp
+// Output words a warp packs at once (a multiple of 4): 10.4 bits per byte, and enough for half a
+// warp's bytes at 16; 16 warps' images, the table, the ring and the records fit twice in an SM.
+// The first words are slack: the up to 15 bytes before a job's first one (its 16-byte group) are
+// encoded too, below its first bit, and never written out.
+constexpr int kImgWords = 348;
+constexpr uint32_t kSlackBits = 256;
+static_assert(kSlackBits >= 15 * kMaxLen && kSlackBits % 128 == 0, "room for 15 codes, whole segments");
+constexpr uint32_t kLaneMaxBits = kLaneBytes * kMaxLen;
+static_assert(kImgWords % 4 == 0 && kImgWords * 32 > kSlackBits + 128 + 17 * kLaneMaxBits,
+              "half a warp fits, with as much again as a lane's bytes after the job's last");
+// gap records: a step closes at most 16 KiB * 16 bits / 128 = 2048 segments, and the records of
+// two steps are live at once
+constexpr uint32_t kRecs = 4096;
+constexpr size_t kEncSmem = (size_t)256 * kLutRep * 8 + (size_t)kRing * kStepBytes +
+                            (size_t)kEncWarps * kImgWords * 4 + (size_t)kRecs * 4;
+constexpr uint32_t kLen4 = 0x01010101u;
+constexpr uint32_t kPieceBias = 0x7f7f7f7fu;  // 0x7f + running length per byte
+
+// What the steps of a region need of it, in shared memory.  Bit positions are
+// 32-bit, relative to the start of the gap word (1024 bits, so also of the
+// 16-byte group of output words) that holds the region's first bit; a region
+// has at most 2^22 bits.
+struct Region {
+    uint32_t* bits;             // output and gap words from there on,
+    uint32_t* gaps;
+    uint32_t nwords, ngaps;     // and how many of them exist
+    uint32_t first_bit;         // the region's first bit
+    uint32_t lo, hi;            // its bytes: [lo, hi) from a multiple of 16
+    bool first, last;           // in its job
+    bool vec;                   // output words are 16-byte aligned
+};
 
 struct EncShared {
     uint64_t mbar[kRing];       // one per ring buffer: its bulk copy landed
@@ -69,14 +109,17 @@ struct EncShared {
     uint64_t agg[2];            // their bit counts
     uint32_t job_id[2];
     uint64_t G;                 // first output bit of the current region
-    uint32_t warp_tot[kEncWarps];
-    uint32_t carry;             // partial output word carried into the next chunk
-    uint32_t gcarry[2];         // partial gap word carried, by chunk parity
+    Region reg;
+    uint32_t gap_head;          // spill at the segment end before G (for a first entry that is odd)
+    uint32_t tot[2][kEncWarps]; // per step parity: the warps' bit counts
+    // the last 32 code bits before warp w's first of step c, at [(16 c + w) % 64]: four steps, since
+    // warp 0 still reads its entry when warp 15 is a step further
+    uint32_t tail[4 * kEncWarps];
     uint64_t nitems;            // regions of the launch
-    uint32_t lut_job;           // job whose code tables are in the LUTs
+    uint32_t lut_job;           // job whose codes are in the table
     uint32_t abort;
-    uint32_t p_issued;          // producer: copies issued so far (chunk sequence number)
-    uint32_t p_chunk;           // producer: chunk index of the next copy within its region
+    uint32_t p_issued;          // producer: copies issued so far (step sequence number)
+    uint32_t p_step;            // producer: step index of the next copy within its region
     int p_which;                // producer: next copy from the current region (0) or the next one (1)
 };
 
@@ -89,7 +132,7 @@ __device__ __forceinline__ void code_of(const EncTable* t, uint32_t byte, uint32
 
 // Warp 0: claims a region into `slot`, copies its job there and publishes
 // its bit count at once, so that no later region's look-back waits on it.
-__device__ __forceinline__ void claim_region(const EncArgs& a, const uint32_t* lutl, EncShared& sh, int slot,
+__device__ __forceinline__ void claim_region(const EncArgs& a, const uint2* lut, EncShared& sh, int slot,
                                              uint32_t lane) {
     uint32_t c = 0;
     if (lane == 0) c = atomicAdd(a.counter, 1u);
@@ -104,12 +147,16 @@ __device__ __forceinline__ void claim_region(const EncArgs& a, const uint32_t* l
         if (lane < sizeof(EncJob) / 8)
             reinterpret_cast<uint64_t*>(&sh.job[slot])[lane] = reinterpret_cast<const uint64_t*>(src)[lane];
         uint64_t part = 0;
+        bool absent = false;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const uint32_t b = lane + 32 * j;
-            const uint32_t len = a.jobs ? ((a.tables[job].e[b] >> 16) & 31u) : (lutl[b << 5] & 31u);
-            part += (uint64_t)a.st_hist[item * 256 + b] * len;
+            const uint32_t len = a.jobs ? ((a.tables[job].e[b] >> 16) & 31u) : lut[b * kLutRep].y;
+            const uint32_t n = a.st_hist[item * 256 + b];
+            absent |= n != 0 && len == 0;
+            part += (uint64_t)n * len;
         }
+        if (absent) atomicOr(a.status, kDevNoCode);
         agg = warp_sum_u64(part);
         if (lane == 0 && item + 1 != a.hook.hold_plus1) lookback_publish(a.st_rec, item, agg, item == src->item0);
     }
@@ -121,20 +168,24 @@ __device__ __forceinline__ void claim_region(const EncArgs& a, const uint32_t* l
     __syncwarp();
 }
 
-__device__ __forceinline__ uint32_t st_chunks(const EncJob& J, uint64_t st) {
-    const uint64_t v0 = st * (uint64_t)J.st_bytes;
-    const uint64_t v1 = (v0 + J.st_bytes < J.hi) ? v0 + J.st_bytes : J.hi;
-    return (uint32_t)((v1 - v0 + kEncChunkBytes - 1) / kEncChunkBytes);
+// End of region st of job J (virtual input index, like J.lo / J.hi).
+__device__ __forceinline__ uint64_t region_end(const EncJob& J, uint64_t st) {
+    const uint64_t v1 = (st + 1) * (uint64_t)J.st_bytes;
+    return v1 < J.hi ? v1 : J.hi;
+}
+
+__device__ __forceinline__ uint32_t region_steps(const EncJob& J, uint64_t st) {
+    return (uint32_t)((region_end(J, st) - st * (uint64_t)J.st_bytes + kStepBytes - 1) / kStepBytes);
 }
 
 // The bulk-copy producer: thread 0 at region boundaries, the last warp's first
-// thread after each chunk's second barrier (never both at once; barriers order
-// them).  Copies go out in the order the CTA encodes chunks: the rest of the
-// current region, then the claimed next one; at most kRing beyond the last
-// chunk whose buffer is free again.  Its state lives in shared memory (one
-// thread touches it at a time), sparing every thread the registers.
+// thread after each step's barrier (never both at once; barriers order them).
+// Copies go out in the order the CTA encodes steps: the rest of the current
+// region, then the claimed next one; at most kRing beyond the last step whose
+// buffer is free again.  Its state lives in shared memory (one thread touches
+// it at a time), sparing every thread the registers.
 __device__ __forceinline__ void produce(const EncArgs& a, uint8_t* ring, EncShared& sh, uint32_t freed, int cur_slot) {
-    uint32_t issued = sh.p_issued, pc = sh.p_chunk;
+    uint32_t issued = sh.p_issued, ps = sh.p_step;
     int which = sh.p_which;
     while (issued < freed + kRing) {
         const int slot = cur_slot ^ which;
@@ -142,48 +193,135 @@ __device__ __forceinline__ void produce(const EncArgs& a, uint8_t* ring, EncShar
         if (item >= sh.nitems) break;
         const EncJob& J = sh.job[slot];
         const uint64_t st = item - J.item0;
-        if (pc >= st_chunks(J, st)) {
+        if (ps >= region_steps(J, st)) {
             if (which == 0) {
                 which = 1;
-                pc = 0;
+                ps = 0;
                 continue;
             }
             break;  // wait for the next claim
         }
-        const uint64_t v = st * (uint64_t)J.st_bytes + (uint64_t)pc * kEncChunkBytes;
-        const uint64_t rem = ((J.hi + 15) & ~15ull) - v;  // through the end of the last 16-byte group
-        const uint32_t bytes = rem >= (uint64_t)kEncChunkBytes ? (uint32_t)kEncChunkBytes : (uint32_t)rem;
+        const uint64_t v = st * (uint64_t)J.st_bytes + (uint64_t)ps * kStepBytes;
+        const uint64_t rem = ((region_end(J, st) + 15) & ~15ull) - v;  // through the last 16-byte group
+        const uint32_t bytes = rem >= (uint64_t)kStepBytes ? (uint32_t)kStepBytes : (uint32_t)rem;
         const uint32_t s = issued % kRing;
-        bulk_load(ring + (size_t)s * kEncChunkBytes, J.in_aligned + v, bytes, &sh.mbar[s]);
+        bulk_load(ring + (size_t)s * kStepBytes, J.in_aligned + v, bytes, &sh.mbar[s]);
         ++issued;
-        ++pc;
+        ++ps;
     }
     sh.p_issued = issued;
-    sh.p_chunk = pc;
+    sh.p_step = ps;
     sh.p_which = which;
+}
+
+// A lane's 32 bytes as eight 64-bit pieces of four codes, left-aligned in
+// hi:lo; byte b of q is 0x7f + the bits of the piece's first b + 1 codes.
+struct Pieces {
+    uint32_t hi[kPieces], lo[kPieces], q[kPieces];
+};
+
+__device__ __forceinline__ uint32_t piece_bits(uint32_t q) { return (q >> 24) - 0x7fu; }
+
+// One input word (four bytes) to a piece.  `lane8`: the lane's byte offset in a
+// table row.
+__device__ __forceinline__ void join_piece(const uint2 (&e)[4], uint32_t& hi, uint32_t& lo, uint32_t& q) {
+    // lengths are at most 16: a pair has at most 32 bits, and shifts by a pair's length clamp at 32
+    const uint32_t c01 = e[0].x | __funnelshift_r(e[1].x, 0u, e[0].y);
+    const uint32_t c23 = e[2].x | __funnelshift_r(e[3].x, 0u, e[2].y);
+    const uint32_t l01 = e[0].y + e[1].y;
+    hi = c01 | __funnelshift_rc(c23, 0u, l01);
+    lo = __funnelshift_rc(0u, c23, l01);
+    q = e[3].y * 0x01000000u + (e[2].y * 0x01010000u + (e[1].y * 0x01010100u + (e[0].y * kLen4 + kPieceBias)));
+}
+
+__device__ __forceinline__ void make_piece(const char* lut, uint32_t lane8, uint32_t w, uint32_t& hi, uint32_t& lo,
+                                           uint32_t& q) {
+    uint2 e[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t b = __byte_perm(w, 0, 0x4440 + k);
+        e[k] = *reinterpret_cast<const uint2*>(lut + (b * (kLutRep * 8) + lane8));
+    }
+    join_piece(e, hi, lo, q);
+}
+
+// Bits of the lane's first i bytes (i <= 32).
+__device__ __forceinline__ uint32_t bits_before(const Pieces& pc, uint32_t i) {
+    uint32_t n = 0;
+#pragma unroll
+    for (int j = 0; j < kPieces; ++j) {
+        const uint32_t m = i > 4u * j ? (i - 4 * j < 4 ? i - 4 * j : 4u) : 0u;  // of piece j's four codes
+        if (m) n += ((pc.q[j] >> (8 * m - 8)) & 0xffu) - 0x7fu;
+    }
+    return n;
+}
+
+// The last 32 bits of the lane's codes, right-aligned (all of them if fewer).
+__device__ __forceinline__ uint32_t last_bits(const Pieces& pc) {
+    // a piece's low 32 bits are hi:lo >> (64 - l), its bits in hi alone if l <= 32
+    auto low = [](uint32_t hi, uint32_t lo, uint32_t l) {
+        return l > 32 ? __funnelshift_r(lo, hi, 64 - l) : __funnelshift_rc(hi, 0u, 32 - l);
+    };
+    uint32_t n = piece_bits(pc.q[kPieces - 1]);
+    uint32_t tail = low(pc.hi[kPieces - 1], pc.lo[kPieces - 1], n);
+#pragma unroll
+    for (int j = kPieces - 2; j >= 0; --j) {
+        const uint32_t l = piece_bits(pc.q[j]);
+        tail |= __funnelshift_lc(0u, low(pc.hi[j], pc.lo[j], l), n);  // (shifted out where n >= 32)
+        n += l;
+        if (j < kPieces - 2 && n >= 32) break;  // two more pieces nearly always do
+    }
+    return tail;
+}
+
+// Packs the lane's pieces from bit p of the warp's image on (image bit
+// kSlackBits = the start of the segment that the warp's first bit is in).
+// `cur` is what the lane's first word holds before p; stores every word
+// completed, returns the unfinished last one, and the end bit in p.  Every
+// segment end reached leaves a record (see the top): they are indexed by
+// segment, rec0 = 4 * (the segment of image bit 0, minus 1).
+__device__ __forceinline__ uint32_t pack(const Pieces& pc, uint32_t* img, char* recs, uint32_t rec0, uint32_t& p,
+                                         uint32_t cur) {
+    uint32_t a = p >> 5;
+#pragma unroll
+    for (int j = 0; j < kPieces; ++j) {
+        const uint32_t q = pc.q[j];
+        const uint32_t x = q - (~p & 127u) * kLen4;  // per byte: 0x80 + running length - distance to the segment's end
+        const uint32_t x0 = cur | __funnelshift_r(pc.hi[j], 0u, p);
+        const uint32_t x1 = __funnelshift_r(pc.lo[j], pc.hi[j], p);
+        const uint32_t x2 = __funnelshift_r(0u, pc.lo[j], p);
+        p += piece_bits(q);
+        const uint32_t b = p >> 5;
+        if (b != a) img[a] = x0;
+        if (b > a + 1) img[a + 1] = x1;
+        cur = b == a ? x0 : b == a + 1 ? x1 : x2;
+        if ((int32_t)x < 0) *reinterpret_cast<uint32_t*>(recs + ((b + rec0) & (4 * kRecs - 4))) = x;
+        a = b;
+    }
+    return cur;
 }
 
 __global__ void __launch_bounds__(kEncThreads, 2)
     encode_kernel(const __grid_constant__ EncArgs a, const __grid_constant__ EncTable tab) {
-    extern __shared__ __align__(16) uint32_t smem[];
-    uint32_t* lutc = smem;                // [byte][lane]: code << (32 - len)
-    uint32_t* lutl = smem + kLutWords;    // [byte][lane]: len (0x200 if absent)
-    uint8_t* ring = reinterpret_cast<uint8_t*>(smem + 2 * kLutWords);  // kRing input chunks
-    uint32_t* img = reinterpret_cast<uint32_t*>(ring + (size_t)kRing * kEncChunkBytes);
-    uint8_t* spills = reinterpret_cast<uint8_t*>(img + kImgWords);     // per image word
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint2* lut = reinterpret_cast<uint2*>(smem);                       // [byte][lane & 15]: {code << (32 - len), len}
+    uint8_t* ring = smem + (size_t)256 * kLutRep * 8;                  // kRing input steps
+    uint32_t* img_all = reinterpret_cast<uint32_t*>(ring + (size_t)kRing * kStepBytes);
+    uint32_t* recs = img_all + kEncWarps * kImgWords;                  // gap records, by segment
     __shared__ EncShared sh;
 
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    auto load_luts = [&](const EncTable& t) {
-        for (int i = tid; i < kLutWords; i += kEncThreads) {
-            const uint32_t e = t.e[i >> 5];
+    const uint32_t lane8 = (lane & (kLutRep - 1)) * 8;
+    uint32_t* const img = img_all + warp * kImgWords;                  // this warp's output words
+    auto load_lut = [&](const EncTable& t) {
+        for (int i = tid; i < 256 * kLutRep / 2; i += kEncThreads) {  // two copies a store
+            const uint32_t e = t.e[i / (kLutRep / 2)];
             const uint32_t l = (e >> 16) & 31u;
-            lutc[i] = l ? (e & 0xffffu) << (32 - l) : 0u;
-            lutl[i] = (e == kEncAbsent) ? 0x200u : l;
+            const uint32_t c = l ? (e & 0xffffu) << (32 - l) : 0u;
+            reinterpret_cast<uint4*>(lut)[i] = make_uint4(c, l, c, l);
         }
     };
-    if (!a.jobs) load_luts(tab);
-    for (int i = tid; i < kImgWords; i += kEncThreads) img[i] = 0;
+    if (!a.jobs) load_lut(tab);
     if (tid == 0) {
         // single path: the histograms in the workspace must come from this very input
         sh.abort = a.tag && (a.tag[0] != a.single.hi - a.single.lo ||
@@ -192,7 +330,7 @@ __global__ void __launch_bounds__(kEncThreads, 2)
         sh.lut_job = a.jobs ? ~0u : 0u;
         sh.nitems = a.nitems_dev ? *a.nitems_dev : a.nitems;
         sh.p_issued = 0;
-        sh.p_chunk = 0;
+        sh.p_step = 0;
         sh.p_which = 0;
         for (int s = 0; s < kRing; ++s) mbar_init(&sh.mbar[s], 1);
         mbar_init_fence();
@@ -201,10 +339,10 @@ __global__ void __launch_bounds__(kEncThreads, 2)
     if (sh.abort) return;
 
     int cur_slot = 0;   // slot of the current region; the next one is in cur_slot ^ 1
-    uint32_t cons = 0;  // chunks consumed so far (the ring's sequence number)
+    uint32_t cons = 0;  // steps consumed so far (the ring's sequence number)
     if (warp == 0) {
-        claim_region(a, lutl, sh, 0, lane);
-        if (sh.item[0] < sh.nitems) claim_region(a, lutl, sh, 1, lane);
+        claim_region(a, lut, sh, 0, lane);
+        if (sh.item[0] < sh.nitems) claim_region(a, lut, sh, 1, lane);
         else if (lane == 0) sh.item[1] = ~0ull;
         if (lane == 0) produce(a, ring, sh, 0, 0);
     }
@@ -217,27 +355,27 @@ __global__ void __launch_bounds__(kEncThreads, 2)
         const uint32_t jid = sh.job_id[cur_slot];
         const uint64_t st = item - J.item0;  // region within the job
 
-        // ---- warp 0: G of the current region, bits before G ---------------------
+        // ---- warp 0: G of the current region, what precedes G in its word and gap byte ----
         if (warp == 0) {
             const uint64_t G =
                 J.bit0 + lookback_resolve<4>(a.st_rec, item, sh.agg[cur_slot], st == 0, a.status, lane,
                                              wait_limit(a.hook), item + 1 != a.hook.hold_plus1);
-            uint32_t head = 0, gcarry = 0;
+            uint32_t head = 0, gap_head = 0;
             const uint32_t r = (uint32_t)(G & 31);
-            const uint32_t nibs = (uint32_t)((G >> 7) & 7);
-            if (G > 0 && (r != 0 || nibs != 0)) {
+            const bool odd = ((G >> 7) & 1) != 0;
+            if (G > 0 && (r != 0 || odd)) {
                 // walk the previous region's codes backwards from G
-                const uint64_t wstart = G - r;
-                const uint64_t gs = (G >> 10) << 10;
+                const uint64_t wstart = G - r;              // the word's first bit
+                const uint64_t bnd = G & ~127ull;           // the segment end at or before G
                 // codes starting at or below `stop` can no longer reach the head
-                // word (bits >= wstart) nor cross a boundary >= gs + 128
+                // word (bits >= wstart) nor cross or end at bnd
                 uint64_t stop = r ? wstart : ~0ull;
-                if (nibs && gs + 127 < stop) stop = gs + 127;
+                if (odd && bnd - 1 < stop) stop = bnd - 1;
                 uint64_t end = G;
                 const uint64_t vfirst = st * (uint64_t)J.st_bytes;  // first byte of this region
-                // 32 bytes a step, one per lane, going backwards; the bytes of kWalkAhead
-                // steps are loaded at once (one memory round trip, not one per step)
-                constexpr int kWalkAhead = 4;
+                // 32 bytes a round, one per lane, going backwards; the bytes of kWalkAhead
+                // rounds are loaded at once (one memory round trip, not one per round)
+                constexpr int kWalkAhead = 2;
                 for (uint64_t base0 = 0;; base0 += 32 * kWalkAhead) {
                     uint32_t pre[kWalkAhead];
 #pragma unroll
@@ -252,12 +390,12 @@ __global__ void __launch_bounds__(kEncThreads, 2)
                         if (done) break;
                         uint32_t c = 0, len = 0;
                         if (pre[k] < 0x100u) {
-                            const uint32_t byte = pre[k];
                             if (a.jobs) {
-                                code_of(a.tables + jid, byte, c, len);
+                                code_of(a.tables + jid, pre[k], c, len);
                             } else {
-                                c = lutc[(byte << 5) | lane];
-                                len = lutl[(byte << 5) | lane] & 31u;
+                                const uint2 e = lut[pre[k] * kLutRep + (lane & (kLutRep - 1))];
+                                c = e.x;
+                                len = e.y;
                             }
                         }
                         const uint32_t incl = warp_incl_scan(len, lane);
@@ -266,194 +404,229 @@ __global__ void __launch_bounds__(kEncThreads, 2)
                         if (len) {
                             if (r && ce > wstart)  // the code's right-aligned value, placed to end at ce
                                 head |= (uint32_t)(((uint64_t)(c >> (32 - len))) << (wstart + 32 - ce));
-                            const uint64_t b = (ce >> 7) << 7;   // last segment boundary <= end
-                            if (nibs && b > cs && b >= gs + 128)
-                                gcarry |= (uint32_t)(ce - b) << (4 * (uint32_t)(((b >> 7) - 1) & 7));
+                            if (odd && cs < bnd && bnd <= ce) gap_head = (uint32_t)(ce - bnd);
                         }
                         const uint32_t total = __shfl_sync(kFull, incl, 31);
-                        const uint64_t smin = end - total;  // start of the step's last code
-                        end = smin;
-                        if (smin <= stop || total == 0) done = true;
+                        end -= total;  // start of the round's last code
+                        if (end <= stop || total == 0) done = true;
                     }
                     if (done) break;
                 }
                 head = __reduce_or_sync(kFull, head);
-                gcarry = __reduce_or_sync(kFull, gcarry);
+                gap_head = __reduce_or_sync(kFull, gap_head);
             }
             if (lane == 0) {
+                const uint64_t base = G & ~1023ull, vfirst = st * (uint64_t)J.st_bytes;
+                auto room = [](uint64_t total, uint64_t from) {
+                    return total <= from ? 0u : total - from < 0x40000000ull ? (uint32_t)(total - from) : 0x40000000u;
+                };
                 sh.G = G;
-                sh.carry = head;  // 0 unless G % 32 != 0
-                sh.gcarry[cons & 1] = gcarry;
+                sh.tail[(cons * kEncWarps) % (4 * kEncWarps)] = r ? head >> (32 - r) : 0u;
+                sh.gap_head = gap_head;
+                Region& R = sh.reg;
+                R.bits = J.bits + (base >> 5);
+                R.gaps = J.gaps + (base >> 10);
+                R.nwords = room(J.words, base >> 5);
+                R.ngaps = room(J.gap_words, base >> 10);
+                R.first_bit = (uint32_t)(G - base);
+                R.lo = st == 0 ? (uint32_t)J.lo : 0u;
+                R.hi = (uint32_t)(region_end(J, st) - vfirst);
+                R.first = st == 0;
+                R.last = st + 1 == J.nst;
+                R.vec = J.bits_aligned16 != 0;
             }
         }
-        // batched: the job's code tables into the LUTs (the previous region is done with them)
-        if (a.jobs && jid != sh.lut_job) load_luts(a.tables[jid]);
+        // batched: the job's codes into the table (the previous region is done with it)
+        if (a.jobs && jid != sh.lut_job) load_lut(a.tables[jid]);
         __syncthreads();
         if (tid == 0) sh.lut_job = jid;
-        uint64_t P = sh.G;
-
-        // ---- stream the chunks --------------------------------------------------
-        const uint32_t nchunks = st_chunks(J, st);
-        uint64_t v0 = st * (uint64_t)J.st_bytes + (uint64_t)tid * kEncBpt;  // this thread's first byte
+        const Region& R = sh.reg;
+        uint32_t P = R.first_bit;      // first bit of the step
+        uint32_t gnext = 0;            // next gap word to write
         bool overflow = false;
-        for (uint32_t c = 0; c < nchunks; ++c, ++cons, v0 += kEncChunkBytes) {
-            const uint32_t stage = cons % kRing;
-            mbar_wait(&sh.mbar[stage], (cons / kRing) & 1, a.status, true);
-            const uint4 q = *reinterpret_cast<const uint4*>(ring + (size_t)stage * kEncChunkBytes + tid * 16);
 
-            // lookups: left-aligned code and length per byte, bit count per thread
-            const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
-            uint32_t cc[kEncBpt], ll[kEncBpt];
-            uint32_t nbits = 0;
-            if (v0 >= J.lo && v0 + kEncBpt <= J.hi) {
+        // Gap word g from the records of the region's segments before k_end; `bytes` of it: all
+        // four, or, where the region ends inside it, those whose two entries are known.  A region's
+        // first byte takes its even entry from gap_head; bytes before that belong to the previous
+        // region (the job's first region writes them: entries of no segment are 0).
+        auto emit_gap = [&](uint32_t g, uint32_t k_end, uint32_t bytes) {
+            const uint4* r4 = reinterpret_cast<const uint4*>(recs + ((8 * g) & (kRecs - 1)));
+            const uint4 r0 = r4[0], r1 = r4[1];
+            const uint32_t rr[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+            const uint32_t lo = g == 0 ? R.first_bit >> 7 : 0u;  // first segment that ends in the region
+            const uint32_t hi = k_end - 8 * g < 8 ? k_end - 8 * g : 8u;
+            uint32_t v = 0;
 #pragma unroll
-                for (int k = 0; k < kEncBpt; ++k) {
-                    const uint32_t w = w4[k >> 2];
-                    const int s8 = 8 * (k & 3);
-                    const uint32_t idx = ((s8 >= 5 ? (w >> (s8 - 5)) : (w << 5)) & 0x1fe0u) | lane;
-                    cc[k] = lutc[idx];
-                    ll[k] = lutl[idx];
-                    nbits += ll[k];
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < kEncBpt; ++k) {
-                    const uint32_t idx = (((w4[k >> 2] >> (8 * (k & 3))) & 0xffu) << 5) | lane;
-                    const bool in = v0 + k >= J.lo && v0 + k < J.hi;
-                    cc[k] = in ? lutc[idx] : 0u;
-                    ll[k] = in ? lutl[idx] : 0u;
-                    nbits += ll[k];
-                }
+            for (uint32_t i = 0; i < 8; ++i) {
+                // the first byte with its top bit set: 0x80 + the spill of the code that reached the end
+                const uint32_t s = (__ffs(rr[i] & 0x80808080u) - 8) & 31;
+                v |= ((rr[i] >> s) & 0xfu) << (4 * i);
             }
-            if (nbits >= 0x200u) {  // an absent byte adds 0x200 to the (< 0x200) bit count
-                atomicOr(a.status, kDevNoCode);
-                nbits &= 0x1ffu;
+            v &= (hi == 8 ? ~0u : (1u << (4 * hi)) - 1u) & (~0u << (4 * lo));
+            if (lo & 1u) v |= sh.gap_head << (4 * (lo - 1));
+            const uint32_t b0 = R.first ? 0u : lo >> 1;
+            if (g >= R.ngaps) {
+                overflow = true;
+            } else if (b0 == 0 && bytes == 4) {
+                R.gaps[g] = v;
+            } else {
+                uint8_t* const out = reinterpret_cast<uint8_t*>(R.gaps + g);
+#pragma unroll 1
+                for (uint32_t b = b0; b < bytes; ++b) out[b] = (uint8_t)(v >> (8 * b));
+            }
+        };
+
+        // ---- stream the steps ---------------------------------------------------
+        uint32_t off = warp * (uint32_t)kWarpBytes;              // the warp's first byte in the region
+        for (const uint32_t nsteps_end = cons + (R.hi + kStepBytes - 1) / kStepBytes; cons != nsteps_end;
+             ++cons, off += kStepBytes) {
+            const uint32_t stage = cons % kRing, par = cons & 1;
+            mbar_wait(&sh.mbar[stage], (cons / kRing) & 1, a.status, true);
+            const bool have = off < R.hi;  // the warp's 1 KiB is in the region (whole, unless the job ends in it)
+            // an end of the job in it: bytes before and after the job's are encoded too (the ring holds
+            // something there), but count for nothing and are not written out
+            const bool edge = off < R.lo || (R.last && off + kWarpBytes >= R.hi);
+            Pieces pc;
+            uint32_t nbits = 0;
+            if (have) {
+                const uint4* src = reinterpret_cast<const uint4*>(ring + stage * (uint32_t)kStepBytes + tid * kLaneBytes);
+                const uint4 q0 = src[0], q1 = src[1];
+                const uint32_t w[kPieces] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+                const char* const l8 = reinterpret_cast<const char*>(lut);
 #pragma unroll
-                for (int k = 0; k < kEncBpt; ++k) ll[k] &= 31u;
+                for (int j = 0; j < kPieces; ++j) {
+                    make_piece(l8, lane8, w[j], pc.hi[j], pc.lo[j], pc.q[j]);
+                    nbits += piece_bits(pc.q[j]);
+                }
+                if (edge) {
+                    const uint32_t o = off + lane * (uint32_t)kLaneBytes;
+                    const uint32_t b1 = o >= R.hi ? 0u : R.hi - o < 32u ? R.hi - o : 32u;
+                    nbits = b1 ? bits_before(pc, b1) - (o < R.lo ? bits_before(pc, R.lo - o) : 0u) : 0u;
+                }
             }
             const uint32_t incl = warp_incl_scan(nbits, lane);
-            if (lane == 31) sh.warp_tot[warp] = incl;
-            __syncthreads();  // (1) warp totals visible; this ring buffer read; previous chunk written out
-            // the word carried in (previous chunk's tail, or the rebuilt head word)
-            if (tid == 0 && sh.carry) atomicOr(img + ((P >> 5) & 3), sh.carry);
-            uint32_t wt = lane < (uint32_t)kEncWarps ? sh.warp_tot[lane] : 0u;
-            wt = warp_incl_scan(wt, lane);
-            const uint32_t L = __shfl_sync(kFull, wt, kEncWarps - 1);
-            const uint32_t excl = incl - nbits + (warp ? __shfl_sync(kFull, wt, warp - 1) : 0u);
-
-            // pack two codes at a time (<= 32 bits): at most one word per pair
-            const uint64_t sb = (P >> 5) & ~3ull;  // segment-aligned image base (global word)
-            if (nbits) {
-                const uint32_t p = (uint32_t)(P - 32 * sb) + excl;  // bit offset within the image
-                uint32_t wi = p >> 5;
-                uint32_t nb = p & 31;
-                uint32_t cur_w = 0;
-#pragma unroll
-                for (int k = 0; k < kEncBpt; k += 2) {
-                    const uint32_t l1 = ll[k];
-                    const uint32_t c12 = cc[k] | (cc[k + 1] >> l1);
-                    const uint32_t nbo = nb;
-                    cur_w |= c12 >> nb;
-                    const uint32_t spill = __funnelshift_r(0u, c12, nb);
-                    nb += l1 + ll[k + 1];
-                    if (nb >= 32) {
-                        atomicOr(img + wi, cur_w);  // the image starts clear: OR is a store
-                        // bits of the code crossing the word end that spill over
-                        spills[wi] = (uint8_t)(nbo + l1 >= 32 ? nbo + l1 - 32 : nb - 32);
-                        ++wi;
-                        cur_w = spill;
-                        nb -= 32;
-                    }
-                }
-                if (nb) atomicOr(img + wi, cur_w);
+            if (lane == 31) {
+                sh.tot[par][warp] = incl;
+                if (have) sh.tail[(cons * kEncWarps + warp + 1) % (4 * kEncWarps)] = last_bits(pc);
             }
-            __syncthreads();  // (2) image complete
-            // the last warp, whose write-out share is the smallest, refills the ring
-            // (this chunk's buffer was read before barrier (1))
+            __syncthreads();  // counts and tails visible; this ring buffer read; the previous step's records complete
+            // the last warp refills the ring
             if (tid == kEncThreads - 32) {
                 fence_proxy_async_smem();
                 produce(a, ring, sh, cons + 1, cur_slot);
             }
+            const uint32_t t = lane < (uint32_t)kEncWarps ? sh.tot[par][lane] : 0u;
+            const uint32_t L = __reduce_add_sync(kFull, t);
+            const uint32_t before = __reduce_add_sync(kFull, lane < warp ? t : 0u);
 
-            // write out complete words [P>>5, E>>5), clearing the image behind;
-            // the group holding word E>>5 hands it on as the carry
-            const uint64_t E = P + L;
-            const uint32_t j0 = (uint32_t)((P >> 5) - sb);
-            const uint32_t j1 = (uint32_t)((E >> 5) - sb);
-            uint32_t* const bits = J.bits;
-            const uint64_t words = J.words;
-            for (uint32_t g = tid; g <= j1 / 4; g += kEncThreads) {
-                const uint32_t j = 4 * g;
-                const uint4 wv = *reinterpret_cast<const uint4*>(img + j);
-                const uint64_t w = sb + j;
-                if (J.bits_aligned16 && j >= j0 && j + 4 <= j1 && w + 4 <= words) {
-                    *reinterpret_cast<uint4*>(bits + w) = wv;
-                } else {
-                    const uint32_t wa[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) {
-                        if (j + k < j0 || j + k >= j1) continue;
-                        if (w + k < words) bits[w + k] = wa[k];
-                        else overflow = true;
-                    }
-                    if (j1 - j < 4) {
-                        const uint32_t t = j1 - j;
-                        sh.carry = (E & 31) ? (t == 0 ? wa[0] : t == 1 ? wa[1] : t == 2 ? wa[2] : wa[3]) : 0u;
-                    }
-                }
-                *reinterpret_cast<uint4*>(img + j) = make_uint4(0, 0, 0, 0);
+            // Gap words of the steps before this one, once there are enough to occupy half the warps
+            // (a warp's 32 words take it as long as a fifth of a step, and every warp waits for it at
+            // the next barrier), or before this step's records would reach them.
+            const uint32_t gend = P >> 10;
+            const bool wrap = ((P + L) >> 7) - 8 * gnext >= kRecs - 8;  // (8: segments of bytes after the job's)
+            if (wrap || gend - gnext >= kEncThreads / 2) {  // uniform
+#pragma unroll 1
+                for (uint32_t g = gnext + (kEncThreads - 1 - tid); g < gend; g += kEncThreads) emit_gap(g, P >> 7, 4);
+                gnext = gend;
+                if (wrap) __syncthreads();
             }
-            // gap words [P>>10, kn>>3): one thread per segment k (slot t = k - kb8)
-            // puts its nibble in place, the 8 lanes of a gap word OR them with
-            // shuffles; the word of kn>>3 is partial (or empty) and carried
-            const uint64_t kb = P >> 7, kn = E >> 7;  // segments ending in this chunk: [kb, kn)
-            const uint64_t kb8 = kb & ~7ull;
-            const uint32_t nk = (uint32_t)(8 * ((kn >> 3) - (kb8 >> 3) + 1));
-            // highest warps first: the write-out above took the lowest ones
-            for (uint32_t t0 = (kEncWarps - 1 - warp) * 32; t0 < nk; t0 += kEncThreads) {  // warp-uniform
-                const uint32_t t = t0 + lane;
-                const uint64_t k = kb8 + t;
-                uint32_t v = 0;
-                if (t < nk && k >= kb && k < kn)  // entry k = spill of global word 4k+3
-                    v = (uint32_t)spills[(uint32_t)(4 * k + 3 - sb)] << (4 * (uint32_t)(k & 7));
-                if (t == 0) v |= sh.gcarry[cons & 1];  // nibbles carried into word kb8 >> 3
-                v |= __shfl_xor_sync(kFull, v, 1);
-                v |= __shfl_xor_sync(kFull, v, 2);
-                v |= __shfl_xor_sync(kFull, v, 4);
-                if (t < nk && (t & 7) == 0) {
-                    const uint64_t g = k >> 3;
-                    if (g < (kn >> 3)) {
-                        if (g < J.gap_words) J.gaps[g] = v;
-                        else overflow = true;
+
+            if (have) {
+                const uint32_t Pw = P + before;
+                uint32_t gw = (Pw >> 7) * 4 - kSlackBits / 32;       // output word of image word 0
+                uint32_t p1 = (Pw & 127u) + kSlackBits + incl;       // image bit of the lane's end
+                uint32_t p = p1 - nbits;
+                // lane 0: what the warp's first word already holds
+                const uint32_t before32 = sh.tail[(cons * kEncWarps + warp) % (4 * kEncWarps)];
+                uint32_t cur = lane == 0 ? __funnelshift_r(0u, before32, p) : 0u;
+                // more bits than the image holds: the warp's two halves one after the other
+                const uint32_t pe = __shfl_sync(kFull, p1, 31);
+                const bool split = (pe + (edge ? kLaneMaxBits : 0u)) >> 5 >= (uint32_t)kImgWords;
+                for (uint32_t half = 0;; half = 1) {
+                    const uint32_t pa = __shfl_sync(kFull, p, 16 * half);              // first and end bit
+                    const uint32_t pz = __shfl_sync(kFull, p1, split && !half ? 15 : 31);
+                    const bool act = split ? (lane >> 4) == half : true;
+                    const bool ends = R.last && off + kWarpBytes >= R.hi && (half || !split);  // the job's end
+                    if (edge) {
+                        const uint32_t o = off + lane * (uint32_t)kLaneBytes;
+                        if (o < R.lo) p -= bits_before(pc, R.lo - o);
+                        // words that no lane may complete
+                        if (act && nbits) img[(p + bits_before(pc, 32)) >> 5] = 0;
+                        if (half && lane == 16 && !nbits) img[p >> 5] = cur;
+                        __syncwarp();
+                    }
+                    const bool packs = act && (nbits || !edge);
+                    if (packs) cur = pack(pc, img, reinterpret_cast<char*>(recs), gw - 4, p, cur);
+                    __syncwarp();
+                    // a lane's unfinished word: the next lane stored that word's other bits
+                    if (packs) atomicOr(img + (p >> 5), cur);
+                    __syncwarp();
+                    // words to write: [j0, j1), the last one unfinished only where the job ends
+                    const uint32_t j0 = pa >> 5;
+                    uint32_t j1 = ends ? (pz + 31) >> 5 : pz >> 5;
+                    if (edge) {
+                        if (lane == 0 && off < R.lo) img[j0] &= ~0u >> (pa & 31);
+                        if (lane == 31 && ends && (pz & 31)) img[pz >> 5] &= ~(~0u >> (pz & 31));
+                        __syncwarp();
+                    }
+                    uint32_t* const bits = R.bits + (int32_t)gw;
+                    if (gw + j1 > R.nwords) {
+                        overflow = true;
+                        j1 = R.nwords > gw ? R.nwords - gw : 0u;
+                    }
+                    if (R.vec) {
+                        // whole 16-byte groups, then the words before and after them
+                        const uint32_t g0 = (j0 + 3) & ~3u, g1 = j1 & ~3u;
+#pragma unroll 1
+                        for (uint32_t j = g0 + 4 * lane; j < g1; j += 128)
+                            *reinterpret_cast<uint4*>(bits + j) = *reinterpret_cast<const uint4*>(img + j);
+                        const uint32_t jw = (lane < 4 ? j0 & ~3u : g1 - 4) + lane;
+                        if (jw < j1 && (lane < 4 ? jw >= j0 && jw < g0 : lane < 8 && jw >= g0)) bits[jw] = img[jw];
                     } else {
-                        sh.gcarry[(cons + 1) & 1] = v;
+#pragma unroll 1
+                        for (uint32_t j = j0 + lane; j < j1; j += 32) bits[j] = img[j];
                     }
+                    if (!split || half) break;
+                    // the second half's image starts at the segment of its first bit
+                    const uint32_t by = (__shfl_sync(kFull, p, 16) & ~127u) - kSlackBits;
+                    cur = __shfl_sync(kFull, cur, 15);
+                    if (lane != 16) cur = 0;
+                    p -= by;
+                    p1 -= by;
+                    gw += by >> 5;
+                    __syncwarp();
                 }
             }
-            P = E;
+            P += L;
         }
-        if (overflow) atomicOr(a.status, kDevSize);
-        __syncthreads();  // carries visible; the image is clear again
+        __syncthreads();  // every record of the region visible
 
         // ---- end of the region --------------------------------------------------
-        if (tid == 0) {
-            if (P - sh.G != sh.agg[cur_slot]) atomicOr(a.status, kDevPlan);  // histograms were not this input's
-            if (sh.item[cur_slot] - J.item0 + 1 == J.nst) {
-                if ((P & 31) && (P >> 5) < J.words) J.bits[P >> 5] = sh.carry;
-                const uint64_t gwe = (P >> 7) >> 3;
-                if (gwe < J.gap_words) J.gaps[gwe] = sh.gcarry[cons & 1];
-                if ((P + 31) / 32 != J.words || (P + 127) / 128 != J.segments) atomicOr(a.status, kDevSize);
+        {
+            const uint32_t k_end = P >> 7;
+#pragma unroll 1
+            for (uint32_t g = gnext + (kEncThreads - 1 - tid); g <= (k_end >> 3); g += kEncThreads) {
+                uint32_t bytes = 4;
+                if (g == (k_end >> 3)) bytes = !R.last ? (k_end & 7) >> 1 : g < R.ngaps ? 4u : 0u;  // the region ends in it
+                if (bytes) emit_gap(g, k_end, bytes);
             }
         }
+        if (overflow) atomicOr(a.status, kDevSize);
+        if (tid == 0) {
+            const uint64_t E = (sh.G & ~1023ull) + P;
+            if (E - sh.G != sh.agg[cur_slot]) atomicOr(a.status, kDevPlan);  // histograms were not this input's
+            if (R.last && ((E + 31) / 32 != J.words || (E + 127) / 128 != J.segments)) atomicOr(a.status, kDevSize);
+        }
+        __syncthreads();  // the slot, gap_head and G are read
         if (warp == 0) {
             // the next region becomes current; claim the one after it into the freed slot
             const int old = cur_slot;
-            if (sh.item[old ^ 1] < sh.nitems) claim_region(a, lutl, sh, old, lane);
+            if (sh.item[old ^ 1] < sh.nitems) claim_region(a, lut, sh, old, lane);
             else if (lane == 0) sh.item[old] = ~0ull;
             if (lane == 0) {
                 // the producer's cursor follows its region into the current slot
                 if (sh.p_which == 1) sh.p_which = 0;
-                else sh.p_chunk = 0;
+                else sh.p_step = 0;
                 produce(a, ring, sh, cons, old ^ 1);
             }
         }
