@@ -208,6 +208,7 @@ struct DecBookCache {
     uint32_t min_len = 0;
     bool complete = false;
     bool pairs = false;
+    hgap::DecIndex index;
     hgap::DecTable table;
 };
 
@@ -273,6 +274,11 @@ hgap_status decode_impl(const uint32_t* d_bits, uint64_t words, const uint32_t* 
         if (s != HGAP_OK) return s;
         // two symbols per lookup pay off once about a third of the lookups yield two
         cache.pairs = hgap::dec_pair_fraction(cache.table) >= 0.3;
+        uint32_t first_long = 0, max_len = 0;
+        while (first_long < (1u << hgap::kDecPrefix) && !(cache.table.t1[first_long] & 0x8000u)) ++first_long;
+        for (uint32_t i = 0; i < book.symbol_count; ++i)
+            if (book.symbols[i].length > max_len) max_len = book.symbols[i].length;
+        cache.index = hgap::dec_index(first_long, max_len, complete, hgap::dec_stage_rows(min_len));
         cache.count = cb->symbol_count;
         std::memcpy(cache.symbols, cb->symbols, sizeof(hgap_symlen) * cache.count);
         cache.min_len = min_len;
@@ -280,6 +286,7 @@ hgap_status decode_impl(const uint32_t* d_bits, uint64_t words, const uint32_t* 
         cache.valid = true;
     }
     a.hook = hook;
+    a.index = cache.index;
     // the table travels as a kernel parameter: copied at launch, so the cache may change after
     return cuda_status(hgap::launch_decode(a, cache.table, min_len, complete, cache.pairs, 0, 0, stream));
 }

@@ -12,12 +12,12 @@
 //   5. encode       the single-buffer encoder kernel over all regions, the
 //                   CTA reloading its code tables when the buffer changes.
 // Decompress:
-//   1. bdec_table   one CTA per buffer: checks the book, builds its decoder
-//                   table in shared memory, writes it in the widened form the
-//                   decode kernel keeps in shared memory (DecTableW), and puts
-//                   the buffer in one of 8 classes (decoder stage size by the
-//                   shortest code x complete book or not), and writes its
-//                   decode job (stream, output, tile count);
+//   1. bdec_table   one CTA per buffer: checks the book, writes its decoder
+//                   table in the form the decode kernel keeps in shared
+//                   memory (DecTableW), puts the buffer in one of 8 classes
+//                   (decoder stage size by the shortest code x complete book
+//                   or not), and writes its decode job (stream, output, tile
+//                   count);
 //   2. bdec_setup   one CTA: look-back record numbering over all tiles, and
 //                   per class the numbering of the class's tiles;
 //   3. bdec_map     tile -> buffer map of each class;
@@ -289,18 +289,17 @@ __device__ __forceinline__ uint32_t class_of(uint32_t min_len, bool complete) {
 
 constexpr int kTableThreads = 256;
 
-// One CTA per buffer: checks the entry, builds its two-level decoder table in
-// shared memory and writes the widened form the decode kernel copies per tile
-// (DecTableW), then classifies the buffer and writes its decode job (all but
-// its first look-back record, which bdec_setup numbers).  The table is the one
-// warp_dec_table builds (book.cuh) -- every level-1 prefix, and every level-2
-// suffix of a prefix whose codes are longer than kDecPrefix bits, takes the
-// symbol whose left-aligned code is the largest not above it; the level-2
-// groups sit in prefix order -- but every thread owns 8 consecutive prefixes
-// and a block scan places the groups, and the widened entries and the level-2
-// groups in use go out with coalesced stores, in one launch.  At 32 registers
-// a thread (no spills) seven CTAs fit an SM, bound by shared memory, where 40
-// registers allowed six.
+// One CTA per buffer: checks the entry, writes the buffer's decoder table
+// (DecTableW), classifies the buffer and writes its decode job (all but its
+// first look-back record, which bdec_setup numbers).  Every thread owns 8
+// consecutive 11-bit prefixes, each taking the symbol whose left-aligned code is
+// the largest not above it; the entries (up to three symbols, dec_entry.cuh)
+// come from those in shared memory, the longer codes' by a binary search per
+// entry, spread over all threads.  A book whose one table would be too large
+// (DecIndex) gets two levels, the same ones as warp_dec_table builds (book.cuh):
+// a block scan places the level-2 groups in prefix order.  At 32 registers a
+// thread (no spills) eight CTAs fit an SM.  Measured for 4096 buffers of 4-64
+// KiB: 66 us (80 us while every buffer built two levels).
 __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t count, const hgap_batch_entry* entries,
                                                                    const uint32_t* bits, const uint32_t* gaps,
                                                                    uint8_t* const* outputs, uint32_t tile_segs,
@@ -310,10 +309,9 @@ __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t c
     constexpr uint32_t kT1 = 1u << P, kPer = kT1 / kTableThreads;  // 8 prefixes a thread
     __shared__ BookScratch s;
     __shared__ __align__(16) uint16_t s1[kT1];
-    __shared__ __align__(16) uint16_t s2[kDecT2Cap];
     __shared__ uint16_t s_end[kT1];  // level-2 offset after each prefix's group (0 for none)
     __shared__ uint32_t s_warp[kTableThreads / 32];
-    __shared__ uint32_t s_kraft;
+    __shared__ uint32_t s_kraft, s_long;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint32_t j = blockIdx.x; j < count; j += gridDim.x) {
         const hgap_batch_entry& e = entries[j];
@@ -322,7 +320,10 @@ __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t c
                    (e.n != 0) != (e.words != 0) || (e.n != 0 && n == 0);
         if (warp == 0) {
             const uint32_t kraft = (!bad && n) ? warp_load_symbols(e.symbols, n, s, lane) : 0u;
-            if (lane == 0) s_kraft = kraft;
+            if (lane == 0) {
+                s_kraft = kraft;
+                s_long = kT1;
+            }
         }
         __syncthreads();
         const uint32_t kraft = s_kraft;
@@ -363,66 +364,89 @@ __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t c
                 if (L > P && (s.la[i_last] >> X) == x) {
                     span += 1u << (L - P);
                     pmask |= 1u << k;
+                    s1[x] = 0x8000u;  // (a wide book's get their width and offset below)
                 } else {
                     s1[x] = entry(i_first, v);
                 }
             }
-            // block scan of the spans: the level-2 offset of this thread's first group
+            // the first prefix of a longer code, and the block scan of the spans: the level-2
+            // offset of this thread's first group (a wide book's)
             const uint32_t incl = warp_incl_scan(span, lane);
             if (lane == 31) s_warp[warp] = incl;
+            if (pmask) atomicMin(&s_long, x0 + __ffs(pmask) - 1);
             __syncthreads();
-            const uint32_t wt = warp_incl_scan(lane < kTableThreads / 32 ? s_warp[lane] : 0u, lane);
-            const uint32_t total = __shfl_sync(kFull, wt, kTableThreads / 32 - 1);
-            uint32_t off = (warp ? __shfl_sync(kFull, wt, warp - 1) : 0u) + incl - span;
-            if (total <= (uint32_t)kDecT2Cap) {  // uniform; larger only for an incomplete book
-                // pass 2: the pointer prefixes, and every prefix's level-2 end offset
-                i_first = i_start;
-                for (uint32_t k = 0; k < kPer; ++k) {
-                    const uint32_t x = x0 + k;
-                    const uint32_t v = x << X;
-                    i_first = advance(i_first, v);
-                    if (pmask >> k & 1u) {
-                        i_last = advance(i_first, v | ((1u << X) - 1));
-                        const uint32_t w = s.clen[i_last] - P;
-                        s1[x] = (uint16_t)(0x8000u | (w << 12) | off);
-                        off += 1u << w;
+            const uint32_t cc = class_of(s.clen[0], kraft == (1u << kMaxLen));
+            const int rows = kStageRows[cc >> 1];
+            const uint32_t max_len = s.clen[n - 1], first_long = s_long;
+            const DecIndex ix = dec_index(first_long, max_len, (cc & 1u) != 0, rows);
+            const bool multi = dec_multi(rows, (cc & 1u) != 0);
+            DecTableW& w = wtables[j];
+            if (!ix.wide) {
+                c = cc;
+                const uint32_t extra = 32 - kDecPrefix - ix.shift;
+                for (uint32_t i = tid; i < ix.used; i += kTableThreads) {
+                    uint32_t e2 = kEntInvalid;
+                    const uint32_t v = (uint32_t)((int32_t)i - ix.offset);  // from first_long on: the window's bits
+                    if (i < first_long) {
+                        e2 = multi ? entry_multi(s1, i) : entry_pair(s1, i);
+                    } else if (v < kT1 << extra) {
+                        const uint32_t v16 = v << (kMaxLen - kDecPrefix - extra);
+                        const uint32_t e1 = entry(search(v16), v16);
+                        e2 = multi ? entry_single<true>(e1) : entry_single<false>(e1);
                     }
-                    s_end[x] = (uint16_t)off;
+                    w.t1[i] = e2;
                 }
-                __syncthreads();
-                // the level-2 entries, spread over all threads (the pointer prefixes sit
-                // together at the top of the code space, so per-prefix ownership would leave
-                // a few threads with hundreds of entries): entry k belongs to the first prefix
-                // whose end offset exceeds k
-                const uint32_t used = (total + 7) & ~7u;  // whole 16-byte groups, the tail invalid
-                for (uint32_t k = tid; k < used; k += kTableThreads) {
-                    uint16_t e2 = kDecInvalid;
-                    if (k < total) {
-                        uint32_t lo = 0, hi = kT1 - 1;
-                        while (lo < hi) {
-                            const uint32_t mid = (lo + hi) >> 1;
-                            if (s_end[mid] > k) hi = mid;
-                            else lo = mid + 1;
-                        }
-                        const uint32_t e1 = s1[lo];  // a pointer entry: width and start of its group
-                        const uint32_t w = (e1 >> 12) & 7u;
-                        const uint32_t vy = (lo << X) | ((k - (e1 & 0xfffu)) << (X - w));
-                        e2 = entry(search(vy), vy);
-                    }
-                    s2[k] = e2;
-                }
-                __syncthreads();
-                c = class_of(s.clen[0], kraft == (1u << kMaxLen));
-                const bool multi = dec_multi(kStageRows[c >> 1], (c & 1u) != 0);
-                DecTableW& w = wtables[j];
-                for (uint32_t i = tid; i < kT1; i += kTableThreads) {
-                    w.t1[i] = multi ? widen_multi(s1, i) : widen_pair(s1, i);
-                    w.l1[i] = first_len(s1, i);
-                }
-                for (uint32_t i = tid; i < used / 8; i += kTableThreads)
-                    reinterpret_cast<uint4*>(w.t2)[i] = reinterpret_cast<const uint4*>(s2)[i];
             } else {
-                bad = true;
+                const uint32_t wt = warp_incl_scan(lane < kTableThreads / 32 ? s_warp[lane] : 0u, lane);
+                const uint32_t total = __shfl_sync(kFull, wt, kTableThreads / 32 - 1);
+                uint32_t off = (warp ? __shfl_sync(kFull, wt, warp - 1) : 0u) + incl - span;
+                if (total <= (uint32_t)kDecT2Cap) {  // uniform; larger only for an incomplete book
+                    c = cc;
+                    // pass 2: the pointer prefixes, and every prefix's level-2 end offset
+                    i_first = i_start;
+                    for (uint32_t k = 0; k < kPer; ++k) {
+                        const uint32_t x = x0 + k;
+                        const uint32_t v = x << X;
+                        i_first = advance(i_first, v);
+                        if (pmask >> k & 1u) {
+                            i_last = advance(i_first, v | ((1u << X) - 1));
+                            const uint32_t wd = s.clen[i_last] - P;
+                            s1[x] = (uint16_t)(0x8000u | (wd << 12) | off);
+                            off += 1u << wd;
+                        }
+                        s_end[x] = (uint16_t)off;
+                    }
+                    __syncthreads();
+                    // the level-2 entries, spread over all threads (the pointer prefixes sit
+                    // together at the top of the code space, so per-prefix ownership would leave
+                    // a few threads with hundreds of entries): entry k belongs to the first prefix
+                    // whose end offset exceeds k
+                    const uint32_t used = (total + 7) & ~7u;  // whole 16-byte groups, the tail invalid
+                    for (uint32_t k = tid; k < used; k += kTableThreads) {
+                        uint16_t e2 = kDecInvalid;
+                        if (k < total) {
+                            uint32_t lo = 0, hi = kT1 - 1;
+                            while (lo < hi) {
+                                const uint32_t mid = (lo + hi) >> 1;
+                                if (s_end[mid] > k) hi = mid;
+                                else lo = mid + 1;
+                            }
+                            const uint32_t e1 = s1[lo];  // a pointer entry: width and start of its group
+                            const uint32_t wd = (e1 >> 12) & 7u;
+                            const uint32_t vy = (lo << X) | ((k - (e1 & 0xfffu)) << (X - wd));
+                            e2 = entry(search(vy), vy);
+                        }
+                        w.t2()[k] = e2;
+                    }
+                    for (uint32_t i = tid; i < kT1; i += kTableThreads)
+                        w.t1[i] = multi ? entry_multi(s1, i) : entry_pair(s1, i);
+                } else {
+                    bad = true;
+                }
+            }
+            if (c != kNoClass) {
+                for (uint32_t i = tid; i < n; i += kTableThreads) w.symlen[s.sym[i]] = s.clen[i];
+                if (tid == 0) w.index = ix;
             }
         }
         if (tid == 0) {
@@ -451,7 +475,7 @@ __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t c
             J.ntiles = nt;
             jobs[j] = J;
         }
-        __syncthreads();  // s, s1, s2 are reused for the next buffer
+        __syncthreads();  // s and s1 are reused for the next buffer
     }
 }
 

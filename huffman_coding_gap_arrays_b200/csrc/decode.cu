@@ -3,30 +3,49 @@
 // Replaces gpu_dec_l1_l2 (decoder/src/decoder.cu:454-730).  Same unit of
 // parallelism -- a 128-bit segment that starts at its gap offset -- but each
 // segment is decoded ONCE (the reference decodes it twice: a counting pass,
-// then a writing pass, decoder.cu:529-569,672-725):
-//   1. a persistent CTA of 256 threads takes the next tile of 512 segments
-//      (256 for books with 1-2 bit codes); every thread takes its segments'
-//      words straight from global memory into registers a tile ahead (one
-//      16-byte load per segment, the next segment's first word from the
-//      neighbouring lane) and decodes them one after the other (interleaving
-//      two chains measured slower: the loop is issue-bound) through a
-//      two-level table (level 1 in shared memory, the rarely used level 2 read
-//      from global memory), one 32-bit phase per word, so the loop tests only
-//      the phase end; each segment's symbols are parked in its own shared row
-//      sized for the book's shortest code (a segment holds at most
-//      ceil(128 / shortest length) symbols);
-//   2. block scan of the symbol counts (both halves of the tile packed in one
-//      warp scan) + one bounded decoupled look-back
-//      with a 64-tile window gives the tile's output offset;
-//   3. the rows are compacted (whole words where the destination is aligned)
-//      into a shared image of the tile's output and written one tile later,
-//      once its offset is known, with 16-byte coalesced stores (byte stores
-//      only on the two ragged edges), clipped at exactly n bytes (the
-//      reference writes past n, decoder.cu:529).
+// then a writing pass, decoder.cu:529-569,672-725).
+//
+// A persistent CTA of W decoding warps (8 or 16) and one more warp takes tiles
+// of 32 W consecutive segments of one stream.  A decoding warp owns 32 of
+// them, one per lane, and everything that is large is its own (no other warp
+// reads or writes it), so a tile costs the CTA one barrier:
+//   1. decode: a lane has its segment's words in registers (loaded a tile
+//      ahead: one 16-byte load, the next segment's first word from the
+//      neighbouring lane) and runs four phases of 32 bits, so its loop tests
+//      only the phase's end.  One table in shared memory serves all code
+//      lengths without a branch (DecIndex).  Position and output address
+//      advance in one addition: an entry holds the bits and the number of its
+//      symbols where the state has the position and the address.  The symbols
+//      go to the lane's row in shared memory, sized for the book's shortest code;
+//   2. the warps publish their symbol counts at the barrier;
+//   3. the warp writes the PREVIOUS tile's symbols out of its image, with
+//      16-byte stores shifted to the output's alignment (bytes at both ends),
+//      clipped at exactly n bytes (the reference writes past n,
+//      decoder.cu:529), and joins the rows of this tile to its image: a lane
+//      stores the words it completes and ORs its unfinished last word into the
+//      next lane's first (a segment has at least 8 symbols, so no word sees
+//      three lanes).
+// Meanwhile the extra warp publishes the tile's symbol count, resolves the
+// tile's output offset with a bounded decoupled look-back, claims a tile two
+// ahead, fetches its job, and copies the next tile's table into shared memory
+// if it is another buffer's: none of those round trips is on the decoding
+// warps' path, which need their results one barrier later.
 // Checks: every segment must end exactly where the next gap entry says the
 // next segment starts, every codeword must exist, and the stream must yield at
 // least n symbols; failures set kDevCorrupt / kDevSize, never trap.
+//
+// The kernel is bound by shared-memory wavefronts (one lookup of 32 random
+// entries and one or two byte stores per step: 84 % of the pipe on Zipf(1.2))
+// and by instruction issue (72 %), not by HBM.  Measured (B200, 256 MiB, call
+// without the status read), against a kernel with four CTA barriers a tile, a
+// branch to a second table level and byte-wise compaction: Zipf(1.2) 524 -> 376
+// us, mixed 489 -> 393, BF16 mantissa 422 -> 363, BF16 exponents 324 -> 266,
+// clamped Gaussians of sigma 1 / 3 431 -> 306 / 321 -> 261; 1024 buffers of
+// 4 KiB - 4 MiB (593 MB) 1047 -> 851 us.  Of that the branch-free table gives
+// Zipf(1.2) 439 -> 401 us and the batch 896 -> 858.
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "dec_entry.cuh"
 #include "device_util.cuh"
@@ -34,68 +53,58 @@
 
 namespace hgap {
 
-constexpr int kDecThreads = 256;
-// Segments per tile: dec_tile_segs(R) by default, 256 or 512 by the launch shape
-// (dec_tile_segs_for, hgap_internal.h).
-// Look-back window = 32 * kDecLookK tiles per round trip.  Small is best:
-// the resolve runs between two barriers, and a narrow window costs fewer
-// loads per lane (measured 256 / 128 / 64 / 32 records: 0.731 / 0.679 /
-// 0.674 / 0.683 ms for 256 MiB of the mixed stream).
-constexpr int kDecLookK = 2;
+// Look-back window = 32 * kDecLookK tiles per round trip.  One load a lane: the
+// extra warps of all CTAs read the same few lines, and a wider window costs
+// each of them more than the round trips it saves (Zipf(1.2) 256 MiB at 32 / 64 /
+// 128 records: 443 / 453 / 479 us, BF16 mantissa 371 / 378 / 392).
+constexpr int kDecLookK = 1;
 
-// R: stage rows of 4 symbols per segment (at most 4R symbols per segment);
-// SEGS: segments per tile, 256 (one per thread) or 512 (two per thread).
-template <int R, int SEGS>
+// R: stage rows of 4 symbols per segment (at most 4R symbols per segment); W: decoding warps;
+// S: segments per lane of a tile.
+template <int R, int W, int S>
 struct DecCfg {
     static constexpr int kMaxSym = 4 * R;
-    static constexpr int kSegs = SEGS;
-    static constexpr int kPer = kSegs / kDecThreads;   // segments per thread
-    static constexpr int kWarps = kDecThreads / 32;
-    static constexpr int kT1 = 1 << kDecPrefix;        // u32 level-1 entries
-    static constexpr int kGapStage = kSegs / 8 + 4;     // gap words of the tile (+1 before)
-    // stage row of one segment: its symbols (a multi entry's tail store may put two
-    // bytes past the count: 4 spare bytes there), an odd number of words so that
-    // the 32 rows a warp writes start in 32 different banks
-    static constexpr int kRowWords = ((kMaxSym + (dec_multi(R, true) ? 4 : 0) + 3) / 4) | 1;
-    static constexpr int kRow = 4 * kRowWords;
-    static constexpr int kStageBytes = kSegs * kRow + 16;
-    static constexpr int kCompactBytes = kSegs * kMaxSym + 64;
-    // the level-2 table stays in global memory (or the kernel parameter): codes longer
-    // than the 11-bit prefix are rare, and its shared memory buys CTAs per SM; so do
-    // the multi entries' first-code lengths (read only where a multi entry would run
-    // past the segment: 2 KiB less takes the 32-row decoder from 2 to 3 CTAs per SM)
-    static constexpr size_t kSmem = (size_t)(kT1 + kGapStage) * 4 + kStageBytes + kCompactBytes;
-    // CTAs per SM the shared memory allows (227 KiB usable, ~1.5 KiB static and
-    // reserved per CTA), at most 5 for 256-segment tiles (48 registers a thread, no
-    // spills) and 4 for 512-segment ones (64 registers: two segments' words in flight)
+    static constexpr int kSegs = 32 * W * S;           // segments per tile
+    static constexpr int kThreads = 32 * (W + 1);
+    static constexpr int kTab = (int)dec_table_cap(R); // u32 table entries
+    // one segment's row: its symbols, a byte or two that a multi-symbol entry stores past the
+    // count, and the word after the last whole one; an odd number of words, so that the 32 rows a
+    // warp writes start in 32 different banks (11 rows: at most 43 symbols, so 11 words do)
+    static constexpr int kRowWords = R == 11 ? 11 : (R + 1) | 1;
+    static constexpr int kRowBytes = 4 * kRowWords;
+    static constexpr int kRowsBytes = 32 * S * kRowBytes;
+    static constexpr int kImgBytes = 32 * S * kMaxSym + 32;  // the write-out reads 16-byte groups past the end
+    static constexpr int kWarpBytes = kRowsBytes + kImgBytes;
+    static constexpr size_t kSmem = 256 + (size_t)kTab * 4 + (size_t)W * kWarpBytes;
+    // CTAs per SM: by shared memory (227 KiB usable, ~1.5 KiB static and reserved per CTA) and by
+    // registers (40 a thread, 56 for two segments: 12 or 9 warps in each quarter of the SM)
     static constexpr int kBySmem = (int)((227u * 1024u) / (kSmem + 1536u));
-    static constexpr int kCap = SEGS == 256 ? 5 : 4;
-    static constexpr int kMinBlocks = kBySmem >= kCap ? kCap : (kBySmem < 1 ? 1 : kBySmem);
-    static_assert(kT1 % 4 == 0 && kGapStage % 4 == 0 && kStageBytes % 16 == 0, "16-byte aligned areas");
+    static constexpr int kByRegs = (S == 1 ? 48 : 36) / (W + 1);
+    static constexpr int kMinBlocks = kBySmem < 1 ? 1 : kBySmem < kByRegs ? kBySmem : kByRegs;
+    static_assert(kImgBytes % 16 == 0 && kRowsBytes % 16 == 0, "16-byte aligned areas");
 };
 
-// One codeword from the 32-bit window x at the current position: level-1
-// lookup, level 2 for the rare longer codes.  Returns the widened entry.
-__device__ __forceinline__ uint32_t lookup(const uint32_t* t1, const uint16_t* __restrict__ t2, uint32_t x) {
-    uint32_t e = t1[x >> (32 - kDecPrefix)];
-    if (e & 0x80000000u) {
+// The decoder's table for one tile (DecIndex).
+struct Table {
+    const uint32_t* t1;      // shared memory
+    const uint8_t* symlen;   // shared memory
+    const uint16_t* t2;      // wide books: level 2, global memory
+    uint32_t shift;
+    int32_t offset;
+};
+
+// The entry (dec_entry.cuh) of the 32-bit window x at a code's start.
+template <bool WIDE, bool MULTI>
+__device__ __forceinline__ uint32_t lookup(const Table& t, uint32_t x) {
+    const int32_t i1 = (int32_t)(x >> (32 - kDecPrefix));
+    if (!WIDE) return t.t1[max(i1, (int32_t)(x >> t.shift) + t.offset)];
+    uint32_t e = t.t1[i1];
+    if (e & kEntPointer) {
         const uint32_t wd = (e >> 16) & 7u;
-        e = widen_entry(t2[(e & 0xffffu) + ((x << kDecPrefix) >> (32 - wd))]);
+        e = entry_single<MULTI>(t.t2[(e & 0xffffu) + ((x << kDecPrefix) >> (32 - wd))]);
     }
     return e;
 }
-
-// Length of the first code of a multi entry's prefix: from the widened table's
-// byte array in global memory (batched path) or derived from the u16 level-1
-// table in the kernel parameter (single path).
-struct FirstLen {
-    const uint8_t* g;
-    const uint16_t* t1src;
-    __device__ __forceinline__ uint32_t operator()(uint32_t x) const {
-        const uint32_t i = x >> (32 - kDecPrefix);
-        return g ? (uint32_t)__ldg(g + i) : (uint32_t)first_len(t1src, i);
-    }
-};
 
 // The words of one segment in registers: its own four and the next segment's
 // first (a code that starts in the segment may end up to 15 bits into it).
@@ -103,260 +112,326 @@ struct SegWords {
     uint32_t w0, w1, w2, w3, w4;
 };
 
+__device__ __forceinline__ void st_shared_u8(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
 // Decodes the codes that start in one 128-bit segment (not the stream's last
 // one), from bit `pos` (its gap offset), as four phases of 32 bits: phase k
 // decodes the codes starting in word k, from the window of words k and k+1,
-// so the loop tests only `pos < 32` -- no word refill, no end test.  Codes of
-// a pair / multi entry all start inside the segment in phases 0-2 (they fit
-// the 11-bit window and phase 2 ends 32 bits before the segment does); in
-// phase 3 that holds while pos <= 21, and the last bits take only the codes
-// that start before bit 32 of the phase.  Returns the end bit of the last
-// code relative to phase 3 (32 + the next gap entry for a valid stream; larger
-// after an invalid code) and advances `out` past the symbols.
-template <bool COMPLETE, bool PAIRS, bool MULTI>
-__device__ __forceinline__ uint32_t decode_segment(const uint32_t* t1, const uint16_t* __restrict__ t2,
-                                                   const FirstLen& fl, const SegWords& w, uint32_t pos,
-                                                   uint8_t*& out) {
-    constexpr uint32_t kBad = 1u << 16;  // position after an invalid code: every loop ends
-    auto run_fast = [&](uint32_t cw, uint32_t nw, uint32_t stop) {
-        while (pos < stop) {
-            const uint32_t e = lookup(t1, t2, __funnelshift_l(nw, cw, pos));
-            if (!COMPLETE && (e & 0x40000000u)) {
-                pos = kBad;
-                break;
-            }
-            if (MULTI) {
-                out[0] = (uint8_t)e;
-                out[1] = (uint8_t)(e >> 8);
-                out[2] = (uint8_t)(e >> 16);
-                out += 1 + ((e >> 29) & 3u);
+// so the loop tests only bit 5 of the position -- no word refill, no end test.
+// Codes of a pair / multi entry all start inside the segment in phases 0-2
+// (they fit the 11-bit window and phase 2 ends 32 bits before the segment
+// does); in phase 3 that holds while pos <= 21, and the last bits take only
+// the codes that start before bit 32 of the phase.  The symbols go to shared
+// address `row` on; their number is returned in `cnt`.  Returns the end bit of
+// the last code relative to phase 3 (32 + the next gap entry for a valid
+// stream), or a value no stream yields after an invalid code.
+template <bool WIDE, bool COMPLETE, bool PAIRS, bool MULTI>
+__device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWords& w, uint32_t pos, uint32_t row,
+                                                   uint32_t& cnt) {
+    static_assert(!MULTI || COMPLETE, "multi entries: complete books");
+    constexpr uint32_t kBad = 1u << 16;
+    constexpr uint32_t kEarly = kDecPrefix - 1;  // the last phase's fast loop ends this many bits early
+    if (MULTI) {
+        uint32_t out = row;
+        auto fast = [&](uint32_t cw, uint32_t nw) {
+            while (!(pos & 32)) {
+                const uint32_t e = lookup<WIDE, true>(t, __funnelshift_l(nw, cw, pos));
+                st_shared_u8(out, e);
+                st_shared_u8(out + 1, e >> 8);
+                st_shared_u8(out + 2, e >> 16);
+                out += 1 + (e >> 29);
                 pos += (e >> 24) & 31u;
-            } else if (PAIRS) {
-                out[0] = (uint8_t)e;
-                out[1] = (uint8_t)(e >> 8);  // a single entry's second byte: overwritten or past the count
-                out += 1 + ((e >> 16) & 1u);
-                pos += e >> 24;
-            } else {
-                *out++ = (uint8_t)e;
-                pos += e >> 24;
             }
+        };
+        fast(w.w0, w.w1);
+        pos -= 32;
+        fast(w.w1, w.w2);
+        pos -= 32;
+        fast(w.w2, w.w3);
+        pos += kEarly - 32;
+        fast(w.w3 >> kEarly, __funnelshift_r(w.w4, w.w3, kEarly));
+        pos -= kEarly;
+        while (!(pos & 32)) {
+            const uint32_t e = lookup<WIDE, true>(t, __funnelshift_l(w.w4, w.w3, pos));
+            const uint32_t tot = (e >> 24) & 31u, more = e >> 29;
+            st_shared_u8(out, e);
+            st_shared_u8(out + 1, e >> 8);
+            st_shared_u8(out + 2, e >> 16);
+            const bool all = pos + tot <= 32;  // every code of the entry ends, so starts, inside
+            out += all ? 1 + more : 1;
+            pos += all || !more ? tot : t.symlen[e & 0xffu];
         }
-    };
-    run_fast(w.w0, w.w1, 32);
-    pos -= 32;
-    run_fast(w.w1, w.w2, 32);
-    pos -= 32;
-    run_fast(w.w2, w.w3, 32);
-    pos -= 32;
-    if (!PAIRS) {
-        run_fast(w.w3, w.w4, 32);
+        cnt = out - row;
         return pos;
     }
-    run_fast(w.w3, w.w4, 32 - kDecPrefix + 1);
-    while (pos < 32) {  // the last bits: only the codes that start before bit 32
-        const uint32_t x = __funnelshift_l(w.w4, w.w3, pos);
-        const uint32_t e = lookup(t1, t2, x);
-        if (!COMPLETE && (e & 0x40000000u)) {
-            pos = kBad;
-            break;
+    uint32_t s = (row << 8) | pos;
+    auto fast = [&](uint32_t cw, uint32_t nw) -> bool {  // false: an invalid code
+        while (!(s & 32)) {
+            const uint32_t e = lookup<WIDE, false>(t, __funnelshift_l(nw, cw, s));
+            if (!COMPLETE && (e & kEntInvalidBit)) return false;
+            st_shared_u8(s >> 8, e);
+            if (PAIRS) st_shared_u8((s >> 8) + 1, e >> 8);  // a single entry's second byte: overwritten or past the count
+            s += e >> 16;
         }
-        if (MULTI) {
-            const uint32_t tot = (e >> 24) & 31u, more = (e >> 29) & 3u;
-            out[0] = (uint8_t)e;
-            out[1] = (uint8_t)(e >> 8);
-            out[2] = (uint8_t)(e >> 16);
-            if (pos + tot <= 32) {  // every code of the entry ends, so starts, inside
-                out += 1 + more;
-                pos += tot;
-            } else {
-                out += 1;
-                pos += more ? fl(x) : tot;
+        return true;
+    };
+    auto run = [&]() -> bool {
+        if (!fast(w.w0, w.w1)) return false;
+        s -= 32;
+        if (!fast(w.w1, w.w2)) return false;
+        s -= 32;
+        if (!fast(w.w2, w.w3)) return false;
+        s -= 32;
+        if (!PAIRS) return fast(w.w3, w.w4);
+        s += kEarly;
+        if (!fast(w.w3 >> kEarly, __funnelshift_r(w.w4, w.w3, kEarly))) return false;
+        s -= kEarly;
+        while (!(s & 32)) {  // the last bits: only the codes that start before bit 32
+            const uint32_t e = lookup<WIDE, false>(t, __funnelshift_l(w.w4, w.w3, s));
+            if (!COMPLETE && (e & kEntInvalidBit)) return false;
+            st_shared_u8(s >> 8, e);
+            st_shared_u8((s >> 8) + 1, e >> 8);
+            uint32_t by = e >> 16;
+            if (by & 0x200u) {  // two symbols: the second one counts only if it starts inside
+                const uint32_t l1 = t.symlen[e & 0xffu];
+                if ((s & 31u) + l1 >= 32) by = 0x100u + l1;
             }
-        } else {
-            const uint32_t tot = e >> 24;
-            const bool pair = (e & 0x10000u) != 0;
-            const uint32_t l1 = pair ? ((e >> 17) & 15u) : tot;
-            const bool two = pair && pos + l1 < 32;
-            out[0] = (uint8_t)e;
-            if (two) out[1] = (uint8_t)(e >> 8);
-            out += two ? 2 : 1;
-            pos += two ? tot : l1;
+            s += by;
         }
-    }
-    return pos;
+        return true;
+    };
+    const bool valid = run();
+    cnt = (s >> 8) - row;
+    return COMPLETE || valid ? s & 0xffu : kBad;
 }
 
 // The stream's last segment: its codes end at bit `end` (<= 128) and zero
 // padding follows, which may not decode.  One code per step (the first code of
 // any pair or multi entry), the words picked by index.
-template <bool COMPLETE, bool PAIRS, bool MULTI>
-__device__ __forceinline__ uint32_t decode_last_segment(const uint32_t* t1, const uint16_t* __restrict__ t2,
-                                                        const FirstLen& fl, const SegWords& w, uint32_t pos,
-                                                        uint32_t end, uint8_t* out) {
+template <bool WIDE, bool COMPLETE, bool MULTI>
+__device__ __forceinline__ uint32_t decode_last_segment(const Table& t, const SegWords& w, uint32_t pos, uint32_t end,
+                                                        uint32_t row) {
     auto word = [&](uint32_t i) { return i == 0 ? w.w0 : i == 1 ? w.w1 : i == 2 ? w.w2 : i == 3 ? w.w3 : w.w4; };
     uint32_t cnt = 0;
     while (pos < end) {
         const uint32_t wi = pos >> 5;
-        const uint32_t x = __funnelshift_l(word(wi + 1), word(wi), pos);
-        const uint32_t e = lookup(t1, t2, x);
-        if (!COMPLETE && (e & 0x40000000u)) break;  // the padding after the final codeword
-        uint32_t len;
-        if (MULTI) {
-            len = ((e >> 29) & 3u) ? fl(x) : ((e >> 24) & 31u);
-        } else if (PAIRS) {
-            len = (e & 0x10000u) ? ((e >> 17) & 15u) : (e >> 24);
-        } else {
-            len = e >> 24;
-        }
-        out[cnt++] = (uint8_t)e;
-        pos += len;
+        const uint32_t e = lookup<WIDE, MULTI>(t, __funnelshift_l(word(wi + 1), word(wi), pos));
+        if (!COMPLETE && (e & kEntInvalidBit)) break;  // the padding after the final codeword
+        const uint32_t more = MULTI ? e >> 29 : (e >> 24) - 1;
+        const uint32_t len = MULTI ? (e >> 24) & 31u : (e >> 16) & 31u;
+        st_shared_u8(row + cnt, e);
+        ++cnt;
+        pos += more ? t.symlen[e & 0xffu] : len;
     }
     return cnt;
 }
 
-// A claimed tile and its job, in shared memory.
+// A claimed tile, in shared memory: what the decoding warps need of it (clipped
+// to the tile, 32-bit), then what the extra warp does.
 struct DecSlot {
-    DecJob job;
-    uint64_t item;    // tile id in the launch's numbering (>= nitems: none)
-    uint64_t local;   // tile index within its job
+    const uint32_t* bits;  // the tile's first word
+    const uint32_t* gaps;  // and gap word
+    uint32_t nwords;       // words from there to the stream's end (at most one past the tile)
+    uint32_t ngaps;        // gap words of the tile
+    uint32_t nseg;         // segments (0: no tile)
+    uint32_t last_bits;    // bits of the stream's last segment if it is in this tile, else 0
     uint32_t job_id;
-    uint32_t pad;
+    DecIndex index;        // of its job's table
+    bool first, last;      // of its job's tiles
+    uint64_t rec;          // look-back record
+    uint8_t* out;          // the job's output
+    uint64_t n;            // and its size
 };
 
 // COMPLETE: the book's Kraft sum is 1 (every package-merge book with two or
 // more symbols), so no table entry is invalid and the decode loop skips that test.
 // PAIRS: level-1 entries carry two symbols where both codes fit in the window
-// (worth it for short-code books; for long codes the extra selects only cost);
-// with a complete book, up to three (multi entries, widen_multi).
-template <int R, int SEGS, bool COMPLETE, bool PAIRS>
-__global__ void __launch_bounds__(kDecThreads, DecCfg<R, SEGS>::kMinBlocks)
+// (worth it for short-code books; for long codes the extra store only costs);
+// with a complete book of the shortest codes, up to three (dec_multi).
+template <int R, int W, int S, bool COMPLETE, bool PAIRS>
+__global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kMinBlocks)
     decode_kernel(const __grid_constant__ DecArgs a, const __grid_constant__ DecTable tab) {
-    using C = DecCfg<R, SEGS>;
-    extern __shared__ __align__(16) uint32_t smem[];
-    uint32_t* t1 = smem;
-    uint32_t* sg = smem + C::kT1;                         // gap words: sg[j] = gaps[s0/8 - 1 + j]
-    uint8_t* stage = reinterpret_cast<uint8_t*>(sg + C::kGapStage);
-    uint8_t* compact = stage + C::kStageBytes;
-    __shared__ uint32_t warp_tot[C::kWarps];
-    __shared__ DecSlot slot[3];  // ring: the tile being decoded, the next one, the previous one
-    __shared__ uint64_t s_O;
+    using C = DecCfg<R, W, S>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint8_t* const symlen = smem;                          // a symbol's code length, where it is at most kDecPrefix
+    uint32_t* const t1 = reinterpret_cast<uint32_t*>(smem + 256);
+    unsigned char* const areas = smem + 256 + 4 * C::kTab; // per warp: rows, image
+    __shared__ DecSlot slot[4];                            // tile i in slot i % 4
+    __shared__ uint32_t tot[2][W];                         // by tile parity: the warps' symbol counts,
+    __shared__ uint8_t* dst[2];                            // the tile's place in the output,
+    __shared__ uint32_t room[2];                           // and the bytes there until n
+    // completed once for every second tile (by its parity): its counts are published; its slot is
+    // filled; dst and room are set
+    __shared__ uint64_t published[2], filled[2], placed[2];
+    __shared__ uint64_t tbar;                              // a table copy landed
     __shared__ uint64_t s_nitems;
-    __shared__ uint32_t s_lut_job;
 
     constexpr bool MULTI = PAIRS && dec_multi(R, COMPLETE);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // single path: the u16 tables widened here, once per CTA
-    auto load_tables = [&](const DecTable& t) {
-        for (int i = tid; i < C::kT1; i += kDecThreads) {
-            if (MULTI) {
-                t1[i] = widen_multi(t.t1, i);
-            } else {
-                t1[i] = PAIRS ? widen_pair(t.t1, i) : widen_entry(t.t1[i]);
-            }
-        }
-    };
-    // batched path (always PAIRS): the buffer's tables come widened, copied in 16-byte groups
-    auto copy_tables = [&](const DecTableW& t) {
-        const uint4* s1 = reinterpret_cast<const uint4*>(t.t1);
-        for (int i = tid; i < C::kT1 / 4; i += kDecThreads) reinterpret_cast<uint4*>(t1)[i] = s1[i];
-    };
-    // the same for the next tile of another job, as soon as this tile's decode is
-    // done (nothing reads `t1` again before the next tile): asynchronous copies,
-    // so their L2 round trip overlaps the look-back, write-out and compaction
-    auto copy_tables_async = [&](const DecTableW& t) {
-        const uint4* s1 = reinterpret_cast<const uint4*>(t.t1);
-        for (int i = tid; i < C::kT1 / 4; i += kDecThreads) cp_async16(reinterpret_cast<uint4*>(t1) + i, s1 + i);
-        cp_async_commit();
-    };
-    // thread 0: the tile `item` and its job into slot s
+
+    // the tile `item` into slot s (one thread)
     auto fill_slot = [&](int s, uint64_t item) {
         DecSlot& d = slot[s];
-        d.item = item;
-        if (item < s_nitems) {
-            const uint32_t j = a.jobs ? a.job_of[item] : 0u;
-            d.job = a.jobs ? a.jobs[j] : a.single;
-            d.local = a.jobs ? item - a.item0s[j] : item;
-            d.job_id = j;
-        }
+        d.nseg = 0;
+        if (item >= s_nitems) return;
+        const uint32_t j = a.jobs ? a.job_of[item] : 0u;
+        const DecJob& J = a.jobs ? a.jobs[j] : a.single;
+        const uint64_t local = a.jobs ? item - a.item0s[j] : item;
+        const uint64_t s0 = local * C::kSegs, left = J.segments - s0;
+        const uint64_t words = J.words - 4 * s0, gws = J.gap_words - s0 / 8;
+        d.bits = J.bits + 4 * s0;
+        d.gaps = J.gaps + s0 / 8;
+        d.nwords = words < 4 * C::kSegs + 1 ? (uint32_t)words : 4 * C::kSegs + 1;
+        d.ngaps = gws < C::kSegs / 8 ? (uint32_t)gws : C::kSegs / 8;
+        d.nseg = left < (uint64_t)C::kSegs ? (uint32_t)left : (uint32_t)C::kSegs;
+        // (every entry point checks segments == ceil(words / 4))
+        d.last_bits = left <= (uint64_t)C::kSegs ? (uint32_t)(32 * words - 128 * (left - 1)) : 0u;
+        d.job_id = j;
+        d.index = a.jobs ? a.tables[j].index : a.index;
+        d.first = local == 0;
+        d.last = local + 1 == J.ntiles;
+        d.rec = J.item0 + local;
+        d.out = J.out_aligned + J.out_lo;
+        d.n = J.n;
+    };
+    auto copy_table = [&](const DecSlot& d) {  // one thread
+        fence_proxy_async_smem();              // after the reads of the table before it
+        // (symlen and t1 lie together, here and in DecTableW)
+        bulk_load(symlen, a.tables[d.job_id].symlen, 256 + 4 * d.index.used, &tbar);
     };
 
-    // A tile's words go straight from global memory into registers, a tile
-    // ahead: segment col's four words (one 16-byte load where the stream is
-    // 16-byte aligned) and, for lane 31, the first word of the next segment
-    // (the other lanes take it from their neighbour with a shuffle).  Its gap
-    // words are staged in shared memory.
-    uint4 pre_q[C::kPer];
-    uint32_t pre_w4[C::kPer];
-    uint32_t pre_gap = 0;
-    auto prefetch = [&](const DecSlot& ps) {
-        const bool ok = ps.item < s_nitems;
-        const uint64_t s0p = ps.local * C::kSegs;
-        const uint64_t words = ok ? ps.job.words : 0;
-        const uint32_t* const bits = ps.job.bits;
-        const bool al16 = (reinterpret_cast<uintptr_t>(bits) & 15) == 0;
-#pragma unroll
-        for (int k = 0; k < C::kPer; ++k) {
-            const uint64_t w = 4 * (s0p + tid + k * kDecThreads);  // the segment's first word
-            if (al16 && w + 4 <= words) {
-                pre_q[k] = ld_stream_v4(bits + w);
+    if (!a.jobs) {
+        // single path: the u16 tables to shared memory (the areas are still free), and the entries
+        // made from there (the launch parameters' bank serves one address at a time)
+        constexpr int kRaw = sizeof(DecTable) / 8, kT1 = 1 << kDecPrefix;
+        static_assert(sizeof(DecTable) <= (size_t)W * C::kWarpBytes, "the raw table fits the areas");
+        uint64_t* const raw = reinterpret_cast<uint64_t*>(areas);
+        const uint64_t* const src = reinterpret_cast<const uint64_t*>(&tab);
+        for (int i = tid; i < kRaw; i += C::kThreads) raw[i] = src[i];
+        __syncthreads();
+        const DecTable& r = *reinterpret_cast<const DecTable*>(areas);
+        for (int i = tid; i < (int)a.index.used; i += C::kThreads) {
+            uint32_t e = kEntInvalid;
+            if (i < kT1 && (a.index.wide || !(r.t1[i] & 0x8000u))) {
+                e = MULTI ? entry_multi(r.t1, i) : PAIRS ? entry_pair(r.t1, i) : entry_single<false>(r.t1[i]);
+                const uint32_t e1 = r.t1[i];
+                if (!(e1 & (0x8000u | kDecInvalid))) symlen[e1 & 0xffu] = (uint8_t)((e1 >> 8) + 1);
             } else {
-                pre_q[k].x = w < words ? ld_stream_u32(bits + w) : 0u;
-                pre_q[k].y = w + 1 < words ? ld_stream_u32(bits + w + 1) : 0u;
-                pre_q[k].z = w + 2 < words ? ld_stream_u32(bits + w + 2) : 0u;
-                pre_q[k].w = w + 3 < words ? ld_stream_u32(bits + w + 3) : 0u;
+                // a longer code: v = its window's bits down to the longest length
+                const uint32_t v = (uint32_t)(i - a.index.offset), extra = 32 - kDecPrefix - a.index.shift;
+                if (v < (uint32_t)kT1 << extra) {
+                    const uint32_t e1 = r.t1[v >> extra], w = (e1 >> 12) & 7u;
+                    e = entry_single<MULTI>(r.t2[(e1 & 0xfffu) + ((v & ((1u << extra) - 1u)) >> (extra - w))]);
+                }
             }
-            pre_w4[k] = (lane == 31 && w + 4 < words) ? ld_stream_u32(bits + w + 4) : 0u;
+            t1[i] = e;
         }
-        // sg[j] = gaps[pg0 - 1 + j]: j = 0 exists unless the tile is its job's first
-        const uint64_t pg0 = ps.local * (C::kSegs / 8);
-        const uint64_t grem = ok && ps.job.gap_words + 1 > pg0 ? ps.job.gap_words + 1 - pg0 : 0;
-        const uint32_t gavail = grem < (uint64_t)C::kGapStage ? (uint32_t)grem : (uint32_t)C::kGapStage;
-        pre_gap = (tid < gavail && (tid > 0 || pg0 > 0)) ? __ldg(ps.job.gaps + pg0 - 1 + tid) : 0u;
-    };
-
-    if (!a.jobs) load_tables(tab);
-    if (tid == 0) {
+    }
+    if (tid == 32 * W) {
+        for (int k = 0; k < 2; ++k) {
+            mbar_init(&published[k], 1);
+            mbar_init(&filled[k], 1);
+            mbar_init(&placed[k], 1);
+            room[k] = 0;
+        }
+        mbar_init(&tbar, 1);
+        mbar_init_fence();
         s_nitems = a.nitems_dev ? *a.nitems_dev : a.nitems;
         fill_slot(0, atomicAdd(a.counter, 1u));
-        s_lut_job = a.jobs ? ~0u : 0u;
+        mbar_arrive(&filled[0]);
+        if (a.jobs && slot[0].nseg) copy_table(slot[0]);
     }
     __syncthreads();
-    if (a.jobs && slot[0].item < s_nitems) copy_tables(a.tables[slot[0].job_id]);
-    prefetch(slot[0]);
-    if (tid < (uint32_t)C::kGapStage) sg[tid] = pre_gap;
-    int ti = 0;        // slot of the tile decoded in this iteration
-    int prev_s = -1;   // slot of the tile decoded one iteration earlier: its symbols wait in
-                       // `compact` (at tile-local offsets) until its output offset is resolved
-    uint32_t prev_ct = 0;
+    if (slot[0].nseg == 0) return;
+    // Waits between the warps of the CTA: each side's work between them is itself bounded.
+    auto wait = [&](uint64_t* bar, uint32_t i) { return mbar_wait(&bar[i & 1], (i >> 1) & 1, a.status, false); };
 
-    for (;;) {
-        __syncthreads();  // (1) gap words of the tile staged, its tables loaded; `compact` holds prev
-        const DecSlot& T = slot[ti];
-        const bool have = T.item < s_nitems;
-        if (!have && prev_s < 0) break;
-        if (tid == 0 && have) s_lut_job = T.job_id;
-        const int ns = ti == 2 ? 0 : ti + 1;  // slot of the next tile
+    if (warp == W) {
+        // ---- the extra warp -------------------------------------------------------
+        // (the second tile is claimed only now, when the other CTAs have their first: a CTA that
+        // held two consecutive tiles would keep all later ones waiting for its second)
         uint32_t claim = 0;
-        if (tid == 0 && have) claim = atomicAdd(a.counter, 1u);  // its latency hides behind the decode
-        const uint64_t s0 = T.local * C::kSegs;  // first segment of the tile within its job
-        const uint16_t* const t2 = a.jobs ? a.tables[T.job_id].t2 : tab.t2;  // level 2, not staged
-        const FirstLen fl{a.jobs ? a.tables[T.job_id].l1 : nullptr, tab.t1};
-        // tile-local, 32-bit from here on: segments [0, nseg) of the tile; the stream's last
-        // segment (if in this tile) ends at bit end_last instead of at its 128-bit boundary
-        const uint64_t seg_rem = have ? T.job.segments - s0 : 0;
-        const uint32_t nseg = seg_rem < (uint64_t)C::kSegs ? (uint32_t)seg_rem : (uint32_t)C::kSegs;
-        const bool last_tile = seg_rem <= (uint64_t)C::kSegs;
-        // (every entry point checks segments == ceil(words / 4))
-        const uint64_t bits_rem = last_tile && have ? T.job.words * 32 - 128 * s0 : 0;
-        const uint32_t end_last = bits_rem < 128ull * nseg ? (uint32_t)bits_rem : 128 * nseg;
-        const uint32_t first_gap = s0 ? ~0u : 0u;  // the job's first segment starts at bit 0
-        // gap entry of tile segment u - 8 (u >= 7: u = 7 is the segment before the tile)
-        auto gap_at = [&](uint32_t u) -> uint32_t { return (sg[u >> 3] >> (4 * (u & 7))) & 0xfu; };
+        if (lane == 0) {
+            fill_slot(1, atomicAdd(a.counter, 1u));
+            mbar_arrive(&filled[1]);
+        }
+        __syncwarp();
+        for (uint32_t i = 0; slot[i & 3].nseg != 0; ++i) {
+            const DecSlot& T = slot[i & 3];
+            const DecSlot& N = slot[(i + 1) & 3];
+            if (!wait(published, i)) break;  // tile i is decoded: the table is free
+            const uint32_t Ct = __reduce_add_sync(kFull, lane < (uint32_t)W ? tot[i & 1][lane] : 0u);
+            if (lane == 0 && N.nseg) {
+                claim = atomicAdd(a.counter, 1u);  // (its answer is needed only after the look-back)
+                if (a.jobs && N.job_id != T.job_id) copy_table(N);
+            }
+            const uint64_t O = lookback_resolve<kDecLookK>(a.lookback, T.rec, Ct, T.first, a.status, lane,
+                                                           wait_limit(a.hook), T.rec + 1 != a.hook.hold_plus1);
+            if (lane == 0) {
+                if (T.last && O + Ct < T.n) atomicOr(a.status, kDevSize);
+                dst[i & 1] = T.out + O;
+                room[i & 1] = O >= T.n ? 0u : T.n - O < 0x40000000ull ? (uint32_t)(T.n - O) : 0x40000000u;
+                mbar_arrive(&placed[i & 1]);
+                if (N.nseg) fill_slot((i + 2) & 3, claim);
+                else slot[(i + 2) & 3].nseg = 0;
+                mbar_arrive(&filled[i & 1]);
+            }
+            __syncwarp();
+        }
+        return;
+    }
 
-        // ---- 1. decode segments tid (and tid + 256), one after the other -------
-        uint32_t n[C::kPer];
+    // ---- the decoding warps -------------------------------------------------------
+    unsigned char* const rows = areas + warp * C::kWarpBytes;
+    unsigned char* const img = rows + C::kRowsBytes;
+    uint32_t* const row32 = reinterpret_cast<uint32_t*>(rows + lane * C::kRowBytes);  // of the lane's first segment
+    const uint32_t u0 = warp * 32 * S + lane;  // the lane's segments in the tile: u0 + 32 k
+
+    // A tile's words and gap entries, loaded a tile ahead: a segment's four words (one 16-byte load
+    // where the stream is 16-byte aligned), for lane 31 the first word of the next segment, the gap
+    // word of the segment's entry, for lane 0 the one of the entry before.
+    uint4 pre_q[S];
+    uint32_t pre_w4[S], pre_gap[S], pre_gap0[S];
+    auto prefetch = [&](const DecSlot& N) {
+        const uint32_t words = N.nseg ? N.nwords : 0u, ngaps = N.nseg ? N.ngaps : 0u;
+        const bool al16 = (reinterpret_cast<uintptr_t>(N.bits) & 15) == 0;
 #pragma unroll
-        for (int k = 0; k < C::kPer; ++k) {
+        for (int k = 0; k < S; ++k) {
+            const uint32_t u = u0 + 32 * k, w = 4 * u;
+            const uint32_t* const p = N.bits + w;
+            if (al16 && w + 4 <= words) {
+                pre_q[k] = ld_stream_v4(p);
+            } else {
+                pre_q[k].x = w < words ? ld_stream_u32(p) : 0u;
+                pre_q[k].y = w + 1 < words ? ld_stream_u32(p + 1) : 0u;
+                pre_q[k].z = w + 2 < words ? ld_stream_u32(p + 2) : 0u;
+                pre_q[k].w = w + 3 < words ? ld_stream_u32(p + 3) : 0u;
+            }
+            pre_w4[k] = lane == 31 && w + 4 < words ? ld_stream_u32(p + 4) : 0u;
+            pre_gap[k] = (u >> 3) < ngaps ? __ldg(N.gaps + (u >> 3)) : 0u;
+            pre_gap0[k] = lane == 0 && w < words && (u || !N.first) ? __ldg(N.gaps + (u >> 3) - 1) : 0u;
+        }
+    };
+    prefetch(slot[0]);
+    // (a wait that gives up leaves no table to decode with: nothing is decoded from then on)
+    uint32_t copies = a.jobs ? 1 : 0;  // table copies so far
+    bool alive = !copies || mbar_wait(&tbar, 0, a.status, false);
+
+    uint32_t prev_m = 0, prev_before = 0;  // the warp's symbols of the tile before, and those before them in it
+    for (uint32_t i = 0;; ++i) {
+        const DecSlot& T = slot[i & 3];
+        const bool have = T.nseg != 0, prev = i != 0;
+
+        // ---- 1. decode ---------------------------------------------------------------
+        uint32_t n[S];
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            n[k] = 0;
+            if (!have) continue;  // uniform
+            const Table t{t1, symlen, a.jobs ? a.tables[T.job_id].t2() : tab.t2, T.index.shift, T.index.offset};
+            const uint32_t u = u0 + 32 * k;
             SegWords w;
             w.w0 = pre_q[k].x;
             w.w1 = pre_q[k].y;
@@ -364,144 +439,136 @@ __global__ void __launch_bounds__(kDecThreads, DecCfg<R, SEGS>::kMinBlocks)
             w.w3 = pre_q[k].w;
             const uint32_t up = __shfl_down_sync(kFull, pre_q[k].x, 1);
             w.w4 = lane == 31 ? pre_w4[k] : up;
-            const uint32_t col = tid + k * kDecThreads;
-            uint32_t cnt = 0;
-            if (have && col < nseg) {
-                const uint32_t pos = gap_at(col + 7) & (col ? ~0u : first_gap);
-                uint8_t* const row = stage + col * C::kRow;
-                if (last_tile && col + 1 == nseg) {
-                    cnt = decode_last_segment<COMPLETE, PAIRS, MULTI>(t1, t2, fl, w, pos,
-                                                                      end_last - 128 * col, row);
+            const uint32_t gap = (pre_gap[k] >> (4 * (u & 7))) & 0xfu;  // where the next segment's first code starts
+            const uint32_t before = __shfl_up_sync(kFull, gap, 1);
+            const uint32_t pos = lane == 0 ? pre_gap0[k] >> 28 : before;
+            const uint32_t row = smem_addr(row32 + 32 * k * C::kRowWords);
+            // (every wide book's tile takes the second branch: uniform over the CTA)
+            auto segment = [&](auto wide) {
+                constexpr bool WIDE = decltype(wide)::value;
+                if (T.last_bits && u + 1 == T.nseg) {
+                    n[k] = decode_last_segment<WIDE, COMPLETE, MULTI>(t, w, pos, T.last_bits, row);
                 } else {
-                    uint8_t* out = row;
-                    const uint32_t e = decode_segment<COMPLETE, PAIRS, MULTI>(t1, t2, fl, w, pos, out);
-                    cnt = (uint32_t)(out - row);
-                    if (e != 32 + gap_at(col + 8)) atomicOr(a.status, kDevCorrupt);
+                    const uint32_t end = decode_segment<WIDE, COMPLETE, PAIRS, MULTI>(t, w, pos, row, n[k]);
+                    if (end != 32 + gap) atomicOr(a.status, kDevCorrupt);
                 }
+            };
+            if (u < T.nseg && alive) {
+                if (COMPLETE && !T.index.wide) segment(std::integral_constant<bool, false>());
+                else segment(std::integral_constant<bool, true>());
             }
-            n[k] = cnt;
         }
-
-        // ---- 2. scan of the counts: both halves of the tile at once, packed in
-        //         16-bit fields (a warp's 32 segments hold < 2^13 symbols)
-        uint32_t packed = 0;
-#pragma unroll
-        for (int k = 0; k < C::kPer; ++k) packed |= n[k] << (16 * k);
+        // both segments' counts in one scan (a warp's 32 have less than 2^13 symbols)
+        uint32_t packed = n[0];
+        if (S > 1) packed |= n[S - 1] << 16;
         const uint32_t incl = warp_incl_scan(packed, lane);
-        if (lane == 31) warp_tot[warp] = incl;
-        if (tid == 0) {
-            if (have) fill_slot(ns, claim);
-            else slot[ns].item = ~0ull;
-        }
-        __syncthreads();  // (2) decode done; next tile known
-        const DecSlot& N = slot[ns];
-        const bool have_next = N.item < s_nitems;
-        const bool reload = a.jobs && have_next && N.job_id != s_lut_job;
-        if (reload) copy_tables_async(a.tables[N.job_id]);
-        const uint32_t wt = warp_incl_scan(lane < (uint32_t)C::kWarps ? warp_tot[lane] : 0u, lane);
-        const uint32_t totals = __shfl_sync(kFull, wt, C::kWarps - 1);
-        const uint32_t before = warp ? __shfl_sync(kFull, wt, warp - 1) : 0u;
-        const uint32_t total0 = totals & 0xffffu;
-        const uint32_t Ct = total0 + (totals >> 16);
-        const uint32_t ex = before + incl - packed;  // exclusive prefix, both fields
-        uint32_t excl[C::kPer];
-        excl[0] = ex & 0xffffu;
-        if (C::kPer > 1) excl[C::kPer - 1] = total0 + (ex >> 16);
-        if (tid == 0 && have && T.job.item0 + T.local + 1 != a.hook.hold_plus1)
-            lookback_publish(a.lookback, T.job.item0 + T.local, Ct, T.local == 0);
-        if (have_next) prefetch(N);  // in flight while prev is resolved and written
-        if (prev_s >= 0 && warp == 0) {
-            const DecSlot& Pv = slot[prev_s];
-            const uint64_t rec = Pv.job.item0 + Pv.local;
-            const uint64_t O = lookback_resolve<kDecLookK>(a.lookback, rec, prev_ct, Pv.local == 0, a.status, lane,
-                                                           wait_limit(a.hook), rec + 1 != a.hook.hold_plus1);
-            if (lane == 0) s_O = O;
-        }
-        __syncthreads();  // (3) prev's output offset known
-
-        // ---- 3. write out prev: 16-byte output chunk q takes compact bytes
-        //         [16q - base, 16q - base + 16), i.e. parts of two aligned groups
-        if (prev_s >= 0) {
-            const DecSlot& Pv = slot[prev_s];
-            const uint64_t O = s_O;
-            const uint32_t Cp = prev_ct;
-            const uint64_t nout = Pv.job.n;
-            if (tid == 0 && Pv.local + 1 == Pv.job.ntiles && O + Cp < nout) atomicOr(a.status, kDevSize);
-            if (O < nout) {
-                const uint64_t vstart = Pv.job.out_lo + O;
-                const uint32_t base = (uint32_t)(vstart & 15);  // compact byte 0 sits at chunk offset base
-                // tile-local byte positions from here on: [base, vend) of chunks 0..nq-1
-                const uint32_t vend = base + (O + Cp < nout ? Cp : (uint32_t)(nout - O));
-                const uint32_t nq = (vend + 15) >> 4;
-                uint8_t* const out0 = Pv.job.out_aligned + (vstart & ~15ull);  // 16-byte aligned
-                const uint32_t sh = 8 * (base & 3), sel = base >> 2;
-                auto comb = [sh](uint32_t lo, uint32_t hi) { return sh ? __funnelshift_r(lo, hi, 32 - sh) : hi; };
-                for (uint32_t lq = tid; lq < nq; lq += kDecThreads) {
-                    // aligned group lq holds chunk lq's bytes [base, 16) and chunk lq+1's
-                    // [0, base); group lq - 1 (for lq = 0 the stage's slack: bytes below
-                    // base, never stored) the rest
-                    const uint4 g = *reinterpret_cast<const uint4*>(compact + 16 * lq);
-                    const uint4 p = *reinterpret_cast<const uint4*>(compact + 16 * lq - 16);
-                    // output byte b = byte 16 - base + b of the 32-byte pair (p, g): output word i
-                    // joins words k and k+1 of (p.x..p.w, g.x..g.w), k = 3 - base/4 + i
-                    uint32_t o[4];
-                    switch (sel) {  // uniform over the tile
-                        case 0: o[0] = comb(p.w, g.x); o[1] = comb(g.x, g.y); o[2] = comb(g.y, g.z); o[3] = comb(g.z, g.w); break;
-                        case 1: o[0] = comb(p.z, p.w); o[1] = comb(p.w, g.x); o[2] = comb(g.x, g.y); o[3] = comb(g.y, g.z); break;
-                        case 2: o[0] = comb(p.y, p.z); o[1] = comb(p.z, p.w); o[2] = comb(p.w, g.x); o[3] = comb(g.x, g.y); break;
-                        default: o[0] = comb(p.x, p.y); o[1] = comb(p.y, p.z); o[2] = comb(p.z, p.w); o[3] = comb(p.w, g.x); break;
-                    }
-                    const uint32_t c0 = 16 * lq;
-                    if (c0 >= base && c0 + 16 <= vend) {
-                        *reinterpret_cast<uint4*>(out0 + c0) = make_uint4(o[0], o[1], o[2], o[3]);
-                    } else {  // the two ragged chunks
-#pragma unroll
-                        for (uint32_t b = 0; b < 16; ++b) {
-                            const uint32_t vb = c0 + b;
-                            if (vb >= base && vb < vend) out0[vb] = (uint8_t)(o[b >> 2] >> (8 * (b & 3)));
-                        }
-                    }
-                }
-            }
-        }
-        __syncthreads();  // (4) `compact` free again
-
-        // ---- 4. compact this tile at tile-local offsets (alignment applied on write-out)
+        const uint32_t sums = __shfl_sync(kFull, incl, 31);
+        const uint32_t sum0 = S > 1 ? sums & 0xffffu : sums, m = S > 1 ? sum0 + (sums >> 16) : sums;  // the warp's symbols
+        uint32_t before = 0;
+        bool reload = false;
         if (have) {
-#pragma unroll
-            for (int k = 0; k < C::kPer; ++k) {
-                // bytes up to the next word boundary of `compact` one by one, then whole
-                // words (two source words funnel-shifted), then the last bytes
-                const uint8_t* src = stage + (tid + k * kDecThreads) * C::kRow;
-                const uint32_t d = excl[k], m = n[k];
-                uint32_t h = (4u - (d & 3u)) & 3u;
-                if (h > m) h = m;
-                if (h > 0) compact[d] = src[0];
-                if (h > 1) compact[d + 1] = src[1];
-                if (h > 2) compact[d + 2] = src[2];
-                const uint32_t nwords = (m - h) >> 2;
-                const uint32_t* sw32 = reinterpret_cast<const uint32_t*>(src);
-                uint32_t* dw = reinterpret_cast<uint32_t*>(compact + d + h);
-                const uint32_t sh = 8 * h;
-                uint32_t lo = sw32[0];
-                for (uint32_t j = 0; j < nwords; ++j) {
-                    const uint32_t hi = sw32[j + 1];
-                    dw[j] = __funnelshift_r(lo, hi, sh);
-                    lo = hi;
+            if (lane == 0) tot[i & 1][warp] = m;
+            named_barrier(1, 32 * W);  // the counts are in place, the table is free
+            const uint32_t t = lane < (uint32_t)W ? tot[i & 1][lane] : 0u;
+            before = __reduce_add_sync(kFull, lane < warp ? t : 0u);
+            if (warp == 0) {
+                // the aggregate first: nothing that this CTA waits for may hold it back
+                const uint32_t Ct = __reduce_add_sync(kFull, t);
+                if (lane == 0) {
+                    if (T.rec + 1 != a.hook.hold_plus1) lookback_publish(a.lookback, T.rec, Ct, T.first);
+                    mbar_arrive(&published[i & 1]);
                 }
-                const uint32_t t = h + 4 * nwords, tl = m - t;  // 0..3 last bytes
-                if (tl > 0) compact[d + t] = src[t];
-                if (tl > 1) compact[d + t + 1] = src[t + 1];
-                if (tl > 2) compact[d + t + 2] = src[t + 2];
+            }
+            const DecSlot& N = slot[(i + 1) & 3];
+            if (!wait(filled, i + 1)) break;
+            reload = a.jobs && N.nseg && N.job_id != T.job_id;
+            prefetch(N);
+        }
+
+        // ---- 2. write out the tile before -----------------------------------------------
+        if (prev) {
+            if (!wait(placed, i - 1)) break;
+            uint8_t* const out = dst[(i & 1) ^ 1] + prev_before;
+            const uint32_t left = room[(i & 1) ^ 1];
+            uint32_t m = left > prev_before ? left - prev_before : 0u;
+            if (m > prev_m) m = prev_m;
+            uint32_t h = (0u - (uint32_t)reinterpret_cast<uintptr_t>(out)) & 15u;  // bytes before the first 16-byte group
+            if (h > m) h = m;
+            const uint32_t nq = (m - h) >> 4;
+            // the ragged ends: 16 lanes each
+            const uint32_t b = lane < 16 ? lane : h + 16 * nq + lane - 16;
+            if (b < (lane < 16 ? h : m)) out[b] = img[b];
+            const uint4* const src = reinterpret_cast<const uint4*>(img);
+            uint4* const out16 = reinterpret_cast<uint4*>(out + h);
+            const uint32_t sh = 8 * (h & 3);
+#pragma unroll 1
+            for (uint32_t c = lane; c < nq; c += 32) {
+                const uint4 p = src[c], g = src[c + 1];
+                uint4 o;
+                auto join = [sh](uint32_t lo, uint32_t hi) { return __funnelshift_r(lo, hi, sh); };
+                switch (h >> 2) {  // uniform over the warp
+                    case 0: o = make_uint4(join(p.x, p.y), join(p.y, p.z), join(p.z, p.w), join(p.w, g.x)); break;
+                    case 1: o = make_uint4(join(p.y, p.z), join(p.z, p.w), join(p.w, g.x), join(g.x, g.y)); break;
+                    case 2: o = make_uint4(join(p.z, p.w), join(p.w, g.x), join(g.x, g.y), join(g.y, g.z)); break;
+                    default: o = make_uint4(join(p.w, g.x), join(g.x, g.y), join(g.y, g.z), join(g.z, g.w)); break;
+                }
+                out16[c] = o;
             }
         }
-        if (have_next) {  // sg is no longer read for this tile
-            if (reload) cp_async_wait_all();
-            if (tid < (uint32_t)C::kGapStage) sg[tid] = pre_gap;
+
+        if (!have) break;
+
+        // ---- 3. this tile's rows to the image --------------------------------------------
+        {
+            prev_before = before;
+            prev_m = m;
+            uint32_t* to[S];
+            uint32_t full[S], rest[S], shift[S];
+            __syncwarp();  // the image is written out
+#pragma unroll
+            for (int k = 0; k < S; ++k) {
+                uint32_t* const r = row32 + 32 * k * C::kRowWords;
+                const uint32_t c = n[k];
+                const uint32_t d = k == 0 ? (incl & (S > 1 ? 0xffffu : ~0u)) - c : sum0 + (incl >> 16) - c;  // first byte
+                const uint32_t sh = 8 * (d & 3), whole = c >> 2;
+                shift[k] = sh;
+                full[k] = ((d & 3) + c) >> 2;
+                to[k] = reinterpret_cast<uint32_t*>(img) + (d >> 2);
+                // the row's word after the last whole one: what is past the count cleared
+                const uint32_t xl = r[whole] & ((1u << (8 * (c & 3))) - 1u);
+                r[whole] = xl;
+                // the lane's unfinished word
+                const uint32_t xk = whole ? r[whole - 1] : 0u;
+                rest[k] = full[k] > whole ? __funnelshift_l(xl, 0u, sh) : (xl << sh) | __funnelshift_l(xk, 0u, sh);
+                // the words that no lane completes: the last lane's, and in the stream's last tile, whose
+                // last segment may have fewer symbols, any lane's
+                if (T.last_bits || (k == S - 1 && lane == 31)) to[k][full[k]] = 0;
+            }
+            if (T.last_bits) __syncwarp();
+#pragma unroll
+            for (int k = 0; k < S; ++k) {
+                const uint32_t* const r = row32 + 32 * k * C::kRowWords;
+                const uint32_t sh = shift[k];
+                const uint32_t most = __reduce_max_sync(kFull, full[k]);
+                uint32_t cur = 0;
+#pragma unroll
+                for (int j = 0; j <= R; ++j) {
+                    if ((uint32_t)j >= most) break;  // uniform
+                    const uint32_t x = r[j];
+                    if ((uint32_t)j < full[k]) to[k][j] = cur | (x << sh);
+                    cur = __funnelshift_l(x, 0u, sh);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < S; ++k)
+                if (n[k]) atomicOr(to[k] + full[k], rest[k]);
+            __syncwarp();
         }
-        prev_s = have ? ti : -1;
-        prev_ct = Ct;
-        ti = ns;
+        if (reload) {
+            alive = mbar_wait(&tbar, copies & 1, a.status, false) && alive;
+            ++copies;
+        }
     }
 }
 
@@ -510,25 +577,28 @@ uint64_t decode_tiles(uint64_t segments, uint32_t min_len, uint32_t tile_segs) {
     return (segments + segs - 1) / segs;
 }
 
-template <int R, int SEGS, bool COMPLETE, bool PAIRS>
+template <int R, int W, int S, bool COMPLETE, bool PAIRS>
 static int launch_decode_r(const DecArgs& a, const DecTable& t, int ctas_per_sm, cudaStream_t st) {
-    using C = DecCfg<R, SEGS>;
-    auto kern = decode_kernel<R, SEGS, COMPLETE, PAIRS>;
+    using C = DecCfg<R, W, S>;
+    auto kern = decode_kernel<R, W, S, COMPLETE, PAIRS>;
     static LaunchCache cache;  // one per kernel instantiation
-    const LaunchFacts f = cache.get(reinterpret_cast<const void*>(kern), kDecThreads, C::kSmem);
+    const LaunchFacts f = cache.get(reinterpret_cast<const void*>(kern), C::kThreads, C::kSmem);
     if (f.err != cudaSuccess) return f.err;
     const int sms = f.sms, per_sm = f.per_sm;
     const int k = (ctas_per_sm > 0 && ctas_per_sm < per_sm) ? ctas_per_sm : per_sm;
     const uint64_t cap = (uint64_t)sms * k;
     const unsigned grid = (unsigned)(a.nitems_dev ? cap : (a.nitems < cap ? (a.nitems ? a.nitems : 1) : cap));
-    kern<<<grid, kDecThreads, C::kSmem, st>>>(a, t);
+    kern<<<grid, C::kThreads, C::kSmem, st>>>(a, t);
     return cudaGetLastError();
 }
 
 template <int R, bool COMPLETE, bool PAIRS>
 static int launch_decode_s(const DecArgs& a, const DecTable& t, int k, uint32_t tile_segs, cudaStream_t st) {
-    if (dec_tile_segs_for(R, tile_segs) == 512) return launch_decode_r<R, (R >= 32 ? 256 : 512), COMPLETE, PAIRS>(a, t, k, st);
-    return launch_decode_r<R, 256, COMPLETE, PAIRS>(a, t, k, st);
+    if (dec_tile_segs_for(R, tile_segs) == 512) {
+        if (R >= 16) return launch_decode_r<R, (R >= 32 ? 8 : 16), 1, COMPLETE, PAIRS>(a, t, k, st);
+        return launch_decode_r<R, 8, (R >= 16 ? 1 : 2), COMPLETE, PAIRS>(a, t, k, st);
+    }
+    return launch_decode_r<R, 8, 1, COMPLETE, PAIRS>(a, t, k, st);
 }
 
 template <bool COMPLETE, bool PAIRS>

@@ -49,32 +49,6 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
     return t;
 }
 
-// Waits until *p != 0 and returns it.  Bounded: once `limit_ns` of
-// %globaltimer have passed it flags kDevTimeout and returns `fallback`, so the
-// caller finishes its tile and the kernel exits; once a timeout is flagged,
-// every other wait gives up at once.  Other errors (a corrupt stream, a
-// missing codeword, ...) never stop a tile from publishing, so they do not end
-// a wait: a timeout is flagged only when a wait really expired, and in a batch
-// the healthy buffers still decode around a corrupt one.
-__device__ __forceinline__ uint64_t wait_nonzero(const uint64_t* p, uint32_t* status, uint64_t fallback,
-                                                 uint64_t limit_ns) {
-    uint64_t v = ld_relaxed_u64(p);
-    if (v != 0) return v;
-    const uint64_t t0 = global_timer_ns();
-    for (uint32_t it = 1;; ++it) {
-        v = ld_relaxed_u64(p);
-        if (v != 0) return v;
-        if ((it & 31) == 0) {
-            if (ld_relaxed_u32(status) & kDevTimeout) return fallback;
-            if (global_timer_ns() - t0 > limit_ns) {
-                atomicOr(status, kDevTimeout);
-                return fallback;
-            }
-            __nanosleep(64);
-        }
-    }
-}
-
 // ------------------------------------------- bulk copies into shared memory --
 // One-dimensional bulk copy (the TMA engine, no tensor map) from global to
 // this CTA's shared memory, completing on an mbarrier with a byte count.
@@ -111,6 +85,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// A barrier of `threads` of the CTA's threads (whole warps), the others not taking part.
+__device__ __forceinline__ void named_barrier(uint32_t id, uint32_t threads) {
+    asm volatile("barrier.sync.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 __device__ __forceinline__ void bulk_load(void* dst_smem, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
                  ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
@@ -118,14 +101,17 @@ __device__ __forceinline__ void bulk_load(void* dst_smem, const void* src, uint3
                  ::"r"(smem_addr(dst_smem)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
 }
 
+// The wait suspends the warp for about this long instead of spinning.
+constexpr uint32_t kTryWaitNs = 20000;
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
+        : "r"(smem_addr(bar)), "r"(parity), "r"(kTryWaitNs)
         : "memory");
     return ok != 0;
 }
@@ -180,14 +166,17 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, uint32_t lane) {
 
 // Single-pass decoupled look-back (the reference's scheme,
 // encoder/src/encoder.cu:222-263, decoder/src/decoder.cu:601-638) run by one
-// full warp, with a window of 32*K predecessors per round trip: lane
-// l holds tiles top-K*l ... top-K*l-K+1 (nearest first, window position
-// K*l + j).  The inclusive-prefix frontier advances at most one window per L2
+// full warp, with a window of 32*K predecessors per round trip: load j of lane
+// l is the tile at window position 32*j + l, counted from the nearest, so that a
+// load of the warp covers 256 consecutive bytes (with K consecutive records a
+// lane, 2 loads took twice the sectors and the decoder 4 % more time).  The inclusive-prefix frontier advances at most one window per L2
 // round trip, so the window must exceed the tiles started per round trip.
-// Only the records between the tile and the nearest inclusive prefix matter:
-// the window is loaded without blocking, and the warp waits only while an
-// unpublished record lies in front of the nearest inclusive prefix (on that
-// one record, bounded), then reloads.
+// Only the records between the tile and the nearest inclusive prefix matter.
+// The window is loaded without blocking; records in front of the nearest
+// unpublished one are summed at once and left behind, and the next window
+// starts at that one, so a wait costs one round trip after its record appears
+// (waiting for one record at a time and then loading the window again
+// took one of these cycles per late predecessor).
 // Publishing the aggregate and resolving the prefix are separate steps, so a
 // CTA can publish a tile's aggregate, decode its next tile, and resolve the
 // first tile afterwards, when its predecessors have long been published.
@@ -198,50 +187,51 @@ __device__ __forceinline__ void lookback_publish(uint64_t* rec, uint64_t tile, u
     st_relaxed_u64(rec + tile, (first ? kFlagP : kFlagA) | (agg & kValueMask));
 }
 
-// `limit_ns` bounds each wait; `publish` = false keeps the inclusive prefix
-// unpublished (the bounded-wait test hook only: LookbackHook).
+// `limit_ns` bounds the wait for each record; `publish` = false keeps the
+// inclusive prefix unpublished (the bounded-wait test hook only: LookbackHook).
 template <int K>
 __device__ __forceinline__ uint64_t lookback_resolve(uint64_t* rec, uint64_t tile, uint64_t agg, bool first,
                                                      uint32_t* status, uint32_t lane, uint64_t limit_ns,
                                                      bool publish = true) {
     if (first) return 0;
-    uint64_t excl = 0;
+    uint64_t excl = 0, t0 = 0;
     int64_t top = (int64_t)tile - 1;
     for (;;) {
         uint64_t v[K];
 #pragma unroll
         for (int j = 0; j < K; ++j) {
-            const int64_t i = top - (int64_t)(K * lane + j);
+            const int64_t i = top - (int64_t)(32 * j + lane);
             v[j] = i >= 0 ? ld_relaxed_u64(rec + i) : kFlagP;
         }
-        int first_p = K, first_z = K;  // nearest inclusive prefix / unpublished record of this lane
+        int gp = 32 * K, gz = 32 * K;  // the window's nearest inclusive prefix / unpublished record
 #pragma unroll
         for (int j = K - 1; j >= 0; --j) {
-            if (v[j] & kFlagP) first_p = j;
-            if (v[j] == 0) first_z = j;
+            const uint32_t pmask = __ballot_sync(kFull, (v[j] & kFlagP) != 0);
+            const uint32_t zmask = __ballot_sync(kFull, v[j] == 0);
+            if (pmask) gp = 32 * j + __ffs(pmask) - 1;
+            if (zmask) gz = 32 * j + __ffs(zmask) - 1;
         }
-        const uint32_t pmask = __ballot_sync(kFull, first_p < K);
-        const uint32_t zmask = __ballot_sync(kFull, first_z < K);
-        const int lp = pmask ? __ffs(pmask) - 1 : 32;
-        const int lz = zmask ? __ffs(zmask) - 1 : 32;
-        const int gp = lp < 32 ? K * lp + __shfl_sync(kFull, first_p, lp) : 32 * K;
-        const int gz = lz < 32 ? K * lz + __shfl_sync(kFull, first_z, lz) : 32 * K;
-        if (gz < gp) {  // an unpublished record in front of the nearest inclusive prefix
-            if ((int)lane == lz) {
-                const int64_t i = top - (int64_t)gz;
-                wait_nonzero(rec + i, status, kFlagP, limit_ns);
-            }
-            __syncwarp();
-            if (ld_relaxed_u32(status) & kDevTimeout) return excl;  // gave up: the status says so
-            continue;  // reload the same window
-        }
+        const int take = gz < gp ? gz : gp < 32 * K ? gp + 1 : 32 * K;  // records to sum
         uint64_t sum = 0;
 #pragma unroll
         for (int j = 0; j < K; ++j)
-            if ((int)(K * lane + j) <= gp) sum += v[j] & kValueMask;
+            if ((int)(32 * j + lane) < take) sum += v[j] & kValueMask;
         excl += warp_sum_u64(sum);
-        if (gp < 32 * K) break;
-        top -= 32 * K;
+        if (gp < gz) break;
+        top -= take;
+        if (take) {
+            t0 = 0;
+        } else {  // the nearest record is unpublished: bounded
+            const uint64_t now = global_timer_ns();
+            bool give_up = false;
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > limit_ns) give_up = true;
+            if (__any_sync(kFull, give_up)) {
+                if (lane == 0) atomicOr(status, kDevTimeout);
+                return excl;
+            }
+            if (ld_relaxed_u32(status) & kDevTimeout) return excl;  // given up elsewhere: the status says so
+        }
     }
     if (lane == 0 && publish) st_relaxed_u64(rec + tile, kFlagP | ((excl + agg) & kValueMask));
     return excl;

@@ -177,21 +177,20 @@ constexpr int kDecPrefix = 11;
 HGAP_HD constexpr int dec_stage_rows(uint32_t min_len) {
     return min_len >= 4 ? 8 : min_len == 3 ? 11 : min_len == 2 ? 16 : 32;
 }
-// Segments per decoder tile for a stage of R rows: two per thread, or one
-// per thread where the stage is large (R >= 16: it halves the stage and
-// compact areas so that more CTAs share an SM; measured 31 % faster for
-// R = 32, 3 % for R = 16, and 33 % slower for R = 11, where the per-tile
-// work then dominates).
-HGAP_HD constexpr int dec_tile_segs(int R) { return R >= 16 ? 256 : 512; }
+// Segments per decoder tile for a stage of R rows: 512, for which the tile's
+// fixed work (claim, look-back, barrier) counts least (256 MiB at 256 -> 512
+// segments: Zipf(1.2), R = 16, 401 -> 376 us; mixed, R = 11, 546 -> 428; BF16
+// mantissa, R = 8, 576 -> 385); 256 for 32 rows, whose 512-segment tile would
+// leave one CTA per SM.
+HGAP_HD constexpr int dec_tile_segs(int R) { return R >= 32 ? 256 : 512; }
 // The same with a launch-shape override of 256 or 512 segments (0: the
-// default).  32 stage rows keep 256: their 512-segment tile would leave one
-// CTA per SM.
+// default; 32 rows keep 256).
 HGAP_HD constexpr int dec_tile_segs_for(int R, uint32_t override_segs) {
     return R >= 32 ? 256 : (override_segs == 256 || override_segs == 512) ? (int)override_segs : dec_tile_segs(R);
 }
 constexpr int kDecT2Cap = 2560;  // >= the largest complete 16-bit book (see host.cpp)
 constexpr uint16_t kDecInvalid = 0x4000;
-struct DecTable {
+struct alignas(16) DecTable {
     uint16_t t1[1 << kDecPrefix];
     uint16_t t2[kDecT2Cap];
 };
@@ -204,17 +203,49 @@ struct DecTable {
 constexpr int kDecMultiMinRows = 32;
 HGAP_HD constexpr bool dec_multi(int rows, bool complete) { return complete && rows >= kDecMultiMinRows; }
 
-// The decode kernel's level-1 tables in their widened form (u32 entries: pair
-// form, or multi form for a complete book, with the length of the first code
-// per prefix), built once per buffer on the batched path so that a CTA moving
-// to another buffer's tile copies them into shared memory with 16-byte loads
-// instead of re-deriving every entry.  The level-2 table (its groups in use)
-// is read from here directly.
-struct DecTableW {
-    uint32_t t1[1 << kDecPrefix];
-    uint8_t l1[1 << kDecPrefix];
-    uint16_t t2[kDecT2Cap];
+// The decode kernel's table in shared memory.  A canonical code's long codes
+// are the last in code order, so ONE table serves all lengths: a 32-bit window
+// x at a code's start has the entry max(x >> 21, (x >> shift) + offset) -- below
+// the first prefix with codes of more than kDecPrefix bits its 11-bit prefix,
+// from there on its first kMaxLen (or the book's longest length) bits, counted
+// on from that prefix (both lines meet there, and the second is the steeper
+// one).  No second lookup, no branch.  Of 1500 books of the batched workload's
+// distributions 97 % (99.6 % of the bytes) fit dec_table_cap entries; the others
+// ("wide") keep two levels: 2048 entries, and a level-2 table in global memory
+// for the codes over 11 bits, reached by a branch.
+HGAP_HD constexpr uint32_t dec_table_cap(int rows) { return rows >= 32 ? 3840u : 2432u; }
+struct DecIndex {
+    uint32_t used;   // entries
+    uint32_t shift;  // of x
+    int32_t offset;
+    uint32_t wide;   // two levels instead
 };
+// From the first 11-bit prefix of a longer code (2048: none), the longest
+// length, and whether the book is complete (an incomplete one is wide: its
+// prefixes without a code have no place in one table).
+HGAP_HD inline DecIndex dec_index(uint32_t first_long, uint32_t max_len, bool complete, int rows) {
+    constexpr uint32_t n1 = 1u << kDecPrefix;
+    DecIndex d;
+    const uint32_t extra = max_len > (uint32_t)kDecPrefix && first_long < n1 ? max_len - kDecPrefix : 0u;
+    const uint32_t used = extra ? first_long + ((n1 - first_long) << extra) : n1;
+    d.wide = !complete || used > dec_table_cap(rows);
+    d.used = d.wide ? n1 : (used + 3) & ~3u;
+    d.shift = 32 - kDecPrefix - (d.wide ? 0u : extra);
+    d.offset = d.wide || !extra ? 0 : (int32_t)first_long - (int32_t)(first_long << extra);
+    return d;
+}
+
+// The same table in global memory, built once per buffer on the batched path
+// so that a CTA moving to another buffer's tile gets it (symlen and the used
+// entries) with one bulk copy.  A wide book's level-2 table is read from here.
+struct alignas(16) DecTableW {
+    DecIndex index;
+    uint8_t symlen[256];  // each symbol's code length
+    uint32_t t1[dec_table_cap(32)];
+    HGAP_HD uint16_t* t2() { return reinterpret_cast<uint16_t*>(t1 + (1 << kDecPrefix)); }
+    HGAP_HD const uint16_t* t2() const { return reinterpret_cast<const uint16_t*>(t1 + (1 << kDecPrefix)); }
+};
+static_assert(((1 << kDecPrefix) + kDecT2Cap / 2) <= (int)dec_table_cap(32), "level 2 of a wide book fits behind level 1");
 static_assert(sizeof(DecTableW) % 16 == 0, "16-byte copies");
 
 // One stream to decode (same single / batched scheme as EncJob).  Its tiles
@@ -239,6 +270,7 @@ struct DecArgs {
     const uint32_t* job_of;     // batched: [nitems] job of each tile of this launch
     const uint64_t* item0s;     // batched: [count] first tile of each job in this launch's numbering
     const DecTableW* tables;    // batched: [count]
+    DecIndex index;             // single path: the table's
     uint32_t count;
     uint64_t nitems;            // tiles in this launch
     const uint64_t* nitems_dev; // batched: the tile count in device memory (overrides nitems)

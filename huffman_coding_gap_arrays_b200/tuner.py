@@ -33,7 +33,7 @@ ENC_CTAS = (1, 2)
 # decoder CTAs per SM; each decoder is clamped to what fits it (5 for 256-segment tiles, 4 for
 # 512-segment ones, 3 for 32 stage rows), and 0 takes that maximum
 DEC_CTAS = (1, 2, 3, 4, 0)
-DEC_TILES = (0, 256, 512)  # decoder tile: by the book's shortest code (0), or 256 / 512 segments for all
+DEC_TILES = (0, 256, 512)  # decoder tile: the default (0), or 256 / 512 segments
 DEC_SPACE = tuple(itertools.product(DEC_CTAS, DEC_TILES))  # (CTAs per SM, tile) pairs
 
 
