@@ -1,61 +1,112 @@
 // host.cpp -- host-side half of the path: codebook construction, the
 // encoder/decoder tables the kernels take as launch parameters, and the
 // container format.  Pure C++ (no CUDA calls).
-#include <algorithm>
 #include <cstring>
-#include <vector>
 
 #include "hgap_internal.h"
 
 namespace {
 
-struct Leaf {
-    uint8_t symbol;
-    uint32_t count;
-};
+// The present bytes by ascending count, ties in byte order: key = count << 8 |
+// byte.  Radix sort by the counts' bytes (stable, and a histogram's keys come in
+// byte order); returns their number.
+uint32_t sorted_keys(const uint32_t hist[256], uint64_t key[256]) {
+    uint64_t tmp[256];
+    uint32_t n = 0, all = 0;
+    for (uint32_t b = 0; b < 256; ++b) {
+        key[n] = ((uint64_t)hist[b] << 8) | b;
+        n += hist[b] != 0;
+        all |= hist[b];
+    }
+    for (int shift = 8; shift < 40 && (all >> (shift - 8)) != 0; shift += 8) {
+        uint32_t at[256] = {};
+        for (uint32_t i = 0; i < n; ++i) ++at[(key[i] >> shift) & 0xff];
+        uint32_t sum = 0;
+        for (uint32_t d = 0; d < 256; ++d) {
+            const uint32_t c = at[d];
+            at[d] = sum;
+            sum += c;
+        }
+        for (uint32_t i = 0; i < n; ++i) tmp[at[(key[i] >> shift) & 0xff]++] = key[i];
+        std::memcpy(key, tmp, n * sizeof(uint64_t));
+    }
+    return n;
+}
 
 // Length-limited (16-bit) code lengths by package-merge, with the
 // reference's tie rule: a package precedes a leaf of equal weight
-// (encoder/src/package_merge.cpp:37,52,136).  `leaves` ascend by count.
-// Level 1 is the leaf list; level l merges the leaves with the pairwise
-// packages of level l-1; the top level keeps 2n-2 items.  Walking down from
-// the top, the leaves inside each level's active prefix gain one bit, and the
-// packages in it make the next level's active prefix twice as long.
-void package_merge(const std::vector<Leaf>& leaves, std::vector<uint8_t>& len) {
-    const int n = (int)leaves.size();
+// (encoder/src/package_merge.cpp:37,52,136).  `leaf` holds n >= 2 weights,
+// ascending.  Level 1 is the leaf list; level l merges the leaves with the
+// pairwise packages of level l-1 and keeps 2n-2 items.  Walking down from the
+// top, the leaves inside each level's active prefix gain one bit, and the
+// packages in it make the next level's active prefix twice as long; the leaves
+// in a prefix are counted by what the merge noted, how many leaves precede each
+// item.
+// A merge is a chain of dependent steps (compare, advance, load), so each level
+// is cut into kCuts pieces whose starts a binary search finds, and the pieces
+// are merged side by side: 256 leaves in 9 us where one chain over pushed-back
+// vectors took 40.
+void package_merge(const uint64_t* leaf, int n, uint8_t* len) {
+    constexpr int kCuts = 4, kMaxItems = 512;
+    constexpr uint64_t kNone = ~0ull;
     const int keep = 2 * n - 2;
-    struct Item {
-        uint64_t w;
-        bool pkg;
-    };
-    std::vector<std::vector<Item>> lvl(hgap::kMaxLen + 1);
-    lvl[1].reserve(n);
-    for (const Leaf& l : leaves) lvl[1].push_back({l.count, false});
+    uint64_t leaves[256 + 1], w[kMaxItems + 2], pk[kMaxItems / 2 + 1];
+    uint16_t before[hgap::kMaxLen + 1][kMaxItems + 1];  // [level][k]: leaves among the level's first k items
+    int size[hgap::kMaxLen + 1];
+    std::memcpy(leaves, leaf, n * sizeof(uint64_t));
+    leaves[n] = kNone;
+    std::memcpy(w, leaf, n * sizeof(uint64_t));
+    for (int k = 0; k <= n; ++k) before[1][k] = (uint16_t)k;
+    size[1] = n;
     for (int l = 2; l <= hgap::kMaxLen; ++l) {
-        const std::vector<Item>& below = lvl[l - 1];
-        std::vector<Item>& cur = lvl[l];
-        cur.reserve(keep);
-        const size_t npk = below.size() / 2;
-        size_t li = 0, pi = 0;
-        while ((int)cur.size() < keep && (li < (size_t)n || pi < npk)) {
-            const bool have_pkg = pi < npk;
-            const uint64_t pw = have_pkg ? below[2 * pi].w + below[2 * pi + 1].w : 0;
-            if (have_pkg && (li >= (size_t)n || pw <= leaves[li].count)) {
-                cur.push_back({pw, true});
-                ++pi;
-            } else {
-                cur.push_back({leaves[li].count, false});
-                ++li;
+        const int np = size[l - 1] / 2;
+        for (int j = 0; j < np; ++j) pk[j] = w[2 * j] + w[2 * j + 1];
+        pk[np] = kNone;
+        const int m = keep < n + np ? keep : n + np;
+        const int step = (m + kCuts - 1) / kCuts;
+        // leaves among the first d items: leaf i precedes package j iff its weight is smaller
+        int li[kCuts], pi[kCuts];
+        for (int c = 0; c < kCuts; ++c) {
+            const int d = c * step < m ? c * step : m;
+            int lo = d > np ? d - np : 0, hi = d < n ? d : n;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (leaves[mid] < pk[d - mid - 1]) lo = mid + 1;
+                else hi = mid;
             }
+            li[c] = lo;
+            pi[c] = d - lo;
         }
+        uint16_t* const bf = before[l];
+        auto one = [&](int c, int k) {
+            const uint64_t a = pk[pi[c]], b = leaves[li[c]];
+            bf[k] = (uint16_t)li[c];
+            const int take = a <= b;  // (whichever list has run out is kNone there: the other goes on)
+            w[k] = take ? a : b;
+            pi[c] += take;
+            li[c] += 1 - take;
+        };
+        const int full = m - (kCuts - 1) * step;  // the last piece's items
+        int k = 0;
+        for (; k < full; ++k)
+#pragma GCC unroll 4
+            for (int c = 0; c < kCuts; ++c) one(c, c * step + k);
+        for (; k < step; ++k)
+            for (int c = 0; c < kCuts; ++c)
+                if (c * step + k < m) one(c, c * step + k);
+        int leaves_in = 0;
+        for (int c = 0; c < kCuts; ++c)
+            if (c * step < m) leaves_in = li[c];
+        bf[m] = (uint16_t)leaves_in;
+        size[l] = m;
     }
-    len.assign(n, 0);
-    size_t active = keep;
+    std::memset(len, 0, n);
+    int active = keep;
     for (int l = hgap::kMaxLen; l >= 1 && active > 0; --l) {
-        size_t nleaf = 0, npkg = 0;
-        for (size_t k = 0; k < active && k < lvl[l].size(); ++k) (lvl[l][k].pkg ? npkg : nleaf)++;
-        for (size_t i = 0; i < nleaf; ++i) len[i]++;
-        active = 2 * npkg;
+        if (active > size[l]) active = size[l];
+        const int nleaf = before[l][active];
+        for (int i = 0; i < nleaf; ++i) len[i]++;
+        active = 2 * (active - nleaf);
     }
 }
 
@@ -199,21 +250,18 @@ uint64_t hgap_encoded_bits(const hgap_codebook* cb, const uint32_t hist[256]) {
 hgap_status hgap_codebook_build(const uint32_t hist[256], hgap_codebook* cb, hgap_sizes* sizes) {
     if (!hist || !cb) return HGAP_ERR_INVALID_ARG;
     std::memset(cb, 0, sizeof(*cb));
-    std::vector<Leaf> leaves;
-    for (int b = 0; b < 256; ++b)
-        if (hist[b]) leaves.push_back({(uint8_t)b, hist[b]});
-    std::stable_sort(leaves.begin(), leaves.end(),
-                     [](const Leaf& x, const Leaf& y) { return x.count < y.count; });
-    const uint32_t n = (uint32_t)leaves.size();
+    uint64_t key[256], weight[256];
+    const uint32_t n = sorted_keys(hist, key);
+    for (uint32_t i = 0; i < n; ++i) weight[i] = key[i] >> 8;
     cb->symbol_count = n;
-    std::vector<uint8_t> len;
+    uint8_t len[256];
     if (n == 1) {
-        len.assign(1, 1);  // defined here; the reference is undefined (package_merge.cpp:113-132)
+        len[0] = 1;  // defined here; the reference is undefined (package_merge.cpp:113-132)
     } else if (n >= 2) {
-        package_merge(leaves, len);
+        package_merge(weight, (int)n, len);
     }
     for (uint32_t i = 0; i < n; ++i) {  // container order: most frequent first (huff.cpp:114)
-        cb->symbols[i].symbol = leaves[n - 1 - i].symbol;
+        cb->symbols[i].symbol = (uint8_t)key[n - 1 - i];
         cb->symbols[i].length = len[n - 1 - i];
     }
     const hgap_status st = assign_codes(cb);
