@@ -273,12 +273,8 @@ hgap_status decode_impl(const uint32_t* d_bits, uint64_t words, const uint32_t* 
         s = hgap::make_dec_table(book, &cache.table);
         if (s != HGAP_OK) return s;
         // two symbols per lookup pay off once about a third of the lookups yield two
-        cache.pairs = hgap::dec_pair_fraction(cache.table) >= 0.3;
-        uint32_t first_long = 0, max_len = 0;
-        while (first_long < (1u << hgap::kDecPrefix) && !(cache.table.t1[first_long] & 0x8000u)) ++first_long;
-        for (uint32_t i = 0; i < book.symbol_count; ++i)
-            if (book.symbols[i].length > max_len) max_len = book.symbols[i].length;
-        cache.index = hgap::dec_index(first_long, max_len, complete, hgap::dec_stage_rows(min_len));
+        cache.pairs = hgap::dec_pair_fraction(book) >= 0.3;
+        cache.index = hgap::dec_index_of(book, complete, hgap::dec_stage_rows(min_len));
         cache.count = cb->symbol_count;
         std::memcpy(cache.symbols, cb->symbols, sizeof(hgap_symlen) * cache.count);
         cache.min_len = min_len;

@@ -290,7 +290,9 @@ int launch_decode(const DecArgs& a, const DecTable& t, uint32_t min_len, bool co
 // Fraction of level-1 entries that decode two symbols (the decoder's pair
 // rate under the code's own distribution, where every 11-bit prefix is
 // equally likely).
-double dec_pair_fraction(const DecTable& t);
+double dec_pair_fraction(const hgap_codebook& cb);
+// DecIndex of a book on the host.
+DecIndex dec_index_of(const hgap_codebook& cb, bool complete, int rows);
 // Tiles of a stream for a book whose shortest code is min_len bits (the
 // decoder's tile size depends on it, and on a tile-size override, 0: none);
 // min_len = 1 with 256-segment tiles gives the most.

@@ -194,20 +194,25 @@ hgap_status make_dec_table(const hgap_codebook& cb, DecTable* t) {
     return HGAP_OK;
 }
 
-double dec_pair_fraction(const DecTable& t) {
-    constexpr uint32_t P = kDecPrefix, mask = (1u << P) - 1u;
-    auto direct_len = [&](uint32_t x) -> uint32_t {  // 0 unless a valid direct entry
-        const uint16_t e = t.t1[x];
-        return (e & 0x8000u) || (e & kDecInvalid) ? 0u : ((e >> 8) & 15u) + 1u;
-    };
-    uint32_t pairs = 0;
-    for (uint32_t x = 0; x <= mask; ++x) {
-        const uint32_t l1 = direct_len(x);
-        if (l1 == 0 || l1 >= P) continue;
-        const uint32_t l2 = direct_len((x << l1) & mask);
-        if (l2 && l1 + l2 <= P) ++pairs;
+// From the numbers of codes of each length: a window of a pair has a first code
+// of l1 bits, a second of l2, and any 11 - l1 - l2 bits after them.
+double dec_pair_fraction(const hgap_codebook& cb) {
+    constexpr uint32_t P = kDecPrefix;
+    uint32_t of[kMaxLen + 1] = {}, pairs = 0;
+    for (uint32_t i = 0; i < cb.symbol_count; ++i) ++of[cb.symbols[i].length];
+    for (uint32_t l1 = 1; l1 < P; ++l1)
+        for (uint32_t l2 = 1; l1 + l2 <= P; ++l2) pairs += (of[l1] * of[l2]) << (P - l1 - l2);
+    return pairs / double(1u << P);
+}
+
+DecIndex dec_index_of(const hgap_codebook& cb, bool complete, int rows) {
+    uint32_t first_long = 0, max_len = 0;
+    for (uint32_t i = 0; i < cb.symbol_count; ++i) {
+        const uint32_t l = cb.symbols[i].length;
+        if (l <= (uint32_t)kDecPrefix) first_long += 1u << (kDecPrefix - l);
+        if (l > max_len) max_len = l;
     }
-    return pairs / double(mask + 1);
+    return dec_index(first_long, max_len, complete, rows);
 }
 
 }  // namespace hgap
