@@ -37,10 +37,16 @@
 namespace hgap {
 namespace {
 
-// Books (warps) per CTA of the book kernels: 14 KiB of scratch a book, so two a
-// CTA put 14 books on an SM (seven CTAs), where four a CTA fitted 12 (three).
+// Books (warps) per CTA of the book kernels.  A book is one warp's serial chain,
+// so its latency and the books in flight set the time: with 32-bit weights a
+// book's scratch takes 6.3 KiB and 32 books share an SM.  1024 books 69 -> 31 us,
+// 4096 books 158 -> 58 (64-bit weights throughout, 14 books an SM, both lists'
+// heads loaded in every merge step).  A book of kBook32 bytes or more takes
+// 64-bit weights and the whole CTA's scratch, after the CTA's other books.
 constexpr int kBookWarps = 2;
-constexpr size_t kBookSmem = kBookWarps * sizeof(BookScratch);
+using Book32 = BookScratch<uint32_t>;
+using Book64 = BookScratch<uint64_t>;
+constexpr size_t kBookSmem = kBookWarps * sizeof(Book32) > sizeof(Book64) ? kBookWarps * sizeof(Book32) : sizeof(Book64);
 constexpr int kScanThreads = 1024;
 constexpr uint32_t kClasses = 8;
 constexpr uint32_t kNoClass = 0xffu;
@@ -174,52 +180,77 @@ __global__ void __launch_bounds__(kScanThreads) benc_setup_kernel(uint32_t count
     }
 }
 
-// One warp per book: codebook from the buffer's histogram.  Optional outputs:
-// the public codebook, sizes, encoder table, batch entry.
-__global__ void __launch_bounds__(32 * kBookWarps) book_kernel(uint32_t count, const uint32_t* hists,
+// The codebook of histogram h, on one warp.  Optional outputs (book j's): the
+// public codebook, sizes, encoder table, batch entry.
+template <class W>
+__device__ __forceinline__ void make_book(const uint32_t* h, BookScratch<W>& s, uint32_t lane, uint32_t j,
+                                          hgap_codebook* books, hgap_sizes* sizes, EncTable* enc,
+                                          hgap_batch_entry* entries, const uint64_t* in_sizes) {
+    const uint32_t n = warp_code_lengths(h, s, lane);
+    warp_assign_codes(s, n, lane);
+    uint64_t part = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t b = lane + 32 * k;
+        part += (uint64_t)h[b] * s.blen[b];
+    }
+    const uint64_t bits = warp_sum_u64(part);
+    const uint64_t words = (bits + 31) / 32, segs = (bits + 127) / 128;
+    if (books) warp_write_book(s.syms, n, books + j, lane);
+    if (enc) warp_write_enc_table(s.syms, n, enc + j, lane);
+    if (sizes && lane == 0) {
+        sizes[j].bits = bits;
+        sizes[j].words = words;
+        sizes[j].segments = segs;
+        sizes[j].gap_words = (segs + 7) / 8;
+    }
+    if (entries) {
+        hgap_batch_entry& e = entries[j];
+        for (uint32_t c = lane; c < n; c += 32) {
+            e.symbols[c].symbol = s.syms.sym[c];
+            e.symbols[c].length = s.syms.clen[c];
+        }
+        if (lane == 0) {
+            e.n = in_sizes ? in_sizes[j] : 0;
+            e.bits = bits;
+            e.words = words;
+            e.segments = segs;
+            e.gap_words = (segs + 7) / 8;
+            e.symbol_count = n;
+            e.status = 0;
+        }
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(32 * kBookWarps, 16) book_kernel(uint32_t count, const uint32_t* hists,
                                                                hgap_codebook* books, hgap_sizes* sizes,
                                                                EncTable* enc, hgap_batch_entry* entries,
                                                                const uint64_t* in_sizes) {
     extern __shared__ __align__(16) unsigned char book_smem[];
-    BookScratch& s = reinterpret_cast<BookScratch*>(book_smem)[threadIdx.x >> 5];
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t j = blockIdx.x * kBookWarps + (threadIdx.x >> 5); j < count; j += gridDim.x * kBookWarps) {
-        const uint32_t* h = hists + 256 * (uint64_t)j;
-        const uint32_t n = warp_code_lengths(h, s, lane);
-        warp_assign_codes(s, n, lane);
-        uint64_t part = 0;
+    __shared__ uint32_t s_large[kBookWarps];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint64_t j0 = (uint64_t)blockIdx.x * kBookWarps; j0 < count; j0 += (uint64_t)gridDim.x * kBookWarps) {
+        const uint32_t j = (uint32_t)(j0 + warp);
+        bool large = false;
+        if (j0 + warp < count) {
+            const uint32_t* h = hists + 256 * (uint64_t)j;
+            uint64_t sum = 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t b = lane + 32 * k;
-            part += (uint64_t)h[b] * s.blen[b];
+            for (int k = 0; k < 8; ++k) sum += h[lane + 32 * k];
+            large = warp_sum_u64(sum) >= kBook32;
+            if (!large)
+                make_book(h, reinterpret_cast<Book32*>(book_smem)[warp], lane, j, books, sizes, enc, entries, in_sizes);
         }
-        const uint64_t bits = warp_sum_u64(part);
-        const uint64_t words = (bits + 31) / 32, segs = (bits + 127) / 128;
-        if (books) warp_write_book(s, n, books + j, lane);
-        if (enc) warp_write_enc_table(s, n, enc + j, lane);
-        if (sizes && lane == 0) {
-            sizes[j].bits = bits;
-            sizes[j].words = words;
-            sizes[j].segments = segs;
-            sizes[j].gap_words = (segs + 7) / 8;
+        if (lane == 0) s_large[warp] = large;
+        __syncthreads();
+        if (warp == 0) {
+            for (uint32_t k = 0; k < (uint32_t)kBookWarps; ++k)
+                if (s_large[k])
+                    make_book(hists + 256 * (j0 + k), *reinterpret_cast<Book64*>(book_smem), lane, (uint32_t)j0 + k, books,
+                              sizes, enc, entries, in_sizes);
         }
-        if (entries) {
-            hgap_batch_entry& e = entries[j];
-            for (uint32_t c = lane; c < n; c += 32) {
-                e.symbols[c].symbol = s.sym[c];
-                e.symbols[c].length = s.clen[c];
-            }
-            if (lane == 0) {
-                e.n = in_sizes ? in_sizes[j] : 0;
-                e.bits = bits;
-                e.words = words;
-                e.segments = segs;
-                e.gap_words = (segs + 7) / 8;
-                e.symbol_count = n;
-                e.status = 0;
-            }
-        }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -307,7 +338,7 @@ __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t c
                                                                    uint32_t* status) {
     constexpr uint32_t P = kDecPrefix, X = kMaxLen - kDecPrefix;  // 11, 5
     constexpr uint32_t kT1 = 1u << P, kPer = kT1 / kTableThreads;  // 8 prefixes a thread
-    __shared__ BookScratch s;
+    __shared__ BookSyms s;
     __shared__ __align__(16) uint16_t s1[kT1];
     __shared__ uint16_t s_end[kT1];  // level-2 offset after each prefix's group (0 for none)
     __shared__ uint32_t s_warp[kTableThreads / 32];
@@ -579,8 +610,8 @@ __global__ void bdec_map_kernel(uint32_t count, const DecJob* jobs, const uint8_
 // One warp per book: the decoder table of a public codebook.
 __global__ void __launch_bounds__(32 * kBookWarps) dec_table_kernel(uint32_t count, const hgap_codebook* books,
                                                                     uint16_t* tables, uint32_t* status) {
-    extern __shared__ __align__(16) unsigned char book_smem[];
-    BookScratch& s = reinterpret_cast<BookScratch*>(book_smem)[threadIdx.x >> 5];
+    __shared__ BookSyms scratch[kBookWarps];
+    BookSyms& s = scratch[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31;
     for (uint32_t j = blockIdx.x * kBookWarps + (threadIdx.x >> 5); j < count; j += gridDim.x * kBookWarps) {
         const uint32_t n = books[j].symbol_count;
@@ -718,8 +749,7 @@ hgap_status hgap_decode_table_build_device(uint32_t count, const hgap_codebook* 
                                            uint32_t* d_status, hgap_stream_t stream) {
     if (count == 0) return HGAP_OK;
     if (!d_books || !d_tables) return HGAP_ERR_INVALID_ARG;
-    if (set_book_smem(dec_table_kernel) != cudaSuccess) return HGAP_ERR_CUDA;
-    dec_table_kernel<<<book_grid(count), 32 * kBookWarps, kBookSmem, reinterpret_cast<cudaStream_t>(stream)>>>(
+    dec_table_kernel<<<book_grid(count), 32 * kBookWarps, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
         count, d_books, d_tables, d_status);
     return cuda_status(cudaGetLastError());
 }

@@ -9,13 +9,17 @@
 // order by count, the same package-merge tie rule, the same canonical codes
 // and the same two-level decoder table.
 //
-//   * sort: bitonic sort of (count << 8 | byte) keys, so equal counts keep
-//     byte order (what the reference's qsort yields on glibc);
+//   * sort: bitonic sort of (count << 8 | byte) keys in registers, eight a
+//     lane, so equal counts keep byte order (what the reference's qsort yields
+//     on glibc);
 //   * package-merge, L = 16: level l merges the sorted leaves with the pairwise
 //     packages of level l-1 (a package first on equal weight), keeping 2n-2
 //     items; each level is one merge-path step -- every lane finds where its
-//     16 outputs start by a binary search on its diagonal, then merges them;
-//     a 16-bit mask per lane records which items are packages;
+//     16 outputs start by a binary search on its diagonal, then merges them
+//     with one load a step, of whichever list it advanced (a book is a serial
+//     chain on one warp: 58 us while every step loaded the heads of both lists
+//     and summed a package); a 16-bit mask per lane records which items are
+//     packages;
 //   * lengths: walking down from level 16, the packages in a level's active
 //     prefix make the next level's active prefix twice as long; a leaf's
 //     length is the number of levels whose active prefix holds it;
@@ -35,23 +39,38 @@
 namespace hgap {
 
 // The package-merge lanes read items 16 apart (weights) and about 8 apart
-// (leaves): unpadded, a whole warp's 8-byte reads land in one bank pair (the
+// (leaves): unpadded, a whole warp's reads land in one or two banks (the
 // capture of one-warp-per-book showed two thirds of its shared wavefronts were
 // conflicts).  One pad slot per 16 weights and per 8 keys spreads them.
 __device__ __forceinline__ uint32_t wpad(uint32_t i) { return i + (i >> 4); }
 __device__ __forceinline__ uint32_t kpad(uint32_t i) { return i + (i >> 3); }
 
+// A book's symbols in container order: what the decoder's side needs.
+struct BookSyms {
+    uint32_t la[256];             // code << (16 - length)
+    uint8_t sym[256];             // bytes
+    uint8_t clen[256];            // lengths
+    uint32_t seen[8];             // bitmap of the bytes (warp_load_symbols)
+};
+
+// W: 32-bit weights where the counts' sum is below kBook32, 64-bit otherwise.  A
+// package's weight is at most 15 times that sum, and a key is count << 8 | byte
+// (the largest stands for an absent byte).
+template <class W>
 struct BookScratch {
-    uint64_t w[2][512 + 32];      // weights of two consecutive package-merge levels (at wpad)
-    uint64_t key[256 + 32];       // count << 8 | byte, ~0 for absent bytes; sorted in place (at kpad)
+    union {
+        W w[512 + 32];            // weights of one package-merge level (at wpad)
+        BookSyms syms;            // the result, once the weights are done with
+    };
+    W leaf[256 + 32 + 2];         // leaf weights, ascending (at kpad), then ~0
+    W pack[256 + 32 + 2];         // the level's packages (at kpad), then ~0
     uint16_t pk[kMaxLen + 1][32]; // bit b of pk[l][q]: item 16q+b of level l is a package
     uint16_t size[kMaxLen + 1];   // items kept at each level
-    uint32_t la[256];             // container order: code << (16 - length)
+    uint8_t order[256];           // ascending-count order: bytes
     uint8_t len[256];             // ascending-count order: code lengths
-    uint8_t sym[256];             // container order: bytes
-    uint8_t clen[256];            // container order: lengths
     uint8_t blen[256];            // per byte: code length (0: absent)
 };
+constexpr uint64_t kBook32 = (1u << 24) - 1;
 
 __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t lane, uint32_t* total) {
     const uint32_t incl = warp_incl_scan(v, lane);
@@ -59,34 +78,60 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t lane, ui
     return incl - v;
 }
 
-// Fills s.key (sorted) and s.len for the present bytes of `hist` and returns
-// their number n.  Leaf r (ascending count, ties by byte) is s.key[kpad(r)].
-__device__ inline uint32_t warp_code_lengths(const uint32_t* hist, BookScratch& s, uint32_t lane) {
-    uint32_t n = 0;
+// Sorts 256 keys, eight a lane (element 8 * lane + r in k[r]), ascending.
+template <class W>
+__device__ __forceinline__ void warp_sort256(W (&k)[8], uint32_t lane) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const uint32_t b = lane + 32 * j;
-        const uint32_t h = hist[b];
-        s.key[kpad(b)] = h ? (((uint64_t)h << 8) | b) : ~0ull;
-        n += __popc(__ballot_sync(kFull, h != 0));
-    }
-    __syncwarp();
-    // bitonic sort, ascending; absent bytes (~0) sink to the end
-    for (uint32_t k = 2; k <= 256; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+    for (uint32_t size = 2; size <= 256; size <<= 1) {
 #pragma unroll
-            for (uint32_t t = lane; t < 128; t += 32) {
-                const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1));
-                const uint32_t p = i + j;
-                const uint64_t x = s.key[kpad(i)], y = s.key[kpad(p)];
-                if ((x > y) == ((i & k) == 0)) {
-                    s.key[kpad(i)] = y;
-                    s.key[kpad(p)] = x;
+        for (uint32_t j = size >> 1; j > 0; j >>= 1) {
+            if (j >= 8) {  // partners in another lane
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const W o = __shfl_xor_sync(kFull, k[r], j >> 3);
+                    const bool up = ((8 * lane) & size) == 0, low = ((8 * lane) & j) == 0;
+                    k[r] = (up == low) == (o < k[r]) ? o : k[r];
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    if (r & j) continue;
+                    const bool up = size >= 8 ? ((8 * lane) & size) == 0 : (r & size) == 0;
+                    const W x = k[r], y = k[r + j];
+                    const bool swap = (y < x) == up;
+                    k[r] = swap ? y : x;
+                    k[r + j] = swap ? x : y;
                 }
             }
-            __syncwarp();
         }
     }
+}
+
+// Fills s.order and s.len for the present bytes of `hist` and returns their
+// number n (leaf r: ascending count, ties by byte).
+template <class W>
+__device__ inline uint32_t warp_code_lengths(const uint32_t* hist, BookScratch<W>& s, uint32_t lane) {
+    uint32_t n = 0;
+    {
+        W k[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t b = lane + 32 * j;
+            const uint32_t h = hist[b];
+            k[j] = h ? (((W)h << 8) | b) : ~(W)0;  // absent bytes sink to the end
+            n += __popc(__ballot_sync(kFull, h != 0));
+        }
+        warp_sort256(k, lane);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t r = 8 * lane + j;
+            s.order[r] = (uint8_t)k[j];
+            s.leaf[kpad(r)] = r < n ? k[j] >> 8 : ~(W)0;
+            if (r < n) s.w[wpad(r)] = k[j] >> 8;
+        }
+        if (lane == 0) s.leaf[kpad(256)] = ~(W)0;
+    }
+    __syncwarp();
     if (n == 1) {
         if (lane == 0) s.len[0] = 1;  // one symbol: a 1-bit code (the reference is undefined here)
         __syncwarp();
@@ -95,17 +140,19 @@ __device__ inline uint32_t warp_code_lengths(const uint32_t* hist, BookScratch& 
     if (n < 2) return n;
 
     const uint32_t keep = 2 * n - 2;
-    for (uint32_t r = lane; r < 512; r += 32) s.w[0][wpad(r)] = r < n ? (s.key[kpad(r)] >> 8) : 0;
     s.pk[1][lane] = 0;
     if (lane == 0) s.size[1] = (uint16_t)n;
-    __syncwarp();
     uint32_t prev_size = n;
-    int cur = 0;
     for (int l = 2; l <= kMaxLen; ++l) {
-        const uint64_t* below = s.w[cur];
-        uint64_t* out = s.w[cur ^ 1];
         const uint32_t np = prev_size / 2;
         const uint32_t m = keep < n + np ? keep : n + np;
+#pragma unroll
+        for (uint32_t t = 0; t < 8; ++t) {
+            const uint32_t j = lane + 32 * t;
+            if (j < np) s.pack[kpad(j)] = s.w[wpad(2 * j)] + s.w[wpad(2 * j + 1)];
+        }
+        if (lane == 0) s.pack[kpad(np)] = ~(W)0;
+        __syncwarp();  // the packages are made: w is free for this level's items
         const uint32_t d = 16 * lane;
         uint32_t mask = 0;
         if (d < m) {
@@ -113,28 +160,29 @@ __device__ inline uint32_t warp_code_lengths(const uint32_t* hist, BookScratch& 
             uint32_t lo = d > np ? d - np : 0, hi = d < n ? d : n;
             while (lo < hi) {
                 const uint32_t mid = (lo + hi) >> 1;
-                const uint32_t jj = d - mid - 1;
-                if ((s.key[kpad(mid)] >> 8) < below[wpad(2 * jj)] + below[wpad(2 * jj + 1)]) lo = mid + 1;
+                if (s.leaf[kpad(mid)] < s.pack[kpad(d - mid - 1)]) lo = mid + 1;
                 else hi = mid;
             }
             uint32_t i = lo, j = d - lo;
-            const uint32_t e = d + 16 < m ? d + 16 : m;
-            for (uint32_t pos = d; pos < e; ++pos) {
-                const uint64_t pw = j < np ? below[wpad(2 * j)] + below[wpad(2 * j + 1)] : 0;
-                if (j < np && (i >= n || pw <= (s.key[kpad(i)] >> 8))) {
-                    out[wpad(pos)] = pw;
-                    mask |= 1u << (pos - d);
-                    ++j;
-                } else {
-                    out[wpad(pos)] = s.key[kpad(i)] >> 8;
-                    ++i;
-                }
+            W lw = s.leaf[kpad(i)], pw = s.pack[kpad(j)];
+            const uint32_t cnt = m - d < 16 ? m - d : 16u;
+            W* const out = s.w + wpad(d);  // (16 items between two pad slots)
+#pragma unroll
+            for (uint32_t pos = 0; pos < 16; ++pos) {
+                if (pos >= cnt) break;
+                const bool take = pw <= lw;  // (the list that has run out is ~0)
+                out[pos] = take ? pw : lw;
+                mask |= (uint32_t)take << pos;
+                i += !take;
+                j += take;
+                const W next = *(take ? s.pack + kpad(j) : s.leaf + kpad(i));
+                lw = take ? lw : next;
+                pw = take ? next : pw;
             }
         }
         s.pk[l][lane] = (uint16_t)mask;
         if (lane == 0) s.size[l] = (uint16_t)m;
         prev_size = m;
-        cur ^= 1;
         __syncwarp();
     }
     // walk down: leaves in each level's active prefix gain one bit
@@ -162,9 +210,10 @@ __device__ inline uint32_t warp_code_lengths(const uint32_t* hist, BookScratch& 
 }
 
 // Container order from ascending order (symbol i = leaf n-1-i) and the
-// canonical codes, into s.sym / s.clen / s.la, plus the per-byte lengths
-// s.blen.  Returns the Kraft sum in units of 2^-16 (65536: a complete book).
-__device__ inline uint32_t warp_assign_codes(BookScratch& s, uint32_t n, uint32_t lane) {
+// canonical codes, into s.syms, plus the per-byte lengths s.blen.  Returns the
+// Kraft sum in units of 2^-16 (65536: a complete book).
+template <class W>
+__device__ inline uint32_t warp_assign_codes(BookScratch<W>& s, uint32_t n, uint32_t lane) {
     for (uint32_t b = lane; b < 256; b += 32) s.blen[b] = 0;
     __syncwarp();
     uint32_t kr[8], tot = 0;
@@ -175,9 +224,9 @@ __device__ inline uint32_t warp_assign_codes(BookScratch& s, uint32_t n, uint32_
         if (c < n) {
             const uint32_t r = n - 1 - c;
             const uint32_t L = s.len[r];
-            const uint32_t sym = (uint32_t)(s.key[kpad(r)] & 0xff);
-            s.sym[c] = (uint8_t)sym;
-            s.clen[c] = (uint8_t)L;
+            const uint32_t sym = s.order[r];
+            s.syms.sym[c] = (uint8_t)sym;
+            s.syms.clen[c] = (uint8_t)L;
             s.blen[sym] = (uint8_t)L;
             kr[t] = 1u << (kMaxLen - L);
         }
@@ -188,7 +237,7 @@ __device__ inline uint32_t warp_assign_codes(BookScratch& s, uint32_t n, uint32_
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
         const uint32_t c = 8 * lane + t;
-        if (c < n) s.la[c] = run;
+        if (c < n) s.syms.la[c] = run;
         run += kr[t];
     }
     __syncwarp();
@@ -196,7 +245,7 @@ __device__ inline uint32_t warp_assign_codes(BookScratch& s, uint32_t n, uint32_
 }
 
 // The book in the public layout (symbols in container order, per-byte table).
-__device__ inline void warp_write_book(const BookScratch& s, uint32_t n, hgap_codebook* cb, uint32_t lane) {
+__device__ inline void warp_write_book(const BookSyms& s, uint32_t n, hgap_codebook* cb, uint32_t lane) {
     for (uint32_t b = lane; b < 256; b += 32) {
         cb->table[b].code = 0;
         cb->table[b].length = 0;
@@ -214,7 +263,7 @@ __device__ inline void warp_write_book(const BookScratch& s, uint32_t n, hgap_co
 }
 
 // The encoder's per-byte table (code | length << 16, kEncAbsent if absent).
-__device__ inline void warp_write_enc_table(const BookScratch& s, uint32_t n, EncTable* t, uint32_t lane) {
+__device__ inline void warp_write_enc_table(const BookSyms& s, uint32_t n, EncTable* t, uint32_t lane) {
     for (uint32_t b = lane; b < 256; b += 32) t->e[b] = kEncAbsent;
     __syncwarp();
     for (uint32_t c = lane; c < n; c += 32) {
@@ -227,10 +276,10 @@ __device__ inline void warp_write_enc_table(const BookScratch& s, uint32_t n, En
 // The same container-order arrays from a given symbol list (decoder side).
 // Returns the Kraft sum, or ~0u if the list is not a valid canonical book
 // (a length outside 1..16, a repeated byte, lengths not ascending, Kraft > 1).
-__device__ inline uint32_t warp_load_symbols(const hgap_symlen* syms, uint32_t n, BookScratch& s, uint32_t lane) {
+__device__ inline uint32_t warp_load_symbols(const hgap_symlen* syms, uint32_t n, BookSyms& s, uint32_t lane) {
     uint32_t kr[8], tot = 0;
     bool bad = n > 256;
-    if (lane < 8) s.key[lane] = 0;  // byte-seen bitmap: 256 bits in key[0..3]
+    if (lane < 8) s.seen[lane] = 0;
     __syncwarp();
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
@@ -242,8 +291,8 @@ __device__ inline uint32_t warp_load_symbols(const hgap_symlen* syms, uint32_t n
             s.clen[c] = (uint8_t)L;
             if (L < 1 || L > (uint32_t)kMaxLen) bad = true;
             else kr[t] = 1u << (kMaxLen - L);
-            const unsigned long long bit = 1ull << (sym & 63);
-            if (atomicOr(reinterpret_cast<unsigned long long*>(&s.key[sym >> 6]), bit) & bit) bad = true;
+            const uint32_t bit = 1u << (sym & 31);
+            if (atomicOr(&s.seen[sym >> 5], bit) & bit) bad = true;
         }
         tot += kr[t];
     }
@@ -267,7 +316,7 @@ __device__ inline uint32_t warp_load_symbols(const hgap_symlen* syms, uint32_t n
 // Decoder table (layout in hgap_internal.h) from the container-order arrays
 // s.la / s.sym / s.clen of n >= 1 symbols.  Returns false if the level-2 part
 // would exceed kDecT2Cap (only possible for an incomplete book).
-__device__ inline bool warp_dec_table(const BookScratch& s, uint32_t n, DecTable* t, uint32_t lane) {
+__device__ inline bool warp_dec_table(const BookSyms& s, uint32_t n, DecTable* t, uint32_t lane) {
     constexpr uint32_t P = kDecPrefix, X = kMaxLen - kDecPrefix;  // 11, 5
     // symbol index of the largest left-aligned code <= v, starting from i
     auto advance = [&](uint32_t i, uint32_t v) {
