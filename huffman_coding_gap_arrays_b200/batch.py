@@ -24,8 +24,8 @@ from .codec import Codebook, Compressed, StreamSizes, _stream
 
 ENTRY_BYTES = C.sizeof(BatchEntry)
 # Kernels one batched call launches (csrc/batch.cu): compress = benc_setup, hist_st, book,
-# benc_place, encode; decompress = bdec_table, bdec_setup, bdec_map and one decoder per class (8).
-COMPRESS_KERNELS = 5
+# benc_place, enc_plan, encode; decompress = bdec_table, bdec_setup, bdec_map and one decoder per class (8).
+COMPRESS_KERNELS = 6
 DECOMPRESS_KERNELS = 11
 
 

@@ -32,15 +32,14 @@ hgap_status hgap_histogram(const void* d_in, uint64_t n, uint32_t* d_hist, hgap_
 
 size_t hgap_encode_workspace_bytes(uint64_t n) {
     const uint64_t nst = hgap::encode_super_tiles_cap(n);  // every input of up to n bytes, any alignment
-    return hgap::kEncWsHeader + (size_t)nst * (sizeof(uint64_t) + 256 * sizeof(uint32_t));
+    return hgap::encode_workspace(nst).bytes;
 }
 
 }  // extern "C"
 
 namespace {
 
-// Carves the encoder workspace for input (d_in, n):
-// [status][counter][..][tag @16][scratch hist @1024][st_rec @2048][st_hist].
+// Carves the encoder workspace for input (d_in, n) (EncWorkspace).
 hgap_status encode_layout(const void* d_in, uint64_t n, void* d_workspace, size_t workspace_bytes,
                           hgap::EncArgs* a, hgap::HistStArgs* h) {
     if (!d_in || !d_workspace || !aligned(d_workspace, 16)) return HGAP_ERR_INVALID_ARG;
@@ -49,8 +48,8 @@ hgap_status encode_layout(const void* d_in, uint64_t n, void* d_workspace, size_
     const uint64_t st_bytes = hgap::encode_st_chunks(n) * hgap::kEncChunkBytes;
     const uint64_t nst = hgap::encode_super_tiles(lo + n, n);
     if (nst >= 0xffffffffull) return HGAP_ERR_UNSUPPORTED;
-    const size_t need = hgap::kEncWsHeader + (size_t)nst * (sizeof(uint64_t) + 256 * sizeof(uint32_t));
-    if (workspace_bytes < need) return HGAP_ERR_WORKSPACE;
+    const hgap::EncWorkspace w = hgap::encode_workspace(nst);
+    if (workspace_bytes < w.bytes) return HGAP_ERR_WORKSPACE;
     uint8_t* ws = static_cast<uint8_t*>(d_workspace);
     std::memset(a, 0, sizeof(*a));
     std::memset(h, 0, sizeof(*h));
@@ -65,15 +64,17 @@ hgap_status encode_layout(const void* d_in, uint64_t n, void* d_workspace, size_
     a->nitems = nst;
     a->status = reinterpret_cast<uint32_t*>(ws);
     a->counter = reinterpret_cast<uint32_t*>(ws) + 1;
-    a->tag = reinterpret_cast<const uint64_t*>(ws + hgap::kEncWsTag);
-    a->st_rec = reinterpret_cast<uint64_t*>(ws + hgap::kEncWsHeader);
-    a->st_hist = reinterpret_cast<const uint32_t*>(a->st_rec + nst);
+    a->nitems_dev = reinterpret_cast<uint64_t*>(ws + 8);
+    a->tag = reinterpret_cast<const uint64_t*>(ws + w.tag);
+    a->st_rec = reinterpret_cast<uint64_t*>(ws + w.st_rec);
+    a->plan = reinterpret_cast<hgap::EncRegion*>(ws + w.plan);
+    a->st_hist = reinterpret_cast<const uint32_t*>(ws + w.st_hist);
     h->single = J;
     h->count = 1;
     h->nitems = nst;
-    h->hist = reinterpret_cast<uint32_t*>(ws + hgap::kEncWsScratchHist);
+    h->hist = reinterpret_cast<uint32_t*>(ws + w.scratch);
     h->st_hist = const_cast<uint32_t*>(a->st_hist);
-    h->tag = reinterpret_cast<uint64_t*>(ws + hgap::kEncWsTag);
+    h->tag = reinterpret_cast<uint64_t*>(ws + w.tag);
     return HGAP_OK;
 }
 
@@ -95,13 +96,10 @@ hgap_status encode_outputs(const hgap_codebook* cb, uint32_t* d_bits, uint64_t w
     return HGAP_OK;
 }
 
-// Clears status + counter, and the super-tile look-back records.
+// Clears what a call starts from; with `tag_too` also the tag and the scratch histogram.
 hgap_status encode_clear(const hgap::EncArgs& a, bool tag_too, cudaStream_t st) {
-    uint8_t* ws = reinterpret_cast<uint8_t*>(a.status);
-    if (cudaMemsetAsync(ws, 0, tag_too ? hgap::kEncWsHeader : hgap::kEncWsTag, st) != cudaSuccess)
-        return HGAP_ERR_CUDA;
-    if (cudaMemsetAsync(a.st_rec, 0, sizeof(uint64_t) * a.nitems, st) != cudaSuccess) return HGAP_ERR_CUDA;
-    return HGAP_OK;
+    const hgap::EncWorkspace w = hgap::encode_workspace(a.nitems);
+    return cudaMemsetAsync(a.status, 0, tag_too ? w.plan : w.tag, st) == cudaSuccess ? HGAP_OK : HGAP_ERR_CUDA;
 }
 
 }  // namespace

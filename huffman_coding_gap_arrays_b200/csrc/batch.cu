@@ -9,8 +9,10 @@
 //                   encoder table, sizes (book.cuh);
 //   4. benc_place   one CTA: scans of the stream sizes place every bitstream
 //                   (16-byte aligned) and gap array in the two arenas;
-//   5. encode       the single-buffer encoder kernel over all regions, the
-//                   CTA reloading its code tables when the buffer changes.
+//   5. enc_plan     one warp per region: bit count, first output bit, all that
+//                   a CTA needs to start on it;
+//   6. encode       the single-buffer encoder kernel over all regions, the
+//                   CTA reloading its code table when the buffer changes.
 // Decompress:
 //   1. bdec_table   one CTA per buffer: checks the book, writes its decoder
 //                   table in the form the decode kernel keeps in shared
@@ -657,12 +659,12 @@ uint32_t base_chunks(const hgap_batch_config* cfg) {
 }
 
 // Compress workspace: [header 1024: status @0, counter @4, nitems @64]
-// [jobs] [item0s] [tables] [hists] then the per-region arrays [st_rec | st_hist]
+// [jobs] [item0s] [tables] [hists] then the per-region arrays [st_rec | plan | st_hist]
 // for as many regions as the rest of the workspace holds.
-constexpr size_t kEncPerRegion = 8 + 1024;
+constexpr size_t kEncPerRegion = 8 + sizeof(EncRegion) + 1024;
 
 struct EncLayout {
-    size_t jobs, item0s, tables, hists, st_rec, st_hist, fixed;
+    size_t jobs, item0s, tables, hists, st_rec, plan, st_hist, fixed;
     uint64_t max_regions;
 };
 
@@ -678,9 +680,10 @@ EncLayout enc_layout(uint32_t count, size_t workspace_bytes) {
     L.hists = off;
     off = align256(off + 1024 * (size_t)count);
     L.fixed = off;
-    L.max_regions = workspace_bytes > off + 256 ? (workspace_bytes - off - 256) / kEncPerRegion : 0;
+    L.max_regions = workspace_bytes > off + 512 ? (workspace_bytes - off - 512) / kEncPerRegion : 0;
     L.st_rec = off;
-    L.st_hist = align256(off + 8 * (size_t)L.max_regions);
+    L.plan = align256(off + 8 * (size_t)L.max_regions);
+    L.st_hist = align256(L.plan + sizeof(EncRegion) * (size_t)L.max_regions);
     return L;
 }
 
@@ -802,6 +805,7 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
     uint32_t* hists = reinterpret_cast<uint32_t*>(ws + L.hists);
     uint64_t* st_rec = reinterpret_cast<uint64_t*>(ws + L.st_rec);
     uint32_t* st_hist = reinterpret_cast<uint32_t*>(ws + L.st_hist);
+    EncRegion* plan = reinterpret_cast<EncRegion*>(ws + L.plan);
 
     if (cudaMemsetAsync(ws, 0, 1024, st) != cudaSuccess) return HGAP_ERR_CUDA;
     if (cudaMemsetAsync(hists, 0, 1024 * (size_t)count, st) != cudaSuccess) return HGAP_ERR_CUDA;
@@ -835,7 +839,9 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
     a.item0s = item0s;
     a.tables = tables;
     a.count = count;
+    a.nitems = L.max_regions;
     a.nitems_dev = nitems;
+    a.plan = plan;
     a.st_rec = st_rec;
     a.st_hist = st_hist;
     a.counter = status + 1;

@@ -8,10 +8,10 @@
 // run one job, the batched ones thousands, each with its own codebook (the
 // CTA reloads its code table when the job changes).  A region's bit count is
 // one dot product of its histogram (recorded by hist_st_kernel in the same
-// pass that builds the global histogram) with the code lengths, so a single
-// bounded look-back over regions gives its first output bit G.  A CTA claims
-// its next region one ahead and publishes that one's bit count at once, so no
-// look-back ever waits on a claimed region.
+// pass that builds the global histogram) with the code lengths, so a small
+// kernel before the encoder gives every region's first output bit G
+// (enc_plan_kernel).  A CTA holds its next region's plan and claims the one
+// after it while it encodes; nothing in the encoder waits for another CTA.
 //
 // Input: steps of 16 KiB are staged in a ring of shared-memory buffers by 1-D
 // bulk copies (completion on an mbarrier), one step ahead of the one being
@@ -88,84 +88,24 @@ constexpr size_t kEncSmem = (size_t)256 * kLutRep * 8 + (size_t)kRing * kStepByt
 constexpr uint32_t kLen4 = 0x01010101u;
 constexpr uint32_t kPieceBias = 0x7f7f7f7fu;  // 0x7f + running length per byte
 
-// What the steps of a region need of it, in shared memory.  Bit positions are
-// 32-bit, relative to the start of the gap word (1024 bits, so also of the
-// 16-byte group of output words) that holds the region's first bit; a region
-// has at most 2^22 bits.
-struct Region {
-    uint32_t* bits;             // output and gap words from there on,
-    uint32_t* gaps;
-    uint32_t nwords, ngaps;     // and how many of them exist
-    uint32_t first_bit;         // the region's first bit
-    uint32_t lo, hi;            // its bytes: [lo, hi) from a multiple of 16
-    bool first, last;           // in its job
-    bool vec;                   // output words are 16-byte aligned
-};
-
 struct EncShared {
     uint64_t mbar[kRing];       // one per ring buffer: its bulk copy landed
-    EncJob job[2];              // slots: the current region's job and the next claimed one's
-    uint64_t item[2];           // their global region ids (>= nitems: none)
-    uint64_t agg[2];            // their bit counts
-    uint32_t job_id[2];
-    uint64_t G;                 // first output bit of the current region
-    Region reg;
-    uint32_t gap_head;          // spill at the segment end before G (for a first entry that is odd)
+    EncRegion reg[3];           // the CTA's k-th region in reg[k % 3]: the current one, the next, the one after
+    EncTable next_codes;        // the next region's codes, if they are another job's
     uint32_t tot[2][kEncWarps]; // per step parity: the warps' bit counts
     // the last 32 code bits before warp w's first of step c, at [(16 c + w) % 64]: four steps, since
     // warp 0 still reads its entry when warp 15 is a step further
     uint32_t tail[4 * kEncWarps];
-    uint64_t nitems;            // regions of the launch
     uint32_t lut_job;           // job whose codes are in the table
-    uint32_t abort;
     uint32_t p_issued;          // producer: copies issued so far (step sequence number)
     uint32_t p_step;            // producer: step index of the next copy within its region
     int p_which;                // producer: next copy from the current region (0) or the next one (1)
 };
 
-// Length and left-aligned code of `byte` from a job's table in global memory.
-__device__ __forceinline__ void code_of(const EncTable* t, uint32_t byte, uint32_t& c, uint32_t& len) {
-    const uint32_t e = t->e[byte];
+// Length and left-aligned code of an entry of a job's table.
+__device__ __forceinline__ void code_of(uint32_t e, uint32_t& c, uint32_t& len) {
     len = (e >> 16) & 31u;
     c = len ? (e & 0xffffu) << (32 - len) : 0u;
-}
-
-// Warp 0: claims a region into `slot`, copies its job there and publishes
-// its bit count at once, so that no later region's look-back waits on it.
-__device__ __forceinline__ void claim_region(const EncArgs& a, const uint2* lut, EncShared& sh, int slot,
-                                             uint32_t lane) {
-    uint32_t c = 0;
-    if (lane == 0) c = atomicAdd(a.counter, 1u);
-    const uint64_t item = __shfl_sync(kFull, c, 0);
-    uint32_t job = 0;
-    uint64_t agg = 0;
-    __syncwarp();  // every lane is done reading the slot
-    if (item < sh.nitems) {
-        if (a.jobs) job = find_job(a.item0s, a.count, item);
-        const EncJob* src = a.jobs ? a.jobs + job : &a.single;
-        static_assert(sizeof(EncJob) % 8 == 0 && sizeof(EncJob) <= 256, "job copied as u64 lanes");
-        if (lane < sizeof(EncJob) / 8)
-            reinterpret_cast<uint64_t*>(&sh.job[slot])[lane] = reinterpret_cast<const uint64_t*>(src)[lane];
-        uint64_t part = 0;
-        bool absent = false;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t b = lane + 32 * j;
-            const uint32_t len = a.jobs ? ((a.tables[job].e[b] >> 16) & 31u) : lut[b * kLutRep].y;
-            const uint32_t n = a.st_hist[item * 256 + b];
-            absent |= n != 0 && len == 0;
-            part += (uint64_t)n * len;
-        }
-        if (absent) atomicOr(a.status, kDevNoCode);
-        agg = warp_sum_u64(part);
-        if (lane == 0 && item + 1 != a.hook.hold_plus1) lookback_publish(a.st_rec, item, agg, item == src->item0);
-    }
-    if (lane == 0) {
-        sh.item[slot] = item;
-        sh.agg[slot] = agg;
-        sh.job_id[slot] = job;
-    }
-    __syncwarp();
 }
 
 // End of region st of job J (virtual input index, like J.lo / J.hi).
@@ -174,38 +114,188 @@ __device__ __forceinline__ uint64_t region_end(const EncJob& J, uint64_t st) {
     return v1 < J.hi ? v1 : J.hi;
 }
 
-__device__ __forceinline__ uint32_t region_steps(const EncJob& J, uint64_t st) {
-    return (uint32_t)((region_end(J, st) - st * (uint64_t)J.st_bytes + kStepBytes - 1) / kStepBytes);
+constexpr int kPlanThreads = 256;
+constexpr int kPlanWarps = kPlanThreads / 32;  // regions of a group
+constexpr int kPlanLookK = 1;
+
+// One warp per region: its bit count (its histogram times the code lengths),
+// its first output bit, and by re-encoding a few bytes backwards from there
+// what precedes it in its first word and gap byte.  The counts are summed over a
+// CTA's eight regions first, and the look-back runs over these groups (over
+// single regions it took 13 us for the 1171 regions of 256 MiB, here 8): a
+// group in which a job starts publishes the sum from there on as an inclusive
+// prefix.  Groups of one CTA ascend, so a look-back only ever waits for CTAs
+// that are running.
+// All the regions' dependent loads overlap here, where one warp of a persistent
+// encoder CTA went through them between two regions: encoder and plan of 1024
+// buffers in 64 KiB regions 659 -> 543 us, of 4096 small buffers 170 -> 126, of
+// one 16 MiB buffer 25 -> 26; one 256 MiB buffer pays its 8 us (237 -> 249).
+__global__ void __launch_bounds__(kPlanThreads) enc_plan_kernel(const __grid_constant__ EncArgs a,
+                                                                const __grid_constant__ EncTable tab) {
+    __shared__ EncTable s_tab;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    uint64_t nitems = a.nitems;
+    if (a.jobs) {
+        nitems = *a.nitems_dev;
+    } else {
+        s_tab.e[tid] = tab.e[tid];
+        __syncthreads();
+        // single path: the histograms in the workspace must come from this very input
+        const bool fits = a.tag[0] == a.single.hi - a.single.lo &&
+                          a.tag[1] == reinterpret_cast<uint64_t>(a.single.in_aligned) + a.single.lo;
+        if (blockIdx.x == 0 && tid == 0) {
+            *a.nitems_dev = fits ? nitems : 0;
+            if (!fits) atomicOr(a.status, kDevPlan);
+        }
+        if (!fits) return;
+    }
+    __shared__ uint64_t s_agg[kPlanWarps], s_excl;
+    __shared__ uint32_t s_first[kPlanWarps];
+    const uint32_t warp = tid >> 5;
+    for (uint64_t g = blockIdx.x; g * kPlanWarps < nitems; g += gridDim.x) {
+        const uint64_t item = g * kPlanWarps + warp;
+        const bool valid = item < nitems;  // uniform over the warp
+        uint32_t job = 0;
+        if (a.jobs && valid) {  // the last job with item0 <= item: 32 probes a round
+            uint32_t lo = 0, hi = a.count;
+            while (hi - lo > 1) {
+                const uint32_t step = (hi - lo + 31) / 32, at = lo + lane * step;
+                const uint32_t le = __ballot_sync(kFull, at < hi && a.item0s[at] <= item);  // lane 0's always is
+                const uint32_t k = 31 - __clz(le);
+                lo += k * step;
+                hi = lo + step < hi ? lo + step : hi;
+            }
+            job = lo;
+        }
+        const EncJob& J = a.jobs ? a.jobs[job] : a.single;
+        const EncTable& T = a.jobs ? a.tables[job] : s_tab;
+        const uint64_t st = item - J.item0;
+        uint64_t part = 0;
+        bool absent = false;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t b = lane + 32 * j;
+            const uint32_t len = (T.e[b] >> 16) & 31u;
+            const uint32_t n = valid ? a.st_hist[item * 256 + b] : 0u;
+            absent |= n != 0 && len == 0;
+            part += (uint64_t)n * len;
+        }
+        if (absent) atomicOr(a.status, kDevNoCode);
+        const uint64_t agg = warp_sum_u64(part);
+        if (lane == 0) {
+            s_agg[warp] = agg;
+            s_first[warp] = valid && st == 0;
+        }
+        __syncthreads();
+        const uint32_t starts = __ballot_sync(kFull, lane < (uint32_t)kPlanWarps && s_first[lane]);  // of jobs, in the group
+        const uint64_t mine = lane < (uint32_t)kPlanWarps ? s_agg[lane] : 0;
+        const bool held = a.hook.hold_plus1 && (a.hook.hold_plus1 - 1) / kPlanWarps == g;
+        if (warp == 0) {
+            const uint32_t from = starts ? 31 - __clz(starts) : 0u;
+            const uint64_t sum = warp_sum_u64(lane >= from ? mine : 0);
+            if (lane == 0 && !held) lookback_publish(a.st_rec, g, sum, starts != 0);
+            const uint64_t e = lookback_resolve<kPlanLookK>(a.st_rec, g, sum, (starts & 1u) != 0, a.status, lane,
+                                                            wait_limit(a.hook), !held && starts == 0);
+            if (lane == 0) s_excl = e;
+        }
+        // the job's bits before this region: in the group, and before it unless the job starts in it
+        const uint32_t upto = starts & ((2u << warp) - 1u);
+        const uint32_t from = upto ? 31 - __clz(upto) : 0u;
+        uint64_t excl = warp_sum_u64(lane >= from && lane < warp ? mine : 0);
+        __syncthreads();
+        if (!upto) excl += s_excl;
+        // (test hook: the regions after a held one in its own group wait for it, too)
+        if (held && item >= a.hook.hold_plus1)
+            lookback_resolve<1>(a.st_rec, g + 1, 0, false, a.status, lane, wait_limit(a.hook), false);
+        const uint64_t vfirst = st * (uint64_t)J.st_bytes;  // first byte of this region
+        const uint64_t G = J.bit0 + excl;
+        uint32_t head = 0, gap_head = 0;
+        const uint32_t r = (uint32_t)(G & 31);
+        const bool odd = ((G >> 7) & 1) != 0;
+        if (valid && G > 0 && (r != 0 || odd)) {
+            // walk the previous region's codes backwards from G
+            const uint64_t wstart = G - r;              // the word's first bit
+            const uint64_t bnd = G & ~127ull;           // the segment end at or before G
+            // codes starting at or below `stop` can no longer reach the head
+            // word (bits >= wstart) nor cross or end at bnd
+            uint64_t stop = r ? wstart : ~0ull;
+            if (odd && bnd - 1 < stop) stop = bnd - 1;
+            uint64_t end = G;
+            for (uint64_t base = 0;; base += 32) {  // 32 bytes a round, one per lane, going backwards
+                const uint64_t v = vfirst - 1 - base - lane;  // may wrap below lo: no byte
+                uint32_t c = 0, len = 0;
+                if (vfirst >= base + lane + 1 && v >= J.lo) code_of(T.e[__ldg(J.in_aligned + v)], c, len);
+                const uint32_t incl = warp_incl_scan(len, lane);
+                const uint64_t ce = end - (incl - len);  // this code's end bit
+                const uint64_t cs = ce - len;            // and start bit
+                if (len) {
+                    if (r && ce > wstart)  // the code's right-aligned value, placed to end at ce
+                        head |= (uint32_t)(((uint64_t)(c >> (32 - len))) << (wstart + 32 - ce));
+                    if (odd && cs < bnd && bnd <= ce) gap_head = (uint32_t)(ce - bnd);
+                }
+                const uint32_t total = __shfl_sync(kFull, incl, 31);
+                end -= total;  // start of the round's last code
+                if (end <= stop || total == 0) break;  // uniform
+            }
+            head = __reduce_or_sync(kFull, head);
+            gap_head = __reduce_or_sync(kFull, gap_head);
+        }
+        if (lane == 0 && valid) {
+            const uint64_t base = G & ~1023ull;
+            auto room = [](uint64_t total, uint64_t from) {
+                return total <= from ? 0u : total - from < 0x40000000ull ? (uint32_t)(total - from) : 0x40000000u;
+            };
+            const bool last = st + 1 == J.nst;
+            EncRegion R;
+            R.in = J.in_aligned + vfirst;
+            R.bits = J.bits + (base >> 5);
+            R.gaps = J.gaps + (base >> 10);
+            R.nwords = room(J.words, base >> 5);
+            R.ngaps = room(J.gap_words, base >> 10);
+            R.lo = st == 0 ? (uint32_t)J.lo : 0u;
+            R.hi = (uint32_t)(region_end(J, st) - vfirst);
+            R.first_bit = (uint32_t)(G - base);
+            R.nbits = (uint32_t)agg;
+            R.tail = r ? head >> (32 - r) : 0u;
+            R.gap_head = gap_head;
+            R.job = job;
+            R.flags = (st == 0 ? kRegionFirst : 0u) | (last ? kRegionLast : 0u) | (J.bits_aligned16 ? kRegionVec : 0u);
+            R.pad[0] = R.pad[1] = 0;
+            a.plan[item] = R;
+            const uint64_t E = G + agg;
+            if (last && ((E + 31) / 32 != J.words || (E + 127) / 128 != J.segments)) atomicOr(a.status, kDevSize);
+        }
+    }
 }
+
+__device__ __forceinline__ uint32_t region_steps(const EncRegion& R) { return (R.hi + kStepBytes - 1) / kStepBytes; }
 
 // The bulk-copy producer: thread 0 at region boundaries, the last warp's first
 // thread after each step's barrier (never both at once; barriers order them).
-// Copies go out in the order the CTA encodes steps: the rest of the current
-// region, then the claimed next one; at most kRing beyond the last step whose
-// buffer is free again.  Its state lives in shared memory (one thread touches
-// it at a time), sparing every thread the registers.
-__device__ __forceinline__ void produce(const EncArgs& a, uint8_t* ring, EncShared& sh, uint32_t freed, int cur_slot) {
+// Copies go out in the order the CTA encodes steps: the rest of region cur,
+// then region next (null: not known yet); at most kRing beyond the last step
+// whose buffer is free again.  Its state lives in shared memory (one thread
+// touches it at a time), sparing every thread the registers.
+__device__ __forceinline__ void produce(uint8_t* ring, EncShared& sh, uint32_t freed, const EncRegion* cur,
+                                        const EncRegion* next) {
     uint32_t issued = sh.p_issued, ps = sh.p_step;
     int which = sh.p_which;
     while (issued < freed + kRing) {
-        const int slot = cur_slot ^ which;
-        const uint64_t item = sh.item[slot];
-        if (item >= sh.nitems) break;
-        const EncJob& J = sh.job[slot];
-        const uint64_t st = item - J.item0;
-        if (ps >= region_steps(J, st)) {
+        const EncRegion* const R = which ? next : cur;
+        if (!R || R->hi == 0) break;
+        if (ps >= region_steps(*R)) {
             if (which == 0) {
                 which = 1;
                 ps = 0;
                 continue;
             }
-            break;  // wait for the next claim
+            break;  // wait for the next region
         }
-        const uint64_t v = st * (uint64_t)J.st_bytes + (uint64_t)ps * kStepBytes;
-        const uint64_t rem = ((region_end(J, st) + 15) & ~15ull) - v;  // through the last 16-byte group
-        const uint32_t bytes = rem >= (uint64_t)kStepBytes ? (uint32_t)kStepBytes : (uint32_t)rem;
+        const uint32_t v = ps * (uint32_t)kStepBytes;
+        const uint32_t rem = ((R->hi + 15) & ~15u) - v;  // through the last 16-byte group
+        const uint32_t bytes = rem >= (uint32_t)kStepBytes ? (uint32_t)kStepBytes : rem;
         const uint32_t s = issued % kRing;
-        bulk_load(ring + (size_t)s * kStepBytes, J.in_aligned + v, bytes, &sh.mbar[s]);
+        bulk_load(ring + s * (uint32_t)kStepBytes, R->in + v, bytes, &sh.mbar[s]);
         ++issued;
         ++ps;
     }
@@ -315,132 +405,72 @@ __global__ void __launch_bounds__(kEncThreads, 2)
     uint32_t* const img = img_all + warp * kImgWords;                  // this warp's output words
     auto load_lut = [&](const EncTable& t) {
         for (int i = tid; i < 256 * kLutRep / 2; i += kEncThreads) {  // two copies a store
-            const uint32_t e = t.e[i / (kLutRep / 2)];
-            const uint32_t l = (e >> 16) & 31u;
-            const uint32_t c = l ? (e & 0xffffu) << (32 - l) : 0u;
+            uint32_t c, l;
+            code_of(t.e[i / (kLutRep / 2)], c, l);
             reinterpret_cast<uint4*>(lut)[i] = make_uint4(c, l, c, l);
         }
     };
+    // warp 0: region `item` of the plan to reg[slot], and a job's codes to next_codes, asynchronously
+    const uint64_t nitems = *a.nitems_dev;
+    auto fetch_region = [&](uint32_t slot, uint64_t item) {
+        EncRegion* const to = &sh.reg[slot];
+        if (item < nitems) {
+            if (lane < sizeof(EncRegion) / 16)
+                cp_async16(reinterpret_cast<uint4*>(to) + lane, reinterpret_cast<const uint4*>(a.plan + item) + lane);
+        } else if (lane == 0) {
+            to->hi = 0;
+        }
+        cp_async_commit();
+    };
+    auto fetch_codes = [&](uint32_t job) {
+        const uint4* const from = reinterpret_cast<const uint4*>(a.tables + job);
+        uint4* const to = reinterpret_cast<uint4*>(&sh.next_codes);
+        for (uint32_t i = lane; i < sizeof(EncTable) / 16; i += 32) cp_async16(to + i, from + i);
+        cp_async_commit();
+    };
     if (!a.jobs) load_lut(tab);
     if (tid == 0) {
-        // single path: the histograms in the workspace must come from this very input
-        sh.abort = a.tag && (a.tag[0] != a.single.hi - a.single.lo ||
-                             a.tag[1] != reinterpret_cast<uint64_t>(a.single.in_aligned) + a.single.lo);
-        if (sh.abort) atomicOr(a.status, kDevPlan);
         sh.lut_job = a.jobs ? ~0u : 0u;
-        sh.nitems = a.nitems_dev ? *a.nitems_dev : a.nitems;
         sh.p_issued = 0;
         sh.p_step = 0;
         sh.p_which = 0;
         for (int s = 0; s < kRing; ++s) mbar_init(&sh.mbar[s], 1);
         mbar_init_fence();
     }
-    __syncthreads();
-    if (sh.abort) return;
-
-    int cur_slot = 0;   // slot of the current region; the next one is in cur_slot ^ 1
-    uint32_t cons = 0;  // steps consumed so far (the ring's sequence number)
     if (warp == 0) {
-        claim_region(a, lut, sh, 0, lane);
-        if (sh.item[0] < sh.nitems) claim_region(a, lut, sh, 1, lane);
-        else if (lane == 0) sh.item[1] = ~0ull;
-        if (lane == 0) produce(a, ring, sh, 0, 0);
+        // the CTA's first region is the one of its number, the later ones are claimed
+        uint32_t item = 0;
+        if (lane == 0) item = atomicAdd(a.counter, 1u);
+        fetch_region(0, blockIdx.x);
+        item = __shfl_sync(kFull, item, 0);
+        fetch_region(1, (uint64_t)gridDim.x + item);
+        cp_async_wait_all();
+        __syncwarp();
+        if (a.jobs && sh.reg[0].hi) fetch_codes(sh.reg[0].job);
+        if (lane == 0) produce(ring, sh, 0, &sh.reg[0], &sh.reg[1]);
+        cp_async_wait_all();
     }
     __syncthreads();
 
-    for (;;) {
-        const uint64_t item = sh.item[cur_slot];
-        if (item >= sh.nitems) break;
-        const EncJob& J = sh.job[cur_slot];
-        const uint32_t jid = sh.job_id[cur_slot];
-        const uint64_t st = item - J.item0;  // region within the job
-
-        // ---- warp 0: G of the current region, what precedes G in its word and gap byte ----
-        if (warp == 0) {
-            const uint64_t G =
-                J.bit0 + lookback_resolve<4>(a.st_rec, item, sh.agg[cur_slot], st == 0, a.status, lane,
-                                             wait_limit(a.hook), item + 1 != a.hook.hold_plus1);
-            uint32_t head = 0, gap_head = 0;
-            const uint32_t r = (uint32_t)(G & 31);
-            const bool odd = ((G >> 7) & 1) != 0;
-            if (G > 0 && (r != 0 || odd)) {
-                // walk the previous region's codes backwards from G
-                const uint64_t wstart = G - r;              // the word's first bit
-                const uint64_t bnd = G & ~127ull;           // the segment end at or before G
-                // codes starting at or below `stop` can no longer reach the head
-                // word (bits >= wstart) nor cross or end at bnd
-                uint64_t stop = r ? wstart : ~0ull;
-                if (odd && bnd - 1 < stop) stop = bnd - 1;
-                uint64_t end = G;
-                const uint64_t vfirst = st * (uint64_t)J.st_bytes;  // first byte of this region
-                // 32 bytes a round, one per lane, going backwards; the bytes of kWalkAhead
-                // rounds are loaded at once (one memory round trip, not one per round)
-                constexpr int kWalkAhead = 2;
-                for (uint64_t base0 = 0;; base0 += 32 * kWalkAhead) {
-                    uint32_t pre[kWalkAhead];
-#pragma unroll
-                    for (int k = 0; k < kWalkAhead; ++k) {
-                        const uint64_t base = base0 + 32 * k;
-                        const uint64_t v = vfirst - 1 - base - lane;  // may wrap below lo: no byte
-                        pre[k] = (vfirst >= base + lane + 1 && v >= J.lo) ? (uint32_t)__ldg(J.in_aligned + v) : 0x100u;
-                    }
-                    bool done = false;  // warp-uniform
-#pragma unroll
-                    for (int k = 0; k < kWalkAhead; ++k) {
-                        if (done) break;
-                        uint32_t c = 0, len = 0;
-                        if (pre[k] < 0x100u) {
-                            if (a.jobs) {
-                                code_of(a.tables + jid, pre[k], c, len);
-                            } else {
-                                const uint2 e = lut[pre[k] * kLutRep + (lane & (kLutRep - 1))];
-                                c = e.x;
-                                len = e.y;
-                            }
-                        }
-                        const uint32_t incl = warp_incl_scan(len, lane);
-                        const uint64_t ce = end - (incl - len);  // this code's end bit
-                        const uint64_t cs = ce - len;            // and start bit
-                        if (len) {
-                            if (r && ce > wstart)  // the code's right-aligned value, placed to end at ce
-                                head |= (uint32_t)(((uint64_t)(c >> (32 - len))) << (wstart + 32 - ce));
-                            if (odd && cs < bnd && bnd <= ce) gap_head = (uint32_t)(ce - bnd);
-                        }
-                        const uint32_t total = __shfl_sync(kFull, incl, 31);
-                        end -= total;  // start of the round's last code
-                        if (end <= stop || total == 0) done = true;
-                    }
-                    if (done) break;
-                }
-                head = __reduce_or_sync(kFull, head);
-                gap_head = __reduce_or_sync(kFull, gap_head);
-            }
-            if (lane == 0) {
-                const uint64_t base = G & ~1023ull, vfirst = st * (uint64_t)J.st_bytes;
-                auto room = [](uint64_t total, uint64_t from) {
-                    return total <= from ? 0u : total - from < 0x40000000ull ? (uint32_t)(total - from) : 0x40000000u;
-                };
-                sh.G = G;
-                sh.tail[(cons * kEncWarps) % (4 * kEncWarps)] = r ? head >> (32 - r) : 0u;
-                sh.gap_head = gap_head;
-                Region& R = sh.reg;
-                R.bits = J.bits + (base >> 5);
-                R.gaps = J.gaps + (base >> 10);
-                R.nwords = room(J.words, base >> 5);
-                R.ngaps = room(J.gap_words, base >> 10);
-                R.first_bit = (uint32_t)(G - base);
-                R.lo = st == 0 ? (uint32_t)J.lo : 0u;
-                R.hi = (uint32_t)(region_end(J, st) - vfirst);
-                R.first = st == 0;
-                R.last = st + 1 == J.nst;
-                R.vec = J.bits_aligned16 != 0;
-            }
-        }
+    uint32_t cons = 0;  // steps consumed so far (the ring's sequence number)
+    for (uint32_t slot = 0;; slot = slot == 2 ? 0 : slot + 1) {
+        const EncRegion& R = sh.reg[slot];
+        if (R.hi == 0) break;
+        const EncRegion* const next = &sh.reg[slot == 2 ? 0 : slot + 1];
         // batched: the job's codes into the table (the previous region is done with it)
-        if (a.jobs && jid != sh.lut_job) load_lut(a.tables[jid]);
+        if (a.jobs && R.job != sh.lut_job) load_lut(sh.next_codes);
+        if (warp == 0) {
+            if (lane == 0) sh.tail[(cons * kEncWarps) % (4 * kEncWarps)] = R.tail;
+            cp_async_wait_all();  // the next region
+        }
         __syncthreads();
-        if (tid == 0) sh.lut_job = jid;
-        const Region& R = sh.reg;
+        // warp 0: the next region's codes, if they are others, and the claim of the region after it
+        uint32_t claim = 0;
+        if (warp == 0 && next->hi) {
+            if (a.jobs && next->job != R.job) fetch_codes(next->job);
+            if (lane == 0) claim = atomicAdd(a.counter, 1u);
+        }
+        if (tid == 0) sh.lut_job = R.job;
         uint32_t P = R.first_bit;      // first bit of the step
         uint32_t gnext = 0;            // next gap word to write
         bool overflow = false;
@@ -463,8 +493,8 @@ __global__ void __launch_bounds__(kEncThreads, 2)
                 v |= ((rr[i] >> s) & 0xfu) << (4 * i);
             }
             v &= (hi == 8 ? ~0u : (1u << (4 * hi)) - 1u) & (~0u << (4 * lo));
-            if (lo & 1u) v |= sh.gap_head << (4 * (lo - 1));
-            const uint32_t b0 = R.first ? 0u : lo >> 1;
+            if (lo & 1u) v |= R.gap_head << (4 * (lo - 1));
+            const uint32_t b0 = R.flags & kRegionFirst ? 0u : lo >> 1;
             if (g >= R.ngaps) {
                 overflow = true;
             } else if (b0 == 0 && bytes == 4) {
@@ -485,7 +515,7 @@ __global__ void __launch_bounds__(kEncThreads, 2)
             const bool have = off < R.hi;  // the warp's 1 KiB is in the region (whole, unless the job ends in it)
             // an end of the job in it: bytes before and after the job's are encoded too (the ring holds
             // something there), but count for nothing and are not written out
-            const bool edge = off < R.lo || (R.last && off + kWarpBytes >= R.hi);
+            const bool edge = off < R.lo || ((R.flags & kRegionLast) && off + kWarpBytes >= R.hi);
             Pieces pc;
             uint32_t nbits = 0;
             if (have) {
@@ -513,7 +543,7 @@ __global__ void __launch_bounds__(kEncThreads, 2)
             // the last warp refills the ring
             if (tid == kEncThreads - 32) {
                 fence_proxy_async_smem();
-                produce(a, ring, sh, cons + 1, cur_slot);
+                produce(ring, sh, cons + 1, &R, next);
             }
             const uint32_t t = lane < (uint32_t)kEncWarps ? sh.tot[par][lane] : 0u;
             const uint32_t L = __reduce_add_sync(kFull, t);
@@ -546,7 +576,7 @@ __global__ void __launch_bounds__(kEncThreads, 2)
                     const uint32_t pa = __shfl_sync(kFull, p, 16 * half);              // first and end bit
                     const uint32_t pz = __shfl_sync(kFull, p1, split && !half ? 15 : 31);
                     const bool act = split ? (lane >> 4) == half : true;
-                    const bool ends = R.last && off + kWarpBytes >= R.hi && (half || !split);  // the job's end
+                    const bool ends = (R.flags & kRegionLast) && off + kWarpBytes >= R.hi && (half || !split);  // the job's end
                     if (edge) {
                         const uint32_t o = off + lane * (uint32_t)kLaneBytes;
                         if (o < R.lo) p -= bits_before(pc, R.lo - o);
@@ -574,7 +604,7 @@ __global__ void __launch_bounds__(kEncThreads, 2)
                         overflow = true;
                         j1 = R.nwords > gw ? R.nwords - gw : 0u;
                     }
-                    if (R.vec) {
+                    if (R.flags & kRegionVec) {
                         // whole 16-byte groups, then the words before and after them
                         const uint32_t g0 = (j0 + 3) & ~3u, g1 = j1 & ~3u;
 #pragma unroll 1
@@ -599,6 +629,13 @@ __global__ void __launch_bounds__(kEncThreads, 2)
             }
             P += L;
         }
+        if (warp == 0) {
+            cp_async_wait_all();  // the next region's codes
+            // the region after the next into the slot that the last barrier freed
+            claim = __shfl_sync(kFull, claim, 0);
+            if (next->hi) fetch_region(slot == 0 ? 2 : slot - 1, (uint64_t)gridDim.x + claim);
+            else if (lane == 0) sh.reg[slot == 0 ? 2 : slot - 1].hi = 0;
+        }
         __syncthreads();  // every record of the region visible
 
         // ---- end of the region --------------------------------------------------
@@ -607,30 +644,19 @@ __global__ void __launch_bounds__(kEncThreads, 2)
 #pragma unroll 1
             for (uint32_t g = gnext + (kEncThreads - 1 - tid); g <= (k_end >> 3); g += kEncThreads) {
                 uint32_t bytes = 4;
-                if (g == (k_end >> 3)) bytes = !R.last ? (k_end & 7) >> 1 : g < R.ngaps ? 4u : 0u;  // the region ends in it
+                if (g == (k_end >> 3)) bytes = !(R.flags & kRegionLast) ? (k_end & 7) >> 1 : g < R.ngaps ? 4u : 0u;  // the region ends in it
                 if (bytes) emit_gap(g, k_end, bytes);
             }
         }
         if (overflow) atomicOr(a.status, kDevSize);
         if (tid == 0) {
-            const uint64_t E = (sh.G & ~1023ull) + P;
-            if (E - sh.G != sh.agg[cur_slot]) atomicOr(a.status, kDevPlan);  // histograms were not this input's
-            if (R.last && ((E + 31) / 32 != J.words || (E + 127) / 128 != J.segments)) atomicOr(a.status, kDevSize);
+            if (P - R.first_bit != R.nbits) atomicOr(a.status, kDevPlan);  // histograms were not this input's
+            // the producer's cursor follows its region, which becomes the current one
+            if (sh.p_which == 1) sh.p_which = 0;
+            else sh.p_step = 0;
+            fence_proxy_async_smem();
+            produce(ring, sh, cons, next, nullptr);
         }
-        __syncthreads();  // the slot, gap_head and G are read
-        if (warp == 0) {
-            // the next region becomes current; claim the one after it into the freed slot
-            const int old = cur_slot;
-            if (sh.item[old ^ 1] < sh.nitems) claim_region(a, lut, sh, old, lane);
-            else if (lane == 0) sh.item[old] = ~0ull;
-            if (lane == 0) {
-                // the producer's cursor follows its region into the current slot
-                if (sh.p_which == 1) sh.p_which = 0;
-                else sh.p_step = 0;
-                produce(a, ring, sh, cons, old ^ 1);
-            }
-        }
-        cur_slot ^= 1;
     }
 
     // every copy issued has been consumed, unless a wait gave up: never leave
@@ -646,14 +672,22 @@ __global__ void __launch_bounds__(kEncThreads, 2)
 // ------------------------------------------------------------- launchers ---
 
 int launch_encode(const EncArgs& a, const EncTable& t, int ctas_per_sm, void* stream) {
-    static LaunchCache cache;
+    static LaunchCache cache, plan_cache;
     const LaunchFacts f = cache.get(reinterpret_cast<const void*>(encode_kernel), kEncThreads, kEncSmem);
     if (f.err != cudaSuccess) return f.err;
-    const int sms = f.sms, per_sm = f.per_sm;
-    const int k = (ctas_per_sm > 0 && ctas_per_sm < per_sm) ? ctas_per_sm : per_sm;
-    const uint64_t cap = (uint64_t)sms * k;
-    const unsigned grid = (unsigned)(a.nitems_dev ? cap : (a.nitems < cap ? (a.nitems ? a.nitems : 1) : cap));
-    encode_kernel<<<grid, kEncThreads, kEncSmem, static_cast<cudaStream_t>(stream)>>>(a, t);
+    const LaunchFacts pf = plan_cache.get(reinterpret_cast<const void*>(enc_plan_kernel), kPlanThreads, 0);
+    if (pf.err != cudaSuccess) return pf.err;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // as many plan warps as there are regions, at most what the GPU holds at once
+    const uint64_t regions = a.nitems ? a.nitems : 1;
+    const uint64_t plan_want = (regions + kPlanWarps - 1) / kPlanWarps;
+    const uint64_t plan_cap = (uint64_t)pf.sms * pf.per_sm;
+    enc_plan_kernel<<<(unsigned)(plan_want < plan_cap ? plan_want : plan_cap), kPlanThreads, 0, st>>>(a, t);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const int k = (ctas_per_sm > 0 && ctas_per_sm < f.per_sm) ? ctas_per_sm : f.per_sm;
+    const uint64_t cap = (uint64_t)f.sms * k;
+    encode_kernel<<<(unsigned)(regions < cap ? regions : cap), kEncThreads, kEncSmem, st>>>(a, t);
     return cudaGetLastError();
 }
 

@@ -78,12 +78,13 @@ constexpr int kEncMaxStChunks = 32;
 constexpr uint64_t kEncCtas = 296;
 constexpr uint64_t kEncStOverhead = 1;  // chunks
 
-// Encoder workspace: [status u32][counter u32][pad][tag: n u64, input u64] ...
-// [scratch histogram u32 x 256 at 1024] [st_rec u64 x nst at 2048] [st_hist u32 x 256 x nst]
-constexpr size_t kEncWsHeader = 2048;
-constexpr size_t kEncWsTag = 16;
-constexpr size_t kEncWsScratchHist = 1024;
-
+// Encoder workspace for nst super-tiles:
+//   [status u32][counter u32][super-tiles to encode u64][st_rec u64 x nst]  cleared by every call
+//   [tag: n u64, input u64][scratch histogram u32 x 256]                    and these by the histogram pass
+//   [plan EncRegion x nst][st_hist u32 x 256 x nst]
+struct EncWorkspace {
+    size_t st_rec, tag, scratch, plan, st_hist, bytes;
+};
 inline uint64_t encode_chunks(uint64_t n) { return (n + 15 + kEncChunkBytes - 1) / kEncChunkBytes; }
 // An upper bound of the super-tile count of every input of up to n bytes (at any
 // alignment), non-decreasing in n: what a workspace for inputs of up to n bytes holds.
@@ -137,14 +138,50 @@ struct alignas(16) EncJob {
 };
 static_assert(sizeof(EncJob) == 96, "EncJob: six 16-byte groups");
 
+// One region as the encoder takes it, made by enc_plan_kernel once the code
+// lengths are known: all that a CTA needs to start on it without another
+// dependent load.  Output words and bit positions count from the gap word (1024
+// bits, so also the 16-byte group of output words) that holds the region's first
+// bit.
+struct alignas(16) EncRegion {
+    const uint8_t* in;          // its bytes are [lo, hi) from here (16-byte aligned)
+    uint32_t* bits;             // output and gap words,
+    uint32_t* gaps;
+    uint32_t nwords, ngaps;     // and how many of them exist
+    uint32_t lo, hi;            // hi = 0: no region
+    uint32_t first_bit;         // the region's first bit
+    uint32_t nbits;             // and bit count
+    uint32_t tail;              // the code bits before it in its first word, right-aligned
+    uint32_t gap_head;          // spill at the segment end at or before it, if its first gap entry is an odd one
+    uint32_t job;
+    uint32_t flags;             // kRegion...
+    uint32_t pad[2];
+};
+static_assert(sizeof(EncRegion) == 80, "EncRegion: five 16-byte groups");
+constexpr uint32_t kRegionFirst = 1u;  // of its job
+constexpr uint32_t kRegionLast = 2u;
+constexpr uint32_t kRegionVec = 4u;    // output words are 16-byte aligned
+
+inline EncWorkspace encode_workspace(uint64_t nst) {
+    EncWorkspace w;
+    w.st_rec = 16;
+    w.tag = (w.st_rec + 8 * (size_t)nst + 15) & ~(size_t)15;
+    w.scratch = w.tag + 16;
+    w.plan = w.scratch + 1024;
+    w.st_hist = w.plan + sizeof(EncRegion) * (size_t)nst;
+    w.bytes = w.st_hist + 1024 * (size_t)nst;
+    return w;
+}
+
 struct EncArgs {
     EncJob single;              // the job, when jobs == nullptr
     const EncJob* jobs;         // batched: [count]
     const uint64_t* item0s;     // batched: [count + 1], item0 of each job and the total
     const EncTable* tables;     // batched: [count]
     uint32_t count;             // jobs (1 for the single-buffer path)
-    uint64_t nitems;            // regions over all jobs
-    const uint64_t* nitems_dev; // batched: the region count in device memory (overrides nitems)
+    uint64_t nitems;            // regions over all jobs (batched: an upper bound)
+    uint64_t* nitems_dev;       // the region count in device memory; single path: written by the plan (0: not this input's)
+    EncRegion* plan;            // [nitems]
     uint64_t* st_rec;           // [nitems] look-back records over regions
     const uint32_t* st_hist;    // [nitems][256] per-region histograms
     const uint64_t* tag;        // single path: {n, input address} written by the histogram pass
@@ -283,6 +320,7 @@ struct DecArgs {
 // --------------------------------------------------------------- launchers --
 // Implemented in the .cu files; return cudaError_t as int.
 int launch_histogram(const void* d_in, uint64_t n, uint32_t* d_hist, void* stream);
+// The plan, then the encoder.
 int launch_encode(const EncArgs& a, const EncTable& t, int ctas_per_sm, void* stream);
 int launch_hist_st(const HistStArgs& a, int ctas_per_sm, void* stream);
 int launch_decode(const DecArgs& a, const DecTable& t, uint32_t min_len, bool complete, bool pairs,
