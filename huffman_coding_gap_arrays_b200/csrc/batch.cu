@@ -2,12 +2,12 @@
 // device-side codebook entry points.  No counterpart in the reference.
 //
 // Compress, all on the stream, nothing back to the host:
-//   1. benc_setup   one CTA: each buffer's alignment, region size and region
-//                   count; an exclusive scan numbers the regions globally;
+//   1. benc_setup   each buffer's alignment, region size and region count; an
+//                   exclusive scan numbers the regions globally;
 //   2. hist_st      per-region histograms and per-buffer histograms;
 //   3. book         one warp per buffer: length-limited canonical codebook,
 //                   encoder table, sizes (book.cuh);
-//   4. benc_place   one CTA: scans of the stream sizes place every bitstream
+//   4. benc_place   scans of the stream sizes place every bitstream
 //                   (16-byte aligned) and gap array in the two arenas;
 //   5. enc_plan     one warp per region: bit count, first output bit, all that
 //                   a CTA needs to start on it;
@@ -20,7 +20,7 @@
 //                   (decoder stage size by the shortest code x complete book
 //                   or not), and writes its decode job (stream, output, tile
 //                   count);
-//   2. bdec_setup   one CTA: look-back record numbering over all tiles, and
+//   2. bdec_setup   look-back record numbering over all tiles, and
 //                   per class the numbering of the class's tiles;
 //   3. bdec_map     tile -> buffer map of each class;
 //   4. decode       one persistent launch per class (all 8, or those the
@@ -120,61 +120,112 @@ __device__ __forceinline__ void block_excl_scan2_u64(uint64_t& a, uint64_t& b, u
 
 // --------------------------------------------------------------- compress ---
 
+// The scans over the buffers run on several CTAs: each takes a run of buffers and
+// sums what precedes its run itself -- independent loads, where one CTA went
+// through the buffers 1024 at a time behind four barriers each (4096 buffers:
+// benc_setup 21 -> 9 us, benc_place 26 -> 9, bdec_setup 14 -> 8).  256
+// buffers a CTA, so that its 1024 threads share the regions of few buffers; at
+// most kScanCtas, so that the repeated reads stay a small multiple of the
+// buffers, and then up to 1024 buffers a step.
+constexpr uint32_t kScanCtas = 64, kScanMin = 256;
+__device__ __forceinline__ uint64_t scan_run(uint32_t count) {  // buffers per CTA
+    const uint64_t per = ((uint64_t)count + gridDim.x - 1) / gridDim.x;
+    const uint64_t unit = per > kScanThreads / 2 ? kScanThreads : kScanMin;
+    return (per + unit - 1) / unit * unit;
+}
+
+// Sum of one u64 per thread over the CTA.
+__device__ __forceinline__ uint64_t block_sum_u64(uint64_t v, uint64_t* s_warp) {
+    const uint64_t w = warp_sum_u64(v);
+    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = w;
+    __syncthreads();
+    const uint64_t t = warp_sum_u64(s_warp[threadIdx.x & 31]);  // 32 warps
+    __syncthreads();  // s_warp free for the next call
+    return t;
+}
+
+// Numbers the regions, starts the encoder jobs and writes every region for the
+// histogram pass (so that no CTA searches for a region's buffer there).
 __global__ void __launch_bounds__(kScanThreads) benc_setup_kernel(uint32_t count, const uint8_t* const* inputs,
                                                                   const uint64_t* sizes,
                                                                   const uint8_t* region_chunks,
                                                                   uint32_t base_chunks, EncJob* jobs,
-                                                                  uint64_t* item0s, uint64_t* nitems,
-                                                                  uint64_t max_regions, uint32_t* status) {
+                                                                  uint64_t* item0s, HistRegion* regions,
+                                                                  uint64_t* nitems, uint64_t max_regions,
+                                                                  uint32_t* status) {
     __shared__ uint64_t s_warp[32];
-    uint64_t carry = 0;
-    // each buffer's size, input pointer and region size, the next 1024 buffers' in flight
-    uint64_t n_next = 0;
-    const uint8_t* in_next = nullptr;
-    uint32_t rc_next = base_chunks;
-    auto load = [&](uint64_t j) {
-        n_next = 0;
-        in_next = nullptr;
-        rc_next = base_chunks;
-        if (j < count) {
-            n_next = sizes[j];
-            in_next = inputs[j];
-            if (region_chunks) rc_next = region_chunks[j];
-        }
+    __shared__ const uint8_t* s_in[kScanThreads];   // of 1024 buffers: aligned input, last byte, first region
+    __shared__ uint64_t s_hi[kScanThreads];
+    __shared__ uint32_t s_item0[kScanThreads + 1], s_st[kScanThreads];  // and region size, lo in its upper half
+    struct Buf {
+        const uint8_t* in;
+        uint64_t n, nst;
+        uint32_t lo, st;
     };
-    load(threadIdx.x);
-    for (uint64_t base = 0; base < count; base += kScanThreads) {
-        const uint64_t j = base + threadIdx.x;
-        const uint64_t n = n_next;
-        const uint8_t* const in = in_next;
-        uint32_t rc = rc_next;
-        load(j + kScanThreads);
-        uint64_t nst = 0, lo = 0;
-        uint32_t st = 0;
+    auto load = [&](uint64_t j) {
+        Buf b = {nullptr, 0, 0, 0, 0};
         if (j < count) {
-            lo = reinterpret_cast<uintptr_t>(in) & 15;
+            b.n = sizes[j];
+            b.in = inputs[j];
+            uint32_t rc = region_chunks ? region_chunks[j] : base_chunks;
             if (rc < base_chunks) rc = base_chunks;
             if (rc > 32) rc = 32;
-            st = rc * (uint32_t)kEncChunkBytes;
-            nst = n ? (lo + n + st - 1) / st : 0;
+            b.lo = (uint32_t)(reinterpret_cast<uintptr_t>(b.in) & 15);
+            b.st = rc * (uint32_t)kEncChunkBytes;
+            b.nst = b.n ? (b.lo + b.n + b.st - 1) / b.st : 0;
         }
+        return b;
+    };
+    const uint64_t run = scan_run(count), first = blockIdx.x * run;
+    const uint64_t end = first + run < count ? first + run : count;
+    uint64_t sum = 0;
+    for (uint64_t j = threadIdx.x; j < first && j < count; j += kScanThreads) sum += load(j).nst;
+    uint64_t carry = block_sum_u64(sum, s_warp);
+    for (uint64_t base = first; base < end; base += kScanThreads) {
+        const uint64_t j = base + threadIdx.x;
+        const Buf b = load(j < end ? j : count);
         uint64_t total = 0;
-        const uint64_t excl = block_excl_scan_u64(nst, &total, s_warp);
-        if (j < count) {
+        const uint64_t excl = block_excl_scan_u64(b.nst, &total, s_warp);
+        if (j < end) {
             EncJob J;
             memset(&J, 0, sizeof(J));
-            J.in_aligned = in - lo;
-            J.lo = lo;
-            J.hi = lo + n;
+            J.in_aligned = b.in - b.lo;
+            J.lo = b.lo;
+            J.hi = b.lo + b.n;
             J.item0 = carry + excl;
-            J.nst = nst;
-            J.st_bytes = st;
+            J.nst = b.nst;
+            J.st_bytes = b.st;
             jobs[j] = J;
             item0s[j] = carry + excl;
         }
+        // the regions of these buffers, spread over the threads (their number per buffer varies widely)
+        s_in[threadIdx.x] = b.in - b.lo;
+        s_hi[threadIdx.x] = b.lo + b.n;
+        s_st[threadIdx.x] = b.st | b.lo;  // (a multiple of 8 KiB, and less than 16)
+        s_item0[threadIdx.x] = (uint32_t)excl;
+        __syncthreads();
+        const uint64_t fit = carry < max_regions ? max_regions - carry : 0, todo = total < fit ? total : fit;
+        for (uint64_t r = threadIdx.x; r < todo; r += kScanThreads) {
+            uint32_t lo = 0, hi = kScanThreads;  // the last buffer with item0 <= r
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (s_item0[mid] <= r) lo = mid;
+                else hi = mid;
+            }
+            const uint32_t st = s_st[lo] & ~15u;
+            const uint64_t k = r - s_item0[lo], v = k * st, left = s_hi[lo] - v;
+            HistRegion R;
+            R.in = s_in[lo] + v;
+            R.lo = k == 0 ? s_st[lo] & 15u : 0u;
+            R.hi = left < st ? (uint32_t)left : st;
+            R.job = (uint32_t)(base + lo);
+            R.pad[0] = R.pad[1] = R.pad[2] = 0;
+            regions[carry + r] = R;
+        }
         carry += total;
+        __syncthreads();
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && first < count && first + run >= count) {  // the last CTA's run
         item0s[count] = carry;
         // a workspace smaller than the query asked for: nothing is encoded
         if (carry > max_regions) atomicOr(status, kDevSize);
@@ -263,29 +314,28 @@ __global__ void __launch_bounds__(kScanThreads) benc_place_kernel(uint32_t count
                                                                   uint64_t bits_cap, uint32_t* gaps,
                                                                   uint64_t gaps_cap, uint32_t* status) {
     __shared__ uint64_t s_warp[2][32];
+    const uint64_t run = scan_run(count), first = blockIdx.x * run;
     uint64_t cb = 0, cg = 0;
-    // each stream's words, gap words and segments, the next 1024 streams' in flight
-    uint64_t w_next = 0, g_next = 0, s_next = 0;
-    auto load = [&](uint64_t j) {
-        w_next = 0;
-        g_next = 0;
-        s_next = 0;
-        if (j < count) {
-            w_next = entries[j].words;
-            g_next = entries[j].gap_words;
-            s_next = entries[j].segments;
-        }
-    };
-    load(threadIdx.x);
-    for (uint64_t base = 0; base < count; base += kScanThreads) {
+    for (uint64_t j = threadIdx.x; j < first && j < count; j += kScanThreads) {
+        cb += (entries[j].words + 3) & ~3ull;
+        cg += entries[j].gap_words;
+    }
+    cb = block_sum_u64(cb, s_warp[0]);
+    cg = block_sum_u64(cg, s_warp[1]);
+    const uint64_t end = first + run < count ? first + run : count;
+    for (uint64_t base = first; base < end; base += kScanThreads) {
         const uint64_t j = base + threadIdx.x;
-        const uint64_t words = w_next, gap_words = g_next, segments = s_next;
-        load(j + kScanThreads);
+        uint64_t words = 0, gap_words = 0, segments = 0;
+        if (j < end) {
+            words = entries[j].words;
+            gap_words = entries[j].gap_words;
+            segments = entries[j].segments;
+        }
         uint64_t ob = (words + 3) & ~3ull, og = gap_words, tb = 0, tg = 0;
         block_excl_scan2_u64(ob, og, &tb, &tg, s_warp);
         ob += cb;
         og += cg;
-        if (j < count) {
+        if (j < end) {
             hgap_batch_entry& e = entries[j];
             EncJob& J = jobs[j];
             e.bits_offset = ob;
@@ -512,14 +562,13 @@ __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t c
     }
 }
 
-// One CTA: the look-back record numbering over all buffers' tiles, and per
-// class the numbering of the class's tiles (the jobs come from bdec_table).
-// Per 1024 buffers: nine warp scans of the tile counts (all tiles, and one per
-// class with the other classes' buffers counting 0) need no barrier; nine
-// warps then scan the 32 warp totals of one sum each, between two barriers,
-// and every buffer writes its record and, for its own class only, its first
-// class tile (the only entry the map and the decoder read).  The next 1024
-// buffers' loads are in flight meanwhile.
+// The look-back record numbering over all buffers' tiles, and per class the
+// numbering of the class's tiles (the jobs come from bdec_table).  Per 1024
+// buffers: nine warp scans of the tile counts (all tiles, and one per class with
+// the other classes' buffers counting 0) need no barrier; nine warps then scan
+// the 32 warp totals of one sum each, between two barriers, and every buffer
+// writes its record and, for its own class only, its first class tile (the
+// only entry the map and the decoder read).
 __global__ void __launch_bounds__(kScanThreads) bdec_setup_kernel(uint32_t count, const uint8_t* cls, DecJob* jobs,
                                                                   uint64_t* item0s, uint64_t* class_nitems,
                                                                   uint64_t tiles_cap, uint32_t class_mask,
@@ -529,24 +578,37 @@ __global__ void __launch_bounds__(kScanThreads) bdec_setup_kernel(uint32_t count
     __shared__ uint64_t s_tot[2][kSums][kWarps];  // by chunk parity: warp totals, then warp offsets
     __shared__ uint64_t s_carry[kSums];           // the sums over the earlier chunks
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x < kSums) s_carry[threadIdx.x] = 0;
-    uint32_t c_next = kNoClass;
-    uint64_t nt_next = 0;
-    if (threadIdx.x < count) {
-        c_next = cls[threadIdx.x];
-        nt_next = jobs[threadIdx.x].ntiles;  // 0 for a buffer in no class
+    const uint64_t run = scan_run(count), first = blockIdx.x * run;
+    if (first >= count) return;  // (uniform)
+    {
+        uint64_t sum[kSums] = {};
+        for (uint64_t j = threadIdx.x; j < first; j += kScanThreads) {
+            const uint32_t c = cls[j];
+            const uint64_t nt = jobs[j].ntiles;  // 0 for a buffer in no class
+#pragma unroll
+            for (uint32_t k = 0; k < kSums; ++k) sum[k] += k == kClasses || c == k ? nt : 0;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kSums; ++k) {
+            const uint64_t w = warp_sum_u64(sum[k]);
+            if (lane == 0) s_tot[0][k][warp] = w;
+        }
+        __syncthreads();
+        if (warp < kSums) {
+            const uint64_t w = warp_sum_u64(s_tot[0][warp][lane]);
+            if (lane == 0) s_carry[warp] = w;
+        }
+        __syncthreads();
     }
     uint32_t par = 0;
-    for (uint64_t base = 0; base < count; base += kScanThreads, par ^= 1u) {
+    const uint64_t end = first + run < count ? first + run : count;
+    for (uint64_t base = first; base < end; base += kScanThreads, par ^= 1u) {
         const uint64_t j = base + threadIdx.x;
-        const uint32_t c = c_next;
-        const uint64_t nt = nt_next;
-        const uint64_t jn = j + kScanThreads;
-        c_next = kNoClass;
-        nt_next = 0;
-        if (jn < count) {
-            c_next = cls[jn];
-            nt_next = jobs[jn].ntiles;
+        uint32_t c = kNoClass;
+        uint64_t nt = 0;
+        if (j < end) {
+            c = cls[j];
+            nt = jobs[j].ntiles;
         }
         uint64_t x_all = nt, x_own = 0;
         for (uint32_t k = 0; k < kSums; ++k) {
@@ -575,11 +637,12 @@ __global__ void __launch_bounds__(kScanThreads) bdec_setup_kernel(uint32_t count
             if (lane == 31) s_carry[warp] = carry + x;
         }
         __syncthreads();
-        if (j < count) {
+        if (j < end) {
             jobs[j].item0 = s_tot[par][kClasses][warp] + x_all - nt;
             if (c < kClasses) item0s[(uint64_t)c * (count + 1) + j] = s_tot[par][c][warp] + x_own - nt;
         }
     }
+    if (first + run < count) return;  // the last CTA's run completes the sums
     // (the last chunk's second barrier orders every s_carry update before these reads)
     const uint64_t all = s_carry[kClasses];
     // a workspace smaller than the query asked for: nothing is decoded
@@ -641,6 +704,11 @@ unsigned book_grid(uint32_t count) {
     const uint64_t want = (count + kBookWarps - 1) / kBookWarps;
     const uint64_t cap = 1u << 24;
     return (unsigned)(want < cap ? (want ? want : 1) : cap);
+}
+
+unsigned scan_grid(uint32_t count) {
+    const uint32_t want = (uint32_t)(((uint64_t)count + kScanMin - 1) / kScanMin);
+    return want < 1 ? 1 : want < kScanCtas ? want : kScanCtas;
 }
 
 // One CTA per buffer: the block scheduler hands a buffer to whichever SM frees
@@ -806,11 +874,14 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
     uint64_t* st_rec = reinterpret_cast<uint64_t*>(ws + L.st_rec);
     uint32_t* st_hist = reinterpret_cast<uint32_t*>(ws + L.st_hist);
     EncRegion* plan = reinterpret_cast<EncRegion*>(ws + L.plan);
+    // (the histogram pass is done with its regions before the plan is made in their place)
+    static_assert(sizeof(HistRegion) <= sizeof(EncRegion), "one array for both");
+    HistRegion* hist_regions = reinterpret_cast<HistRegion*>(plan);
 
     if (cudaMemsetAsync(ws, 0, 1024, st) != cudaSuccess) return HGAP_ERR_CUDA;
     if (cudaMemsetAsync(hists, 0, 1024 * (size_t)count, st) != cudaSuccess) return HGAP_ERR_CUDA;
-    benc_setup_kernel<<<1, kScanThreads, 0, st>>>(count, d_inputs, d_sizes, d_region_chunks, base_chunks(cfg), jobs,
-                                                  item0s, nitems, L.max_regions, status);
+    benc_setup_kernel<<<scan_grid(count), kScanThreads, 0, st>>>(count, d_inputs, d_sizes, d_region_chunks, base_chunks(cfg), jobs,
+                                                  item0s, hist_regions, nitems, L.max_regions, status);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
     if (cudaMemsetAsync(st_rec, 0, 8 * (size_t)L.max_regions, st) != cudaSuccess) return HGAP_ERR_CUDA;
 
@@ -822,6 +893,7 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
     h.nitems_dev = nitems;
     h.hist = hists;
     h.st_hist = st_hist;
+    h.regions = hist_regions;
     h.counter = status + 2;  // in the zeroed header, beside the encoder's region counter
     if (launch_hist_st(h, (int)cfg->hist_ctas_per_sm, stream) != 0) return HGAP_ERR_CUDA;
 
@@ -829,7 +901,7 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
     book_kernel<<<book_grid(count), 32 * kBookWarps, kBookSmem, st>>>(count, hists, nullptr, nullptr, tables,
                                                                       d_entries, d_sizes);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
-    benc_place_kernel<<<1, kScanThreads, 0, st>>>(count, d_entries, jobs, d_bits, bits_capacity, d_gaps,
+    benc_place_kernel<<<scan_grid(count), kScanThreads, 0, st>>>(count, d_entries, jobs, d_bits, bits_capacity, d_gaps,
                                                   gaps_capacity, status);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
 
@@ -877,7 +949,7 @@ hgap_status hgap_batch_decompress(uint32_t count, const hgap_batch_entry* d_entr
     bdec_table_kernel<<<table_grid(count), kTableThreads, 0, st>>>(count, d_entries, d_bits, d_gaps, d_outputs,
                                                                    cfg->dec_tile_segs, wtables, cls, jobs, status);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
-    bdec_setup_kernel<<<1, kScanThreads, 0, st>>>(count, cls, jobs, item0s, class_nitems, L.tiles_cap,
+    bdec_setup_kernel<<<scan_grid(count), kScanThreads, 0, st>>>(count, cls, jobs, item0s, class_nitems, L.tiles_cap,
                                                   cfg->dec_class_mask, status);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
     bdec_map_kernel<<<book_grid(count), 32 * kBookWarps, 0, st>>>(count, jobs, cls, item0s, job_of, L.tiles_cap);

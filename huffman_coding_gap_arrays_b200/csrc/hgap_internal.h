@@ -190,6 +190,15 @@ struct EncArgs {
     LookbackHook hook;
 };
 
+// A batched region as the histogram pass takes it: its bytes are [lo, hi) from `in`.
+struct alignas(16) HistRegion {
+    const uint8_t* in;  // 16-byte aligned
+    uint32_t lo, hi;
+    uint32_t job;
+    uint32_t pad[3];
+};
+static_assert(sizeof(HistRegion) == 32, "HistRegion: two 16-byte groups");
+
 struct HistStArgs {
     EncJob single;
     const EncJob* jobs;
@@ -201,6 +210,7 @@ struct HistStArgs {
     uint32_t* st_hist;          // [nitems][256]
     uint64_t* tag;              // single path: receives {n, input address}
     uint32_t* counter;          // batched: zeroed region counter (regions claimed one at a time)
+    const HistRegion* regions;  // batched: [nitems]
 };
 
 // ---------------------------------------------------------------- decoder ---
