@@ -24,9 +24,10 @@ from .codec import Codebook, Compressed, StreamSizes, _stream
 
 ENTRY_BYTES = C.sizeof(BatchEntry)
 # Kernels one batched call launches (csrc/batch.cu): compress = benc_setup, hist_st, book,
-# benc_place, enc_plan, encode; decompress = bdec_table, bdec_setup, bdec_map and one decoder per class (8).
+# benc_place, enc_plan, encode; decompress = bdec_table, bdec_setup, bdec_map, one decoder per class of
+# complete books (4) and one for the incomplete ones.
 COMPRESS_KERNELS = 6
-DECOMPRESS_KERNELS = 11
+DECOMPRESS_KERNELS = 8
 
 
 @dataclass

@@ -23,9 +23,10 @@
 //   2. bdec_setup   look-back record numbering over all tiles, and
 //                   per class the numbering of the class's tiles;
 //   3. bdec_map     tile -> buffer map of each class;
-//   4. decode       one persistent launch per class (all 8, or those the
-//                   caller names in dec_class_mask), the single-buffer
-//                   decoder kernel over the class's tiles.
+//   4. decode       one persistent launch per class of complete books and one
+//                   for all incomplete ones (or those the caller names in
+//                   dec_class_mask), the single-buffer decoder kernel over the
+//                   class's tiles.
 // Every launch has a fixed grid and reads its work counts from device memory,
 // so the sequence can be captured once and replayed.
 #include <cuda_runtime.h>
@@ -52,6 +53,7 @@ constexpr size_t kBookSmem = kBookWarps * sizeof(Book32) > sizeof(Book64) ? kBoo
 constexpr int kScanThreads = 1024;
 constexpr uint32_t kClasses = 8;
 constexpr uint32_t kNoClass = 0xffu;
+constexpr uint32_t kIncomplete = 6;  // the class number all incomplete books are launched under (32 rows)
 
 // ----------------------------------------------------------- block scans ---
 // Exclusive scan of one u64 per thread over a 1024-thread CTA; returns the
@@ -370,47 +372,81 @@ __device__ __forceinline__ uint32_t class_of(uint32_t min_len, bool complete) {
     return 2 * r + (complete ? 1 : 0);
 }
 
+// The entry (dec_entry.cuh) of a P-bit window x whose first code ends inside it,
+// without a branch: s1 has the code at each 11-bit window, length << 8 | byte
+// (kLongCode: one that ends outside).
+constexpr uint16_t kLongCode = 31 << 8;
+template <uint32_t P, bool MULTI>
+__device__ __forceinline__ uint32_t window_entry(const uint16_t* s1, uint32_t x) {
+    constexpr uint32_t kMask = (1u << kDecPrefix) - 1;
+    x <<= kDecPrefix - P;
+    const uint32_t e1 = s1[x], l1 = e1 >> 8;
+    const uint32_t e2 = s1[x << l1 & kMask], l12 = l1 + (e2 >> 8);
+    const uint32_t two = __byte_perm(e1, e2, 0x7740);  // (the upper bytes of an e are zero)
+    if (!MULTI) return l12 <= P ? two + (l12 << 16) + 0x02000000u : (e1 & 0xffu) + (l1 << 16) + 0x01000000u;
+    const uint32_t e3 = s1[x << (l12 & 31) & kMask], l123 = l12 + (e3 >> 8);
+    return l123 <= P  ? __byte_perm(two, e3, 0x7410) + (l123 << 24) + (2u << 29)
+           : l12 <= P ? two + (l12 << 24) + (1u << 29)
+                      : (e1 & 0xffu) + (l1 << 24);
+}
+
 constexpr int kTableThreads = 256;
 
 // One CTA per buffer: checks the entry, writes the buffer's decoder table
 // (DecTableW), classifies the buffer and writes its decode job (all but its
-// first look-back record, which bdec_setup numbers).  Every thread owns 8
-// consecutive 11-bit prefixes, each taking the symbol whose left-aligned code is
-// the largest not above it; the entries (up to three symbols, dec_entry.cuh)
-// come from those in shared memory, the longer codes' by a binary search per
-// entry, spread over all threads.  A book whose one table would be too large
-// (DecIndex) gets two levels, the same ones as warp_dec_table builds (book.cuh):
-// a block scan places the level-2 groups in prefix order.  At 32 registers a
-// thread (no spills) eight CTAs fit an SM.  Measured for 4096 buffers of 4-64
-// KiB: 66 us (80 us while every buffer built two levels).
+// first look-back record, which bdec_setup numbers).  One symbol a thread: a
+// block scan gives its left-aligned code, and it marks the 11-bit prefix where
+// that code starts; every thread then fills its own 8 prefixes with the last
+// code to start at or below each (a complete book has no holes), and the entries
+// of up to three symbols (dec_entry.cuh) are made from those.  Of codes longer
+// than a prefix every thread writes its symbol's entries.  A book whose one
+// table would be too large (DecIndex) gets two levels, the same ones as
+// warp_dec_table builds (book.cuh): a block scan places the level-2 groups in
+// prefix order.  Bound by instructions and the chain of barriers between the
+// steps; at 32 registers a thread (no spills) eight CTAs fit an SM.  Measured for
+// 4096 buffers of 4-64 KiB: 44 us (58 while one warp read the symbols, every
+// prefix walked the symbol list to its own and every longer code was searched).
 __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t count, const hgap_batch_entry* entries,
                                                                    const uint32_t* bits, const uint32_t* gaps,
                                                                    uint8_t* const* outputs, uint32_t tile_segs,
-                                                                   DecTableW* wtables, uint8_t* cls, DecJob* jobs,
-                                                                   uint32_t* status) {
+                                                                   uint32_t class_mask, DecTableW* wtables, uint8_t* cls,
+                                                                   DecJob* jobs, uint32_t* status) {
     constexpr uint32_t P = kDecPrefix, X = kMaxLen - kDecPrefix;  // 11, 5
     constexpr uint32_t kT1 = 1u << P, kPer = kT1 / kTableThreads;  // 8 prefixes a thread
     __shared__ BookSyms s;
     __shared__ __align__(16) uint16_t s1[kT1];
     __shared__ uint16_t s_end[kT1];  // level-2 offset after each prefix's group (0 for none)
     __shared__ uint32_t s_warp[kTableThreads / 32];
-    __shared__ uint32_t s_kraft, s_long;
+    __shared__ uint32_t s_long;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint32_t j = blockIdx.x; j < count; j += gridDim.x) {
         const hgap_batch_entry& e = entries[j];
         const uint32_t n = e.symbol_count;
         bool bad = n > 256 || e.segments != (e.words + 3) / 4 || e.gap_words != (e.segments + 7) / 8 ||
                    (e.n != 0) != (e.words != 0) || (e.n != 0 && n == 0);
-        if (warp == 0) {
-            const uint32_t kraft = (!bad && n) ? warp_load_symbols(e.symbols, n, s, lane) : 0u;
-            if (lane == 0) {
-                s_kraft = kraft;
-                s_long = kT1;
-            }
-        }
+        // one symbol a thread: the book's checks (as warp_load_symbols), and its left-aligned code
+        if (tid < 8) s.seen[tid] = 0;
+        if (tid == 0) s_long = ~0u;
+        reinterpret_cast<uint4*>(s1)[tid] = make_uint4(~0u, ~0u, ~0u, ~0u);  // no code starts here
         __syncthreads();
-        const uint32_t kraft = s_kraft;
-        if (n && kraft == ~0u) bad = true;
+        const bool mine = !bad && tid < n;
+        uint32_t L = 0, sym = 0, prev = 0;
+        bool wrong = false;
+        if (mine) {
+            L = e.symbols[tid].length;
+            sym = e.symbols[tid].symbol;
+            prev = tid ? e.symbols[tid - 1].length : 0u;
+            const uint32_t bit = 1u << (sym & 31);
+            wrong = L < 1 || L > (uint32_t)kMaxLen || L < prev || (atomicOr(&s.seen[sym >> 5], bit) & bit);
+        }
+        const uint32_t span_c = mine && !wrong ? 1u << (kMaxLen - L) : 0u;
+        const uint32_t run = warp_incl_scan(span_c, lane);
+        if (lane == 31) s_warp[warp] = run;
+        bad = __syncthreads_or(wrong) || bad;
+        const uint32_t runs = warp_incl_scan(lane < kTableThreads / 32 ? s_warp[lane] : 0u, lane);
+        const uint32_t kraft = __shfl_sync(kFull, runs, kTableThreads / 32 - 1);
+        const uint32_t la = (warp ? __shfl_sync(kFull, runs, warp - 1) : 0u) + run - span_c;
+        if (kraft > (1u << kMaxLen)) bad = true;
         uint32_t c = kNoClass;
         if (!bad && n) {  // uniform over the CTA
             // the largest symbol index i >= from with la[i] <= v (la[0] = 0, la ascends)
@@ -428,63 +464,93 @@ __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t c
                 return lo;
             };
             auto entry = [&](uint32_t i, uint32_t v) -> uint16_t {
-                const uint32_t L = s.clen[i];
-                if (v < s.la[i] || v - s.la[i] >= (1u << (kMaxLen - L))) return kDecInvalid;
-                return (uint16_t)(((L - 1) << 8) | s.sym[i]);
+                const uint32_t l = s.clen[i];
+                if (v < s.la[i] || v - s.la[i] >= (1u << (kMaxLen - l))) return kDecInvalid;
+                return (uint16_t)(((l - 1) << 8) | s.sym[i]);
             };
-            const uint32_t x0 = kPer * tid;
-            // pass 1: the level-1 entries, and the widths of this thread's pointer prefixes
-            uint32_t span = 0, pmask = 0;
-            uint32_t i_first = search(x0 << X), i_last = i_first;
-            const uint32_t i_start = i_first;
-#pragma unroll
-            for (uint32_t k = 0; k < kPer; ++k) {
-                const uint32_t x = x0 + k;
-                const uint32_t v = x << X;
-                i_first = advance(i_first, v);
-                i_last = advance(i_last > i_first ? i_last : i_first, v | ((1u << X) - 1));
-                const uint32_t L = s.clen[i_last];
-                if (L > P && (s.la[i_last] >> X) == x) {
-                    span += 1u << (L - P);
-                    pmask |= 1u << k;
-                    s1[x] = 0x8000u;  // (a wide book's get their width and offset below)
-                } else {
-                    s1[x] = entry(i_first, v);
-                }
-            }
-            // the first prefix of a longer code, and the block scan of the spans: the level-2
-            // offset of this thread's first group (a wide book's)
-            const uint32_t incl = warp_incl_scan(span, lane);
-            if (lane == 31) s_warp[warp] = incl;
-            if (pmask) atomicMin(&s_long, x0 + __ffs(pmask) - 1);
-            __syncthreads();
-            const uint32_t cc = class_of(s.clen[0], kraft == (1u << kMaxLen));
+            // the class, and the shape of its table
+            const bool complete = kraft == (1u << kMaxLen);
+            const uint32_t cc = class_of(e.symbols[0].length, complete);
             const int rows = kStageRows[cc >> 1];
-            const uint32_t max_len = s.clen[n - 1], first_long = s_long;
-            const DecIndex ix = dec_index(first_long, max_len, (cc & 1u) != 0, rows);
-            const bool multi = dec_multi(rows, (cc & 1u) != 0);
-            DecTableW& w = wtables[j];
-            if (!ix.wide) {
-                c = cc;
-                const uint32_t extra = 32 - kDecPrefix - ix.shift;
-                for (uint32_t i = tid; i < ix.used; i += kTableThreads) {
-                    uint32_t e2 = kEntInvalid;
-                    const uint32_t v = (uint32_t)((int32_t)i - ix.offset);  // from first_long on: the window's bits
-                    if (i < first_long) {
-                        e2 = multi ? entry_multi(s1, i) : entry_pair(s1, i);
-                    } else if (v < kT1 << extra) {
-                        const uint32_t v16 = v << (kMaxLen - kDecPrefix - extra);
-                        const uint32_t e1 = entry(search(v16), v16);
-                        e2 = multi ? entry_single<true>(e1) : entry_single<false>(e1);
-                    }
-                    w.t1[i] = e2;
+            const uint32_t Pr = dec_prefix(rows);
+            if (mine) {
+                s.la[tid] = la;
+                s.sym[tid] = (uint8_t)sym;
+                s.clen[tid] = (uint8_t)L;
+                s1[la >> X] = L > P ? kLongCode : (uint16_t)((L << 8) | sym);  // (one code, or all long ones)
+                if (L > Pr && prev <= Pr) s_long = la >> (kMaxLen - Pr);
+            }
+            __syncthreads();
+            const uint32_t x0 = kPer * tid;
+            if (complete) {  // every 11-bit prefix's code: the last one to start at or below it
+                uint4* const own = reinterpret_cast<uint4*>(s1) + tid;
+                uint4 q = *own;
+                uint32_t* const h = &q.x;
+                uint32_t cur = h[0] & 0xffffu;
+                if (cur == 0xffffu) {
+                    const uint32_t i = search(x0 << X);  // (shorter than P bits, or a code would start here)
+                    cur = ((uint32_t)s.clen[i] << 8) | s.sym[i];
                 }
+#pragma unroll
+                for (uint32_t k = 0; k < kPer / 2; ++k) {
+                    const uint32_t lo = h[k] & 0xffffu, hi = h[k] >> 16;
+                    const uint32_t e0 = lo == 0xffffu ? cur : lo;
+                    cur = hi == 0xffffu ? e0 : hi;
+                    h[k] = e0 | (cur << 16);
+                }
+                *own = q;
+            }
+            __syncthreads();
+            const DecIndex ix = dec_index(s_long < 1u << Pr ? s_long : 1u << Pr, s.clen[n - 1], complete, rows);
+            const bool multi = dec_multi(rows, complete);
+            DecTableW& w = wtables[j];
+            if (ix.first_long != kDecWide) {
+                c = cc;
+                if (multi)
+                    for (uint32_t i = tid; i < ix.first_long; i += kTableThreads)
+                        w.t1[i] = window_entry<dec_prefix(32), true>(s1, i);
+                else
+                    for (uint32_t i = tid; i < ix.first_long; i += kTableThreads)
+                        w.t1[i] = window_entry<kDecPrefix, false>(s1, i);
+                // the longer codes: each thread its symbol's entries, and the padding to whole 16 bytes
+                const uint32_t len = 32 - ix.shift;  // the longest, or the prefix's if none is longer
+                const uint32_t end = (1u << len) + ix.offset;
+                if (mine && L > Pr) {
+                    const uint32_t v = (((L - 1) << 8) | sym);
+                    const uint32_t e1 = multi ? entry_single<true>(v) : entry_single<false>(v);
+                    uint32_t* const at = w.t1 + (int32_t)(la >> (kMaxLen - len)) + ix.offset;
+                    for (uint32_t k = 0; k < 1u << (len - L); ++k) at[k] = e1;
+                }
+                if (tid < ix.used - end) w.t1[end + tid] = kEntInvalid;
             } else {
+                // two levels: the level-1 entries, and the widths of this thread's pointer prefixes
+                uint32_t span = 0, pmask = 0;
+                const uint32_t i_start = search(x0 << X);
+                uint32_t i_first = i_start, i_last = i_first;
+                for (uint32_t k = 0; k < kPer; ++k) {
+                    const uint32_t x = x0 + k;
+                    const uint32_t v = x << X;
+                    i_first = advance(i_first, v);
+                    i_last = advance(i_last > i_first ? i_last : i_first, v | ((1u << X) - 1));
+                    const uint32_t l = s.clen[i_last];
+                    if (l > P && (s.la[i_last] >> X) == x) {
+                        span += 1u << (l - P);
+                        pmask |= 1u << k;
+                    } else {
+                        s1[x] = entry(i_first, v);
+                    }
+                }
+                // block scan of the spans: the level-2 offset of this thread's first group
+                const uint32_t incl = warp_incl_scan(span, lane);
+                if (lane == 31) s_warp[warp] = incl;
+                __syncthreads();
                 const uint32_t wt = warp_incl_scan(lane < kTableThreads / 32 ? s_warp[lane] : 0u, lane);
                 const uint32_t total = __shfl_sync(kFull, wt, kTableThreads / 32 - 1);
                 uint32_t off = (warp ? __shfl_sync(kFull, wt, warp - 1) : 0u) + incl - span;
                 if (total <= (uint32_t)kDecT2Cap) {  // uniform; larger only for an incomplete book
-                    c = cc;
+                    // (one decoder launch serves the incomplete books of every shortest code: only
+                    // hand-made ones and those of a single symbol are incomplete)
+                    c = complete ? cc : kIncomplete;
                     // pass 2: the pointer prefixes, and every prefix's level-2 end offset
                     i_first = i_start;
                     for (uint32_t k = 0; k < kPer; ++k) {
@@ -522,13 +588,18 @@ __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t c
                         w.t2()[k] = e2;
                     }
                     for (uint32_t i = tid; i < kT1; i += kTableThreads)
-                        w.t1[i] = multi ? entry_multi(s1, i) : entry_pair(s1, i);
+                        w.t1[i] = multi ? entry_multi<kDecPrefix>(s1, i) : entry_pair<kDecPrefix>(s1, i);
                 } else {
                     bad = true;
                 }
             }
+            if (!bad && e.segments && class_mask && !(class_mask >> cc & 1u)) {
+                // a class the caller left out of the launch: the buffer stays undecoded
+                if (tid == 0) atomicOr(status, kDevPlan);
+                c = kNoClass;
+            }
             if (c != kNoClass) {
-                for (uint32_t i = tid; i < n; i += kTableThreads) w.symlen[s.sym[i]] = s.clen[i];
+                if (mine) w.symlen[sym] = (uint8_t)L;
                 if (tid == 0) w.index = ix;
             }
         }
@@ -571,8 +642,7 @@ __global__ void __launch_bounds__(kTableThreads, 8) bdec_table_kernel(uint32_t c
 // only entry the map and the decoder read).
 __global__ void __launch_bounds__(kScanThreads) bdec_setup_kernel(uint32_t count, const uint8_t* cls, DecJob* jobs,
                                                                   uint64_t* item0s, uint64_t* class_nitems,
-                                                                  uint64_t tiles_cap, uint32_t class_mask,
-                                                                  uint32_t* status) {
+                                                                  uint64_t tiles_cap, uint32_t* status) {
     constexpr uint32_t kSums = kClasses + 1;  // the classes, then all tiles
     constexpr uint32_t kWarps = kScanThreads / 32;
     __shared__ uint64_t s_tot[2][kSums][kWarps];  // by chunk parity: warp totals, then warp offsets
@@ -652,8 +722,6 @@ __global__ void __launch_bounds__(kScanThreads) bdec_setup_kernel(uint32_t count
         const uint64_t tk = s_carry[threadIdx.x];
         item0s[(uint64_t)threadIdx.x * (count + 1) + count] = tk;
         class_nitems[threadIdx.x] = fits ? tk : 0;
-        // a class the caller left out of the launch holds buffers: they stay undecoded
-        if (class_mask && tk && !(class_mask >> threadIdx.x & 1u)) atomicOr(status, kDevPlan);
     }
 }
 
@@ -945,12 +1013,17 @@ hgap_status hgap_batch_decompress(uint32_t count, const hgap_batch_entry* d_entr
     uint64_t* records = reinterpret_cast<uint64_t*>(ws + L.records);
     uint32_t* job_of = reinterpret_cast<uint32_t*>(ws + L.job_of);
 
+    // (the workspace's room tells the buffers' average size: a tile for every 2048 bytes)
+    const uint32_t tile_segs = cfg->dec_tile_segs ? cfg->dec_tile_segs
+                               : L.tiles_cap < 32 * (uint64_t)count ? kDecTileSmall
+                                                                    : 0;
     if (cudaMemsetAsync(ws, 0, 1024, st) != cudaSuccess) return HGAP_ERR_CUDA;
     bdec_table_kernel<<<table_grid(count), kTableThreads, 0, st>>>(count, d_entries, d_bits, d_gaps, d_outputs,
-                                                                   cfg->dec_tile_segs, wtables, cls, jobs, status);
+                                                                   tile_segs, cfg->dec_class_mask, wtables, cls, jobs,
+                                                                   status);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
     bdec_setup_kernel<<<scan_grid(count), kScanThreads, 0, st>>>(count, cls, jobs, item0s, class_nitems, L.tiles_cap,
-                                                  cfg->dec_class_mask, status);
+                                                  status);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
     bdec_map_kernel<<<book_grid(count), 32 * kBookWarps, 0, st>>>(count, jobs, cls, item0s, job_of, L.tiles_cap);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
@@ -960,7 +1033,10 @@ hgap_status hgap_batch_decompress(uint32_t count, const hgap_batch_entry* d_entr
     std::memset(&unused, 0, sizeof(unused));
     static const uint32_t kMinLen[4] = {4, 3, 2, 1};  // a representative shortest code per stage size
     for (uint32_t c = 0; c < kClasses; ++c) {
-        if (cfg->dec_class_mask && !(cfg->dec_class_mask >> c & 1u)) continue;
+        // complete books' classes, and one launch for all incomplete ones
+        if (!(c & 1u) && c != kIncomplete) continue;
+        const uint32_t named = c == kIncomplete ? 0x55u : 1u << c;
+        if (cfg->dec_class_mask && !(cfg->dec_class_mask & named)) continue;
         DecArgs a;
         std::memset(&a, 0, sizeof(a));
         a.jobs = jobs;
@@ -974,7 +1050,7 @@ hgap_status hgap_batch_decompress(uint32_t count, const hgap_batch_entry* d_entr
         a.status = status;
         // batched streams are compressible ones on the whole: always two symbols per lookup where they fit
         if (launch_decode(a, unused, kMinLen[c / 2], (c & 1) != 0, true, (int)cfg->dec_ctas_per_sm,
-                          cfg->dec_tile_segs, stream) != 0)
+                          tile_segs, stream) != 0)
             return HGAP_ERR_CUDA;
     }
     return HGAP_OK;

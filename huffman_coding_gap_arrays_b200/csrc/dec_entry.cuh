@@ -35,31 +35,33 @@ __device__ __forceinline__ uint32_t code_in_window(const uint16_t* t1src, uint32
     return e & (0x8000u | kDecInvalid) ? 0u : ((e >> 8) & 15u) + 1u;
 }
 
-// Level-1 entry for prefix x: when the first code leaves room for a whole
-// second code inside the same 11-bit window, both at once.  The second code is
-// known from the bits after the first alone, because it ends inside the window.
+// The entry of P-bit window x: when the first code leaves room for a whole
+// second code inside the same window, both at once.  The second code is known
+// from the bits after the first alone, because it ends inside the window.
+template <uint32_t P>
 __device__ __forceinline__ uint32_t entry_pair(const uint16_t* t1src, uint32_t x) {
-    constexpr uint32_t P = kDecPrefix;
+    const uint32_t x11 = x << (kDecPrefix - P);
     uint32_t s1, s2;
-    const uint32_t l1 = code_in_window(t1src, x, s1);
-    if (l1 == 0 || l1 >= P) return entry_single<false>(t1src[x]);
-    const uint32_t l2 = code_in_window(t1src, x << l1, s2);
-    if (l2 == 0 || l1 + l2 > P) return entry_single<false>(t1src[x]);
+    const uint32_t l1 = code_in_window(t1src, x11, s1);
+    if (l1 == 0 || l1 >= P) return entry_single<false>(t1src[x11]);
+    const uint32_t l2 = code_in_window(t1src, x11 << l1, s2);
+    if (l2 == 0 || l1 + l2 > P) return entry_single<false>(t1src[x11]);
     return s1 | (s2 << 8) | ((l1 + l2) << 16) | 0x02000000u;
 }
 
 // The same with up to three codes (multi form; complete books).
+template <uint32_t P>
 __device__ __forceinline__ uint32_t entry_multi(const uint16_t* t1src, uint32_t x) {
-    constexpr uint32_t P = kDecPrefix;
+    const uint32_t x11 = x << (kDecPrefix - P);
     uint32_t s1, s2, s3;
-    const uint32_t l1 = code_in_window(t1src, x, s1);
-    if (l1 == 0 || l1 >= P) return entry_single<true>(t1src[x]);
-    const uint32_t l2 = code_in_window(t1src, x << l1, s2);
-    if (l2 == 0 || l1 + l2 > P) return entry_single<true>(t1src[x]);
+    const uint32_t l1 = code_in_window(t1src, x11, s1);
+    if (l1 == 0 || l1 >= P) return entry_single<true>(t1src[x11]);
+    const uint32_t l2 = code_in_window(t1src, x11 << l1, s2);
+    if (l2 == 0 || l1 + l2 > P) return entry_single<true>(t1src[x11]);
     const uint32_t l12 = l1 + l2;
     const uint32_t two = s1 | (s2 << 8) | (l12 << 24) | (1u << 29);
     if (l12 >= P) return two;
-    const uint32_t l3 = code_in_window(t1src, x << l12, s3);
+    const uint32_t l3 = code_in_window(t1src, x11 << l12, s3);
     if (l3 == 0 || l12 + l3 > P) return two;
     return s1 | (s2 << 8) | (s3 << 16) | ((l12 + l3) << 24) | (2u << 29);
 }

@@ -66,6 +66,7 @@ struct DecCfg {
     static constexpr int kMaxSym = 4 * R;
     static constexpr int kSegs = 32 * W * S;           // segments per tile
     static constexpr int kThreads = 32 * (W + 1);
+    static constexpr uint32_t P = dec_prefix(R);       // window bits of a lookup
     static constexpr int kTab = (int)dec_table_cap(R); // u32 table entries
     // one segment's row: its symbols, a byte or two that a multi-symbol entry stores past the
     // count, and the word after the last whole one; an odd number of words, so that the 32 rows a
@@ -94,9 +95,9 @@ struct Table {
 };
 
 // The entry (dec_entry.cuh) of the 32-bit window x at a code's start.
-template <bool WIDE, bool MULTI>
+template <uint32_t P, bool WIDE, bool MULTI>
 __device__ __forceinline__ uint32_t lookup(const Table& t, uint32_t x) {
-    const int32_t i1 = (int32_t)(x >> (32 - kDecPrefix));
+    const int32_t i1 = (int32_t)(x >> (32 - (WIDE ? (uint32_t)kDecPrefix : P)));
     if (!WIDE) return t.t1[max(i1, (int32_t)(x >> t.shift) + t.offset)];
     uint32_t e = t.t1[i1];
     if (e & kEntPointer) {
@@ -127,17 +128,17 @@ __device__ __forceinline__ void st_shared_u8(uint32_t addr, uint32_t v) {
 // address `row` on; their number is returned in `cnt`.  Returns the end bit of
 // the last code relative to phase 3 (32 + the next gap entry for a valid
 // stream), or a value no stream yields after an invalid code.
-template <bool WIDE, bool COMPLETE, bool PAIRS, bool MULTI>
+template <uint32_t P, bool WIDE, bool COMPLETE, bool PAIRS, bool MULTI>
 __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWords& w, uint32_t pos, uint32_t row,
                                                    uint32_t& cnt) {
     static_assert(!MULTI || COMPLETE, "multi entries: complete books");
     constexpr uint32_t kBad = 1u << 16;
-    constexpr uint32_t kEarly = kDecPrefix - 1;  // the last phase's fast loop ends this many bits early
+    constexpr uint32_t kEarly = (WIDE ? (uint32_t)kDecPrefix : P) - 1;  // the last phase's fast loop ends this many bits early
     if (MULTI) {
         uint32_t out = row;
         auto fast = [&](uint32_t cw, uint32_t nw) {
             while (!(pos & 32)) {
-                const uint32_t e = lookup<WIDE, true>(t, __funnelshift_l(nw, cw, pos));
+                const uint32_t e = lookup<P, WIDE, true>(t, __funnelshift_l(nw, cw, pos));
                 st_shared_u8(out, e);
                 st_shared_u8(out + 1, e >> 8);
                 st_shared_u8(out + 2, e >> 16);
@@ -154,7 +155,7 @@ __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWord
         fast(w.w3 >> kEarly, __funnelshift_r(w.w4, w.w3, kEarly));
         pos -= kEarly;
         while (!(pos & 32)) {
-            const uint32_t e = lookup<WIDE, true>(t, __funnelshift_l(w.w4, w.w3, pos));
+            const uint32_t e = lookup<P, WIDE, true>(t, __funnelshift_l(w.w4, w.w3, pos));
             const uint32_t tot = (e >> 24) & 31u, more = e >> 29;
             st_shared_u8(out, e);
             st_shared_u8(out + 1, e >> 8);
@@ -169,7 +170,7 @@ __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWord
     uint32_t s = (row << 8) | pos;
     auto fast = [&](uint32_t cw, uint32_t nw) -> bool {  // false: an invalid code
         while (!(s & 32)) {
-            const uint32_t e = lookup<WIDE, false>(t, __funnelshift_l(nw, cw, s));
+            const uint32_t e = lookup<P, WIDE, false>(t, __funnelshift_l(nw, cw, s));
             if (!COMPLETE && (e & kEntInvalidBit)) return false;
             st_shared_u8(s >> 8, e);
             if (PAIRS) st_shared_u8((s >> 8) + 1, e >> 8);  // a single entry's second byte: overwritten or past the count
@@ -189,7 +190,7 @@ __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWord
         if (!fast(w.w3 >> kEarly, __funnelshift_r(w.w4, w.w3, kEarly))) return false;
         s -= kEarly;
         while (!(s & 32)) {  // the last bits: only the codes that start before bit 32
-            const uint32_t e = lookup<WIDE, false>(t, __funnelshift_l(w.w4, w.w3, s));
+            const uint32_t e = lookup<P, WIDE, false>(t, __funnelshift_l(w.w4, w.w3, s));
             if (!COMPLETE && (e & kEntInvalidBit)) return false;
             st_shared_u8(s >> 8, e);
             st_shared_u8((s >> 8) + 1, e >> 8);
@@ -210,14 +211,14 @@ __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWord
 // The stream's last segment: its codes end at bit `end` (<= 128) and zero
 // padding follows, which may not decode.  One code per step (the first code of
 // any pair or multi entry), the words picked by index.
-template <bool WIDE, bool COMPLETE, bool MULTI>
+template <uint32_t P, bool WIDE, bool COMPLETE, bool MULTI>
 __device__ __forceinline__ uint32_t decode_last_segment(const Table& t, const SegWords& w, uint32_t pos, uint32_t end,
                                                         uint32_t row) {
     auto word = [&](uint32_t i) { return i == 0 ? w.w0 : i == 1 ? w.w1 : i == 2 ? w.w2 : i == 3 ? w.w3 : w.w4; };
     uint32_t cnt = 0;
     while (pos < end) {
         const uint32_t wi = pos >> 5;
-        const uint32_t e = lookup<WIDE, MULTI>(t, __funnelshift_l(word(wi + 1), word(wi), pos));
+        const uint32_t e = lookup<P, WIDE, MULTI>(t, __funnelshift_l(word(wi + 1), word(wi), pos));
         if (!COMPLETE && (e & kEntInvalidBit)) break;  // the padding after the final codeword
         const uint32_t more = MULTI ? e >> 29 : (e >> 24) - 1;
         const uint32_t len = MULTI ? (e >> 24) & 31u : (e >> 16) & 31u;
@@ -312,21 +313,33 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
         for (int i = tid; i < kRaw; i += C::kThreads) raw[i] = src[i];
         __syncthreads();
         const DecTable& r = *reinterpret_cast<const DecTable*>(areas);
+        const bool wide = a.index.first_long == kDecWide;
         for (int i = tid; i < (int)a.index.used; i += C::kThreads) {
             uint32_t e = kEntInvalid;
-            if (i < kT1 && (a.index.wide || !(r.t1[i] & 0x8000u))) {
-                e = MULTI ? entry_multi(r.t1, i) : PAIRS ? entry_pair(r.t1, i) : entry_single<false>(r.t1[i]);
-                const uint32_t e1 = r.t1[i];
-                if (!(e1 & (0x8000u | kDecInvalid))) symlen[e1 & 0xffu] = (uint8_t)((e1 >> 8) + 1);
+            if (wide) {
+                e = MULTI   ? entry_multi<kDecPrefix>(r.t1, i)
+                    : PAIRS ? entry_pair<kDecPrefix>(r.t1, i)
+                            : entry_single<false>(r.t1[i]);
+            } else if ((uint32_t)i < a.index.first_long) {
+                e = MULTI   ? entry_multi<C::P>(r.t1, i)
+                    : PAIRS ? entry_pair<C::P>(r.t1, i)
+                            : entry_single<false>(r.t1[i << (kDecPrefix - C::P)]);
             } else {
                 // a longer code: v = its window's bits down to the longest length
-                const uint32_t v = (uint32_t)(i - a.index.offset), extra = 32 - kDecPrefix - a.index.shift;
-                if (v < (uint32_t)kT1 << extra) {
-                    const uint32_t e1 = r.t1[v >> extra], w = (e1 >> 12) & 7u;
-                    e = entry_single<MULTI>(r.t2[(e1 & 0xfffu) + ((v & ((1u << extra) - 1u)) >> (extra - w))]);
+                const uint32_t v = (uint32_t)(i - a.index.offset), len = 32 - a.index.shift;
+                if (v < 1u << len) {
+                    const uint32_t below = len - kDecPrefix;  // (len is 11 or more)
+                    uint32_t e1 = r.t1[v >> below];
+                    if (e1 & 0x8000u)
+                        e1 = r.t2[(e1 & 0xfffu) + ((v & ((1u << below) - 1u)) >> (below - ((e1 >> 12) & 7u)))];
+                    e = entry_single<MULTI>(e1);
                 }
             }
             t1[i] = e;
+        }
+        for (int i = tid; i < kT1; i += C::kThreads) {
+            const uint32_t e1 = r.t1[i];
+            if (!(e1 & (0x8000u | kDecInvalid))) symlen[e1 & 0xffu] = (uint8_t)((e1 >> 8) + 1);
         }
     }
     if (tid == 32 * W) {
@@ -447,14 +460,14 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
             auto segment = [&](auto wide) {
                 constexpr bool WIDE = decltype(wide)::value;
                 if (T.last_bits && u + 1 == T.nseg) {
-                    n[k] = decode_last_segment<WIDE, COMPLETE, MULTI>(t, w, pos, T.last_bits, row);
+                    n[k] = decode_last_segment<C::P, WIDE, COMPLETE, MULTI>(t, w, pos, T.last_bits, row);
                 } else {
-                    const uint32_t end = decode_segment<WIDE, COMPLETE, PAIRS, MULTI>(t, w, pos, row, n[k]);
+                    const uint32_t end = decode_segment<C::P, WIDE, COMPLETE, PAIRS, MULTI>(t, w, pos, row, n[k]);
                     if (end != 32 + gap) atomicOr(a.status, kDevCorrupt);
                 }
             };
             if (u < T.nseg && alive) {
-                if (COMPLETE && !T.index.wide) segment(std::integral_constant<bool, false>());
+                if (COMPLETE && T.index.first_long != kDecWide) segment(std::integral_constant<bool, false>());
                 else segment(std::integral_constant<bool, true>());
             }
         }

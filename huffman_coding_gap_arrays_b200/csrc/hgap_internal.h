@@ -231,9 +231,15 @@ HGAP_HD constexpr int dec_stage_rows(uint32_t min_len) {
 // leave one CTA per SM.
 HGAP_HD constexpr int dec_tile_segs(int R) { return R >= 32 ? 256 : 512; }
 // The same with a launch-shape override of 256 or 512 segments (0: the
-// default; 32 rows keep 256).
+// default; 32 rows keep 256), or kDecTileSmall for a batch of small buffers,
+// whose last tiles are mostly empty: 256 for 16 rows (4096 buffers of 4-64 KiB:
+// that class 81 -> 67 us; 11 rows 58 -> 61 and 8 rows 12.7 -> 11.7, left alone).
+constexpr uint32_t kDecTileSmall = 1;
 HGAP_HD constexpr int dec_tile_segs_for(int R, uint32_t override_segs) {
-    return R >= 32 ? 256 : (override_segs == 256 || override_segs == 512) ? (int)override_segs : dec_tile_segs(R);
+    return override_segs == kDecTileSmall && R == 16                 ? 256
+           : R >= 32                                                 ? 256
+           : (override_segs == 256 || override_segs == 512)          ? (int)override_segs
+                                                                     : dec_tile_segs(R);
 }
 constexpr int kDecT2Cap = 2560;  // >= the largest complete 16-bit book (see host.cpp)
 constexpr uint16_t kDecInvalid = 0x4000;
@@ -252,33 +258,39 @@ HGAP_HD constexpr bool dec_multi(int rows, bool complete) { return complete && r
 
 // The decode kernel's table in shared memory.  A canonical code's long codes
 // are the last in code order, so ONE table serves all lengths: a 32-bit window
-// x at a code's start has the entry max(x >> 21, (x >> shift) + offset) -- below
-// the first prefix with codes of more than kDecPrefix bits its 11-bit prefix,
-// from there on its first kMaxLen (or the book's longest length) bits, counted
-// on from that prefix (both lines meet there, and the second is the steeper
-// one).  No second lookup, no branch.  Of 1500 books of the batched workload's
-// distributions 97 % (99.6 % of the bytes) fit dec_table_cap entries; the others
-// ("wide") keep two levels: 2048 entries, and a level-2 table in global memory
-// for the codes over 11 bits, reached by a branch.
-HGAP_HD constexpr uint32_t dec_table_cap(int rows) { return rows >= 32 ? 3840u : 2432u; }
+// x at a code's start has the entry max(x >> (32 - P), (x >> shift) + offset) --
+// below the first P-bit prefix with codes of more than P bits that prefix, from
+// there on its first bits up to the book's longest length, counted on from that
+// prefix (both lines meet there, and the second is the steeper one).  No second
+// lookup, no branch.  P is 11, or 10 for the 32-row decoder, whose stage leaves
+// room for three CTAs an SM only with a table this small (its books' codes are
+// short: three fit 10 bits nearly as often; 1024 buffers of 4 KiB-4 MiB, that
+// class's launch: 179 us with 11 bits and two CTAs, 150 us).  Of 1500 books of the batched
+// workload's distributions 96 % (99.5 % of the bytes) fit dec_table_cap entries;
+// the others ("wide") keep two levels: 2048 entries for 11 bits, and a level-2
+// table in global memory for longer codes, reached by a branch.
+HGAP_HD constexpr uint32_t dec_prefix(int rows) { return rows >= 32 ? 10u : (uint32_t)kDecPrefix; }
+HGAP_HD constexpr uint32_t dec_table_cap(int rows) { return rows >= 32 ? 2176u : 2432u; }
 struct DecIndex {
-    uint32_t used;   // entries
-    uint32_t shift;  // of x
+    uint32_t used;        // entries
+    uint32_t shift;       // of x
     int32_t offset;
-    uint32_t wide;   // two levels instead
+    uint32_t first_long;  // the first prefix with longer codes; kDecWide: two levels instead
 };
-// From the first 11-bit prefix of a longer code (2048: none), the longest
-// length, and whether the book is complete (an incomplete one is wide: its
-// prefixes without a code have no place in one table).
+constexpr uint32_t kDecWide = ~0u;
+// From the first such prefix (2^P: none), the longest length, and whether the
+// book is complete (an incomplete one is wide: its prefixes without a code have
+// no place in one table).
 HGAP_HD inline DecIndex dec_index(uint32_t first_long, uint32_t max_len, bool complete, int rows) {
-    constexpr uint32_t n1 = 1u << kDecPrefix;
+    const uint32_t P = dec_prefix(rows), n1 = 1u << P;
     DecIndex d;
-    const uint32_t extra = max_len > (uint32_t)kDecPrefix && first_long < n1 ? max_len - kDecPrefix : 0u;
+    const uint32_t extra = max_len > P && first_long < n1 ? max_len - P : 0u;
     const uint32_t used = extra ? first_long + ((n1 - first_long) << extra) : n1;
-    d.wide = !complete || used > dec_table_cap(rows);
-    d.used = d.wide ? n1 : (used + 3) & ~3u;
-    d.shift = 32 - kDecPrefix - (d.wide ? 0u : extra);
-    d.offset = d.wide || !extra ? 0 : (int32_t)first_long - (int32_t)(first_long << extra);
+    const bool wide = !complete || used > dec_table_cap(rows);
+    d.used = wide ? 1u << kDecPrefix : (used + 3) & ~3u;
+    d.shift = wide ? 32 - kDecPrefix : 32 - P - extra;
+    d.offset = wide || !extra ? 0 : (int32_t)first_long - (int32_t)(first_long << extra);
+    d.first_long = wide ? kDecWide : first_long;
     return d;
 }
 
@@ -288,11 +300,11 @@ HGAP_HD inline DecIndex dec_index(uint32_t first_long, uint32_t max_len, bool co
 struct alignas(16) DecTableW {
     DecIndex index;
     uint8_t symlen[256];  // each symbol's code length
-    uint32_t t1[dec_table_cap(32)];
+    uint32_t t1[(1 << kDecPrefix) + kDecT2Cap / 2];
     HGAP_HD uint16_t* t2() { return reinterpret_cast<uint16_t*>(t1 + (1 << kDecPrefix)); }
     HGAP_HD const uint16_t* t2() const { return reinterpret_cast<const uint16_t*>(t1 + (1 << kDecPrefix)); }
 };
-static_assert(((1 << kDecPrefix) + kDecT2Cap / 2) <= (int)dec_table_cap(32), "level 2 of a wide book fits behind level 1");
+static_assert((1 << kDecPrefix) + kDecT2Cap / 2 >= (int)dec_table_cap(8), "room for every table");
 static_assert(sizeof(DecTableW) % 16 == 0, "16-byte copies");
 
 // One stream to decode (same single / batched scheme as EncJob).  Its tiles

@@ -207,9 +207,10 @@ double dec_pair_fraction(const hgap_codebook& cb) {
 
 DecIndex dec_index_of(const hgap_codebook& cb, bool complete, int rows) {
     uint32_t first_long = 0, max_len = 0;
+    const uint32_t P = dec_prefix(rows);
     for (uint32_t i = 0; i < cb.symbol_count; ++i) {
         const uint32_t l = cb.symbols[i].length;
-        if (l <= (uint32_t)kDecPrefix) first_long += 1u << (kDecPrefix - l);
+        if (l <= P) first_long += 1u << (P - l);
         if (l > max_len) max_len = l;
     }
     return dec_index(first_long, max_len, complete, rows);
