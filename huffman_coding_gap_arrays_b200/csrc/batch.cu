@@ -794,9 +794,10 @@ uint32_t base_chunks(const hgap_batch_config* cfg) {
     return rc > 32 ? 32 : rc;
 }
 
-// Compress workspace: [header 1024: status @0, counter @4, nitems @64]
-// [jobs] [item0s] [tables] [hists] then the per-region arrays [st_rec | plan | st_hist]
-// for as many regions as the rest of the workspace holds.
+// Compress workspace: [header 1024: status @0, counter @4, nitems @64] [hists]
+// [st_rec] (zero at the start of a call, together: one memset) [jobs] [item0s]
+// [tables] [plan] [st_hist], the per-region arrays (st_rec, plan, st_hist) for
+// as many regions as the workspace holds.
 constexpr size_t kEncPerRegion = 8 + sizeof(EncRegion) + 1024;
 
 struct EncLayout {
@@ -806,19 +807,16 @@ struct EncLayout {
 
 EncLayout enc_layout(uint32_t count, size_t workspace_bytes) {
     EncLayout L;
-    size_t off = 1024;
-    L.jobs = off;
-    off = align256(off + sizeof(EncJob) * (size_t)count);
-    L.item0s = off;
-    off = align256(off + 8 * ((size_t)count + 1));
-    L.tables = off;
-    off = align256(off + sizeof(EncTable) * (size_t)count);
-    L.hists = off;
-    off = align256(off + 1024 * (size_t)count);
-    L.fixed = off;
-    L.max_regions = workspace_bytes > off + 512 ? (workspace_bytes - off - 512) / kEncPerRegion : 0;
-    L.st_rec = off;
-    L.plan = align256(off + 8 * (size_t)L.max_regions);
+    const size_t jobs = align256(sizeof(EncJob) * (size_t)count), item0s = align256(8 * ((size_t)count + 1));
+    const size_t tables = align256(sizeof(EncTable) * (size_t)count);
+    L.hists = 1024;
+    L.st_rec = L.hists + 1024 * (size_t)count;
+    L.fixed = L.st_rec + jobs + item0s + tables;
+    L.max_regions = workspace_bytes > L.fixed + 512 ? (workspace_bytes - L.fixed - 512) / kEncPerRegion : 0;
+    L.jobs = align256(L.st_rec + 8 * (size_t)L.max_regions);
+    L.item0s = L.jobs + jobs;
+    L.tables = L.item0s + item0s;
+    L.plan = L.tables + tables;
     L.st_hist = align256(L.plan + sizeof(EncRegion) * (size_t)L.max_regions);
     return L;
 }
@@ -831,8 +829,9 @@ uint64_t worst_regions(uint32_t count, const uint64_t* sizes, const hgap_batch_c
 }
 
 // Decompress workspace: [header 1024: status @0, counters[8] @64, class nitems[8] @128]
-// [jobs] [widened tables] [classes] [item0s 8 x (count+1)] then the per-tile arrays
-// [records | job_of 8 x cap] for as many tiles as the rest holds.
+// [records] (zero at the start of a call, together) [jobs] [widened tables] [classes]
+// [item0s 8 x (count+1)] [job_of 8 x cap], the per-tile arrays (records, job_of) for as
+// many tiles as the workspace holds.
 constexpr size_t kDecPerTile = 8 + 4 * kClasses;
 
 struct DecLayout {
@@ -842,19 +841,16 @@ struct DecLayout {
 
 DecLayout dec_layout(uint32_t count, size_t workspace_bytes) {
     DecLayout L;
-    size_t off = 1024;
-    L.jobs = off;
-    off = align256(off + sizeof(DecJob) * (size_t)count);
-    L.wtables = off;
-    off = align256(off + sizeof(DecTableW) * (size_t)count);
-    L.cls = off;
-    off = align256(off + (size_t)count);
-    L.item0s = off;
-    off = align256(off + 8 * (size_t)kClasses * ((size_t)count + 1));
-    L.fixed = off;
-    L.tiles_cap = workspace_bytes > off + 256 ? (workspace_bytes - off - 256) / kDecPerTile : 0;
-    L.records = off;
-    L.job_of = align256(off + 8 * (size_t)L.tiles_cap);
+    const size_t jobs = align256(sizeof(DecJob) * (size_t)count), wtables = align256(sizeof(DecTableW) * (size_t)count);
+    const size_t cls = align256((size_t)count), item0s = align256(8 * (size_t)kClasses * ((size_t)count + 1));
+    L.records = 1024;
+    L.fixed = L.records + jobs + wtables + cls + item0s;
+    L.tiles_cap = workspace_bytes > L.fixed + 256 ? (workspace_bytes - L.fixed - 256) / kDecPerTile : 0;
+    L.jobs = align256(L.records + 8 * (size_t)L.tiles_cap);
+    L.wtables = L.jobs + jobs;
+    L.cls = L.wtables + wtables;
+    L.item0s = L.cls + cls;
+    L.job_of = L.item0s + item0s;
     return L;
 }
 
@@ -946,12 +942,10 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
     static_assert(sizeof(HistRegion) <= sizeof(EncRegion), "one array for both");
     HistRegion* hist_regions = reinterpret_cast<HistRegion*>(plan);
 
-    if (cudaMemsetAsync(ws, 0, 1024, st) != cudaSuccess) return HGAP_ERR_CUDA;
-    if (cudaMemsetAsync(hists, 0, 1024 * (size_t)count, st) != cudaSuccess) return HGAP_ERR_CUDA;
+    if (cudaMemsetAsync(ws, 0, L.st_rec + 8 * (size_t)L.max_regions, st) != cudaSuccess) return HGAP_ERR_CUDA;
     benc_setup_kernel<<<scan_grid(count), kScanThreads, 0, st>>>(count, d_inputs, d_sizes, d_region_chunks, base_chunks(cfg), jobs,
                                                   item0s, hist_regions, nitems, L.max_regions, status);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
-    if (cudaMemsetAsync(st_rec, 0, 8 * (size_t)L.max_regions, st) != cudaSuccess) return HGAP_ERR_CUDA;
 
     HistStArgs h;
     std::memset(&h, 0, sizeof(h));
@@ -1017,7 +1011,7 @@ hgap_status hgap_batch_decompress(uint32_t count, const hgap_batch_entry* d_entr
     const uint32_t tile_segs = cfg->dec_tile_segs ? cfg->dec_tile_segs
                                : L.tiles_cap < 32 * (uint64_t)count ? kDecTileSmall
                                                                     : 0;
-    if (cudaMemsetAsync(ws, 0, 1024, st) != cudaSuccess) return HGAP_ERR_CUDA;
+    if (cudaMemsetAsync(ws, 0, L.records + 8 * (size_t)L.tiles_cap, st) != cudaSuccess) return HGAP_ERR_CUDA;
     bdec_table_kernel<<<table_grid(count), kTableThreads, 0, st>>>(count, d_entries, d_bits, d_gaps, d_outputs,
                                                                    tile_segs, cfg->dec_class_mask, wtables, cls, jobs,
                                                                    status);
@@ -1027,8 +1021,6 @@ hgap_status hgap_batch_decompress(uint32_t count, const hgap_batch_entry* d_entr
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
     bdec_map_kernel<<<book_grid(count), 32 * kBookWarps, 0, st>>>(count, jobs, cls, item0s, job_of, L.tiles_cap);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
-    if (cudaMemsetAsync(records, 0, 8 * (size_t)L.tiles_cap, st) != cudaSuccess) return HGAP_ERR_CUDA;
-
     DecTable unused;
     std::memset(&unused, 0, sizeof(unused));
     static const uint32_t kMinLen[4] = {4, 3, 2, 1};  // a representative shortest code per stage size
