@@ -70,7 +70,6 @@ hgap_status encode_layout(const void* d_in, uint64_t n, void* d_workspace, size_
     a->plan = reinterpret_cast<hgap::EncRegion*>(ws + w.plan);
     a->st_hist = reinterpret_cast<const uint32_t*>(ws + w.st_hist);
     h->single = J;
-    h->count = 1;
     h->nitems = nst;
     h->hist = reinterpret_cast<uint32_t*>(ws + w.scratch);
     h->st_hist = const_cast<uint32_t*>(a->st_hist);
@@ -255,7 +254,6 @@ hgap_status decode_impl(const uint32_t* d_bits, uint64_t words, const uint32_t* 
     J.item0 = 0;
     J.ntiles = hgap::decode_tiles(segments, min_len);
     if (J.ntiles >= 0xffffffffull) return HGAP_ERR_UNSUPPORTED;
-    a.count = 1;
     a.nitems = J.ntiles;
     const size_t need = kWsHeader + sizeof(uint64_t) * (size_t)J.ntiles;
     if (workspace_bytes < need) return HGAP_ERR_WORKSPACE;

@@ -949,9 +949,6 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
 
     HistStArgs h;
     std::memset(&h, 0, sizeof(h));
-    h.jobs = jobs;
-    h.item0s = item0s;
-    h.count = count;
     h.nitems_dev = nitems;
     h.hist = hists;
     h.st_hist = st_hist;
@@ -1035,7 +1032,6 @@ hgap_status hgap_batch_decompress(uint32_t count, const hgap_batch_entry* d_entr
         a.job_of = job_of + (uint64_t)c * L.tiles_cap;
         a.item0s = item0s + (uint64_t)c * (count + 1);
         a.tables = wtables;
-        a.count = count;
         a.nitems_dev = class_nitems + c;
         a.lookback = records;
         a.counter = counters + c;

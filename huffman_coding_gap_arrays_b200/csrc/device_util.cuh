@@ -137,18 +137,6 @@ __device__ __forceinline__ uint64_t wait_limit(const LookbackHook& h) {
     return h.wait_ns ? h.wait_ns : kWaitLimitNs;
 }
 
-// The job owning global work item `it`: the largest j with item0s[j] <= it
-// (item0s ascends, item0s[count] is the total; empty jobs are skipped).
-__device__ __forceinline__ uint32_t find_job(const uint64_t* item0s, uint32_t count, uint64_t it) {
-    uint32_t lo = 0, hi = count;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (item0s[mid] <= it) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
 __device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFull, v, d);

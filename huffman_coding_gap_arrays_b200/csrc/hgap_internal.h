@@ -35,8 +35,6 @@ constexpr uint64_t kFlagA = 1ull << 62;
 constexpr uint64_t kFlagP = 2ull << 62;
 constexpr uint64_t kFlagMask = 3ull << 62;
 constexpr uint64_t kValueMask = ~kFlagMask;
-// Hand-off record: valid bit over a 32-bit payload.
-constexpr uint64_t kHandValid = 1ull << 32;
 
 // Bounded-wait test hook, all zero in every product call: the work item
 // (encoder region / decoder tile, in the launch's numbering) plus one whose
@@ -200,10 +198,7 @@ struct alignas(16) HistRegion {
 static_assert(sizeof(HistRegion) == 32, "HistRegion: two 16-byte groups");
 
 struct HistStArgs {
-    EncJob single;
-    const EncJob* jobs;
-    const uint64_t* item0s;
-    uint32_t count;
+    EncJob single;              // the job, when regions == nullptr
     uint64_t nitems;
     const uint64_t* nitems_dev; // batched: the region count in device memory (overrides nitems)
     uint32_t* hist;             // [count][256] histograms (zeroed before the launch)
@@ -330,7 +325,6 @@ struct DecArgs {
     const uint64_t* item0s;     // batched: [count] first tile of each job in this launch's numbering
     const DecTableW* tables;    // batched: [count]
     DecIndex index;             // single path: the table's
-    uint32_t count;
     uint64_t nitems;            // tiles in this launch
     const uint64_t* nitems_dev; // batched: the tile count in device memory (overrides nitems)
     uint64_t* lookback;
