@@ -16,7 +16,8 @@
 //      lengths without a branch (DecIndex).  Position and output address
 //      advance in one addition: an entry holds the bits and the number of its
 //      symbols where the state has the position and the address.  The symbols
-//      go to the lane's row in shared memory, sized for the book's shortest code;
+//      go to the lane's row in shared memory, sized for the book's shortest code
+//      (of books with 1-bit codes as whole words, the lanes' rows interleaved);
 //   2. the warps publish their symbol counts at the barrier;
 //   3. the warp writes the PREVIOUS tile's symbols out of its image, with
 //      16-byte stores shifted to the output's alignment (bytes at both ends),
@@ -36,7 +37,8 @@
 //
 // The kernel is bound by shared-memory wavefronts (one lookup of 32 random
 // entries and one or two byte stores per step: 84 % of the pipe on Zipf(1.2))
-// and by instruction issue (72 %), not by HBM.  Measured (B200, 256 MiB, call
+// and by instruction issue (72 %), not by HBM: fewer wavefronts at three more
+// instructions a step measured slower (Last, below).  Measured (B200, 256 MiB, call
 // without the status read), against a kernel with four CTA barriers a tile, a
 // branch to a second table level and byte-wise compaction: Zipf(1.2) 524 -> 376
 // us, mixed 489 -> 393, BF16 mantissa 422 -> 363, BF16 exponents 324 -> 266,
@@ -82,7 +84,8 @@ struct DecCfg {
     static constexpr int kBySmem = (int)((227u * 1024u) / (kSmem + 1536u));
     static constexpr int kByRegs = (S == 1 ? 48 : 36) / (W + 1);
     static constexpr int kMinBlocks = kBySmem < 1 ? 1 : kBySmem < kByRegs ? kBySmem : kByRegs;
-    static_assert(kImgBytes % 16 == 0 && kRowsBytes % 16 == 0, "16-byte aligned areas");
+    static_assert(kImgBytes % 16 == 0, "16-byte aligned images");
+    static_assert((256 + 4 * kTab) % 128 == 0 && kRowsBytes % (128 * S) == 0, "rows on a multiple of 128");
 };
 
 // The decoder's table for one tile (DecIndex).
@@ -117,6 +120,28 @@ __device__ __forceinline__ void st_shared_u8(uint32_t addr, uint32_t v) {
     asm volatile("st.shared.u8 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+// Where a lane's symbols go.  One or two a step: bytes to a row of its own (`row`:
+// its shared address).  Up to three (MULTI): whole words, made in a register, word
+// k of lane l at 128 k + 4 l of the warp's rows (`row`: their address, a multiple
+// of 128), which meets no other lane's bank; a lane's unfinished last word stays
+// in the register.  Three byte stores of 32 drifting rows took 6 wavefronts and the
+// shifts between them, one word store takes one: 1024 buffers of 4 KiB - 4 MiB, the
+// 32-row class 150 -> 142 us.  With pairs the word form saves a quarter of the
+// kernel's wavefronts and still loses (Zipf(1.2) 256 MiB 363 -> 385 us): two byte
+// stores cost three instructions less, and there the kernel is short of those.
+struct Last {
+    uint32_t count, word;  // the lane's symbols, and (MULTI) the count % 4 last of them
+};
+// The last four symbols are in acc, the newest at the top; `at8` = 8 * (their
+// number) mod 32: the word that entry e's symbols go on with (what is past them: junk).
+__device__ __forceinline__ uint32_t row_word(uint32_t acc, uint32_t e, uint32_t at8) {
+    return __funnelshift_l(acc, e, at8);
+}
+
 // Decodes the codes that start in one 128-bit segment (not the stream's last
 // one), from bit `pos` (its gap offset), as four phases of 32 bits: phase k
 // decodes the codes starting in word k, from the window of words k and k+1,
@@ -124,25 +149,26 @@ __device__ __forceinline__ void st_shared_u8(uint32_t addr, uint32_t v) {
 // Codes of a pair / multi entry all start inside the segment in phases 0-2
 // (they fit the 11-bit window and phase 2 ends 32 bits before the segment
 // does); in phase 3 that holds while pos <= 21, and the last bits take only
-// the codes that start before bit 32 of the phase.  The symbols go to shared
-// address `row` on; their number is returned in `cnt`.  Returns the end bit of
-// the last code relative to phase 3 (32 + the next gap entry for a valid
+// the codes that start before bit 32 of the phase.  The symbols go to the lane's
+// row; their number is returned in `last`.  Returns the end bit of the last code relative to phase 3 (32 + the next gap entry for a valid
 // stream), or a value no stream yields after an invalid code.
 template <uint32_t P, bool WIDE, bool COMPLETE, bool PAIRS, bool MULTI>
 __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWords& w, uint32_t pos, uint32_t row,
-                                                   uint32_t& cnt) {
+                                                   uint32_t lane4, Last& last) {
     static_assert(!MULTI || COMPLETE, "multi entries: complete books");
     constexpr uint32_t kBad = 1u << 16;
     constexpr uint32_t kEarly = (WIDE ? (uint32_t)kDecPrefix : P) - 1;  // the last phase's fast loop ends this many bits early
     if (MULTI) {
-        uint32_t out = row;
+        uint32_t out = row >> 5, acc = 0;  // (row / 32 is a multiple of 4: out's low bits count the word's bytes)
+        auto put = [&](uint32_t e, uint32_t n) {
+            st_shared_u32(((out << 5) & ~127u) | lane4, row_word(acc, e, out << 3));
+            acc = __funnelshift_r(acc, e, 8 * n);
+            out += n;
+        };
         auto fast = [&](uint32_t cw, uint32_t nw) {
             while (!(pos & 32)) {
                 const uint32_t e = lookup<P, WIDE, true>(t, __funnelshift_l(nw, cw, pos));
-                st_shared_u8(out, e);
-                st_shared_u8(out + 1, e >> 8);
-                st_shared_u8(out + 2, e >> 16);
-                out += 1 + (e >> 29);
+                put(e, 1 + (e >> 29));
                 pos += (e >> 24) & 31u;
             }
         };
@@ -157,14 +183,12 @@ __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWord
         while (!(pos & 32)) {
             const uint32_t e = lookup<P, WIDE, true>(t, __funnelshift_l(w.w4, w.w3, pos));
             const uint32_t tot = (e >> 24) & 31u, more = e >> 29;
-            st_shared_u8(out, e);
-            st_shared_u8(out + 1, e >> 8);
-            st_shared_u8(out + 2, e >> 16);
             const bool all = pos + tot <= 32;  // every code of the entry ends, so starts, inside
-            out += all ? 1 + more : 1;
+            put(e, all ? 1 + more : 1);
             pos += all || !more ? tot : t.symlen[e & 0xffu];
         }
-        cnt = out - row;
+        last.count = out - (row >> 5);
+        last.word = row_word(acc, 0, out << 3);
         return pos;
     }
     uint32_t s = (row << 8) | pos;
@@ -204,7 +228,7 @@ __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWord
         return true;
     };
     const bool valid = run();
-    cnt = (s >> 8) - row;
+    last.count = (s >> 8) - row;
     return COMPLETE || valid ? s & 0xffu : kBad;
 }
 
@@ -212,21 +236,26 @@ __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWord
 // padding follows, which may not decode.  One code per step (the first code of
 // any pair or multi entry), the words picked by index.
 template <uint32_t P, bool WIDE, bool COMPLETE, bool MULTI>
-__device__ __forceinline__ uint32_t decode_last_segment(const Table& t, const SegWords& w, uint32_t pos, uint32_t end,
-                                                        uint32_t row) {
+__device__ __forceinline__ Last decode_last_segment(const Table& t, const SegWords& w, uint32_t pos, uint32_t end,
+                                                    uint32_t row, uint32_t lane4) {
     auto word = [&](uint32_t i) { return i == 0 ? w.w0 : i == 1 ? w.w1 : i == 2 ? w.w2 : i == 3 ? w.w3 : w.w4; };
-    uint32_t cnt = 0;
+    uint32_t cnt = 0, acc = 0;
     while (pos < end) {
         const uint32_t wi = pos >> 5;
         const uint32_t e = lookup<P, WIDE, MULTI>(t, __funnelshift_l(word(wi + 1), word(wi), pos));
         if (!COMPLETE && (e & kEntInvalidBit)) break;  // the padding after the final codeword
         const uint32_t more = MULTI ? e >> 29 : (e >> 24) - 1;
         const uint32_t len = MULTI ? (e >> 24) & 31u : (e >> 16) & 31u;
-        st_shared_u8(row + cnt, e);
+        if (MULTI) {
+            st_shared_u32((row + 32 * (cnt & ~3u)) | lane4, row_word(acc, e, 8 * cnt));
+            acc = __funnelshift_r(acc, e, 8);
+        } else {
+            st_shared_u8(row + cnt, e);
+        }
         ++cnt;
         pos += more ? t.symlen[e & 0xffu] : len;
     }
-    return cnt;
+    return {cnt, row_word(acc, 0, 8 * cnt)};
 }
 
 // A claimed tile, in shared memory: what the decoding warps need of it (clipped
@@ -255,10 +284,10 @@ template <int R, int W, int S, bool COMPLETE, bool PAIRS>
 __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kMinBlocks)
     decode_kernel(const __grid_constant__ DecArgs a, const __grid_constant__ DecTable tab) {
     using C = DecCfg<R, W, S>;
-    extern __shared__ __align__(16) unsigned char smem[];
+    extern __shared__ __align__(128) unsigned char smem[];
     uint8_t* const symlen = smem;                          // a symbol's code length, where it is at most kDecPrefix
     uint32_t* const t1 = reinterpret_cast<uint32_t*>(smem + 256);
-    unsigned char* const areas = smem + 256 + 4 * C::kTab; // per warp: rows, image
+    unsigned char* const areas = smem + 256 + 4 * C::kTab; // the warps' rows, then their images
     __shared__ DecSlot slot[4];                            // tile i in slot i % 4
     __shared__ uint32_t tot[2][W];                         // by tile parity: the warps' symbol counts,
     __shared__ uint8_t* dst[2];                            // the tile's place in the output,
@@ -397,9 +426,11 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
     }
 
     // ---- the decoding warps -------------------------------------------------------
-    unsigned char* const rows = areas + warp * C::kWarpBytes;
-    unsigned char* const img = rows + C::kRowsBytes;
-    uint32_t* const row32 = reinterpret_cast<uint32_t*>(rows + lane * C::kRowBytes);  // of the lane's first segment
+    unsigned char* const rows = areas + warp * C::kRowsBytes;
+    unsigned char* const img = areas + W * C::kRowsBytes + warp * C::kImgBytes;
+    // the lane's first word of its first segment, and the words from one of its words to the next
+    constexpr int kNext = MULTI ? 32 : 1;
+    uint32_t* const row32 = reinterpret_cast<uint32_t*>(rows + lane * (MULTI ? 4 : C::kRowBytes));
     const uint32_t u0 = warp * 32 * S + lane;  // the lane's segments in the tile: u0 + 32 k
 
     // A tile's words and gap entries, loaded a tile ahead: a segment's four words (one 16-byte load
@@ -438,10 +469,10 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
         const bool have = T.nseg != 0, prev = i != 0;
 
         // ---- 1. decode ---------------------------------------------------------------
-        uint32_t n[S];
+        uint32_t n[S], part[S];
 #pragma unroll
         for (int k = 0; k < S; ++k) {
-            n[k] = 0;
+            n[k] = part[k] = 0;
             if (!have) continue;  // uniform
             const Table t{t1, symlen, a.jobs ? a.tables[T.job_id].t2() : tab.t2, T.index.shift, T.index.offset};
             const uint32_t u = u0 + 32 * k;
@@ -455,14 +486,15 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
             const uint32_t gap = (pre_gap[k] >> (4 * (u & 7))) & 0xfu;  // where the next segment's first code starts
             const uint32_t before = __shfl_up_sync(kFull, gap, 1);
             const uint32_t pos = lane == 0 ? pre_gap0[k] >> 28 : before;
-            const uint32_t row = smem_addr(row32 + 32 * k * C::kRowWords);
+            const uint32_t row = smem_addr(row32 + 32 * k * C::kRowWords) - (MULTI ? 4 * lane : 0u);
+            Last last = {0, 0};
             // (every wide book's tile takes the second branch: uniform over the CTA)
             auto segment = [&](auto wide) {
                 constexpr bool WIDE = decltype(wide)::value;
                 if (T.last_bits && u + 1 == T.nseg) {
-                    n[k] = decode_last_segment<C::P, WIDE, COMPLETE, MULTI>(t, w, pos, T.last_bits, row);
+                    last = decode_last_segment<C::P, WIDE, COMPLETE, MULTI>(t, w, pos, T.last_bits, row, 4 * lane);
                 } else {
-                    const uint32_t end = decode_segment<C::P, WIDE, COMPLETE, PAIRS, MULTI>(t, w, pos, row, n[k]);
+                    const uint32_t end = decode_segment<C::P, WIDE, COMPLETE, PAIRS, MULTI>(t, w, pos, row, 4 * lane, last);
                     if (end != 32 + gap) atomicOr(a.status, kDevCorrupt);
                 }
             };
@@ -470,6 +502,8 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
                 if (COMPLETE && T.index.first_long != kDecWide) segment(std::integral_constant<bool, false>());
                 else segment(std::integral_constant<bool, true>());
             }
+            n[k] = last.count;
+            part[k] = last.word;
         }
         // both segments' counts in one scan (a warp's 32 have less than 2^13 symbols)
         uint32_t packed = n[0];
@@ -548,10 +582,10 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
                 full[k] = ((d & 3) + c) >> 2;
                 to[k] = reinterpret_cast<uint32_t*>(img) + (d >> 2);
                 // the row's word after the last whole one: what is past the count cleared
-                const uint32_t xl = r[whole] & ((1u << (8 * (c & 3))) - 1u);
-                r[whole] = xl;
+                const uint32_t xl = MULTI ? part[k] : r[whole] & ((1u << (8 * (c & 3))) - 1u);
+                r[kNext * whole] = xl;
                 // the lane's unfinished word
-                const uint32_t xk = whole ? r[whole - 1] : 0u;
+                const uint32_t xk = whole ? r[kNext * (whole - 1)] : 0u;
                 rest[k] = full[k] > whole ? __funnelshift_l(xl, 0u, sh) : (xl << sh) | __funnelshift_l(xk, 0u, sh);
                 // the words that no lane completes: the last lane's, and in the stream's last tile, whose
                 // last segment may have fewer symbols, any lane's
@@ -567,7 +601,7 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
 #pragma unroll
                 for (int j = 0; j <= R; ++j) {
                     if ((uint32_t)j >= most) break;  // uniform
-                    const uint32_t x = r[j];
+                    const uint32_t x = r[kNext * j];
                     if ((uint32_t)j < full[k]) to[k][j] = cur | (x << sh);
                     cur = __funnelshift_l(x, 0u, sh);
                 }
