@@ -38,12 +38,12 @@
 // The kernel is bound by shared-memory wavefronts (one lookup of 32 random
 // entries and one or two byte stores per step: 84 % of the pipe on Zipf(1.2))
 // and by instruction issue (72 %), not by HBM: fewer wavefronts at three more
-// instructions a step measured slower (Last, below).  Measured (B200, 256 MiB, call
-// without the status read), against a kernel with four CTA barriers a tile, a
+// instructions a step measured slower (Last, below).  Measured (B200, 256 MiB,
+// call without the status read), against a kernel with four CTA barriers a tile, a
 // branch to a second table level and byte-wise compaction: Zipf(1.2) 524 -> 376
 // us, mixed 489 -> 393, BF16 mantissa 422 -> 363, BF16 exponents 324 -> 266,
 // clamped Gaussians of sigma 1 / 3 431 -> 306 / 321 -> 261; 1024 buffers of
-// 4 KiB - 4 MiB (593 MB) 1047 -> 851 us.  Of that the branch-free table gives
+// 4 KiB - 4 MiB (593 MB) 1047 -> 785 us.  Of that the branch-free table gives
 // Zipf(1.2) 439 -> 401 us and the batch 896 -> 858.
 #include <cuda_runtime.h>
 
@@ -147,11 +147,12 @@ __device__ __forceinline__ uint32_t row_word(uint32_t acc, uint32_t e, uint32_t 
 // decodes the codes starting in word k, from the window of words k and k+1,
 // so the loop tests only bit 5 of the position -- no word refill, no end test.
 // Codes of a pair / multi entry all start inside the segment in phases 0-2
-// (they fit the 11-bit window and phase 2 ends 32 bits before the segment
-// does); in phase 3 that holds while pos <= 21, and the last bits take only
+// (they fit the window of P bits and phase 2 ends 32 bits before the segment
+// does); in phase 3 that holds while pos <= 32 - P, and the last bits take only
 // the codes that start before bit 32 of the phase.  The symbols go to the lane's
-// row; their number is returned in `last`.  Returns the end bit of the last code relative to phase 3 (32 + the next gap entry for a valid
-// stream), or a value no stream yields after an invalid code.
+// row; their number is returned in `last`.  Returns the end bit of the last code
+// relative to phase 3 (32 + the next gap entry for a valid stream), or a value no
+// stream yields after an invalid code.
 template <uint32_t P, bool WIDE, bool COMPLETE, bool PAIRS, bool MULTI>
 __device__ __forceinline__ uint32_t decode_segment(const Table& t, const SegWords& w, uint32_t pos, uint32_t row,
                                                    uint32_t lane4, Last& last) {

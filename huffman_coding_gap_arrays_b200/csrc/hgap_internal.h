@@ -60,19 +60,20 @@ constexpr uint32_t kEncAbsent = 0x80000000u;
 // The encoder works on super-tiles: `st_chunks` chunks of kEncChunkBytes input
 // bytes each.  The histogram pass that precedes it also records one 256-bin
 // histogram per super-tile, so a super-tile's bit count -- and, after one
-// look-back over super-tiles, its first output bit -- is known before any of
+// look-back (enc_plan_kernel), its first output bit -- is known before any of
 // its bytes are encoded.  st_chunks depends on n only (hgap_internal
 // encode_st_chunks), so both passes and the workspace query agree.
 constexpr int kEncChunkBytes = 8192;
 constexpr int kEncMaxStChunks = 32;
 // The super-tile size minimises the encoder's modelled makespan: persistent CTAs
 // (2 per SM, 296 on a 148-SM B200) take equal super-tiles of c chunks in waves,
-// each costing c chunks plus about one chunk's worth of fixed work (look-back,
-// the head word rebuilt backwards, the ring crossing into the next super-tile).
-// Measured on C1 (16 MiB, 2048 chunks): 1-chunk super-tiles (7 waves) 0.070 ms,
-// 2 chunks 0.055, 4 chunks 0.047, 7 chunks (one wave) 0.041 ms.  The count is
-// kept under encode_super_tiles_cap, so a workspace sized for n bytes serves
-// every smaller input.
+// each costing c chunks plus about one chunk's worth of fixed work (a last step
+// partly empty, its gap words, two more barriers).  Measured on 16 MiB (2048
+// chunks), encoder and histogram pass: 1-chunk super-tiles (7 waves) 0.070 ms, 2
+// chunks 0.055, 4 chunks 0.047, 7 chunks (one wave) 0.041 ms; with the regions
+// planned by a kernel of their own, sizes of 4 to 24 chunks still found none
+// better.  The count is kept under encode_super_tiles_cap, so a workspace sized
+// for n bytes serves every smaller input.
 constexpr uint64_t kEncCtas = 296;
 constexpr uint64_t kEncStOverhead = 1;  // chunks
 

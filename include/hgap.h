@@ -189,8 +189,9 @@ hgap_status hgap_status_from_word(uint32_t word);
  * No counterpart in the reference, whose look-back spins never give up
  * (encoder/src/encoder.cu:239-241, decoder/src/decoder.cu:615-632).  For
  * testing the bounded waits only: hgap_encode / hgap_decode, except that one
- * work item, `hold` (encoder: region, decoder: tile, numbered from 0 in stream
- * order), never publishes its look-back records, and every look-back wait
+ * work item, `hold` (encoder: region, whose look-back goes in groups of eight;
+ * decoder: tile; numbered from 0 in stream order), never publishes its look-back
+ * records (the region's group does not), and every look-back wait
  * gives up after `wait_limit_ns` (0: the default of 0.5 s).  The items after
  * it wait for the withheld record until the limit, the kernel then finishes
  * with HGAP_ERR_TIMEOUT in the workspace status, and the output is void.
