@@ -33,7 +33,7 @@ DECOMPRESS_KERNELS = 8
 @dataclass
 class LaunchConfig:
     """Launch shape of the batched kernels; no choice changes the output."""
-    region_chunks: int = 8      # encoder region = region_chunks x 8 KiB (1..32)
+    region_chunks: int = 8      # encoder region = region_chunks x 8 KiB (1..32; 0 = by the batch's size)
     hist_ctas_per_sm: int = 0   # persistent grids: CTAs per SM (0 = occupancy maximum)
     enc_ctas_per_sm: int = 0
     dec_ctas_per_sm: int = 0
@@ -74,13 +74,14 @@ def _upload(values, dtype, out: torch.Tensor | None = None, device=None) -> torc
 
 
 class BatchCodec:
-    """Workspaces, arenas and pointer tables for a fixed list of buffer sizes."""
+    """Workspaces, arenas and pointer tables for a fixed list of buffer sizes.
+    Without a config the encoder's regions are sized by the batch (region_chunks 0)."""
 
     def __init__(self, sizes, config: LaunchConfig | None = None, device=None,
                  region_chunks: np.ndarray | None = None, decompress: bool = True, inputs=None, outputs=None):
         self.sizes = np.ascontiguousarray(np.asarray(sizes, dtype=np.uint64))
         self.count = int(self.sizes.size)
-        self.config = config or LaunchConfig()
+        self.config = config or LaunchConfig(region_chunks=0)
         self.device = torch.device(device) if device is not None else torch.device("cuda")
         L = lib()
         cfg = self.config.cstruct()

@@ -794,6 +794,19 @@ uint32_t base_chunks(const hgap_batch_config* cfg) {
     return rc > 32 ? 32 : rc;
 }
 
+// The region size when the caller names none: 8 chunks, and larger ones where the
+// batch still gives every encoder CTA (296) many of them, since each region costs
+// its histogram fold, its plan and a last step that is partly empty.  The host
+// knows the sizes only as what the workspace holds, counted in 8-chunk regions.
+// Compress in us at 8 / 16 / 32 chunks, by regions of 8 chunks: 4 KiB - 4 MiB
+// buffers, 4725 regions 390 / 396 / 431, 9644: 717 / 693 / 723, 19678: 1383 /
+// 1321 / 1329, 39879: 2734 / 2591 / 2558; buffers of 1 MiB, 4352: 358 / 344 /
+// 351, 17408: 1209 / 1146 / 1130; of 256 KiB, 2560: 212 / 210 / 223, 10240: 653 /
+// 619 / 618.  (12 and 24 chunks lie between or above.)
+uint32_t default_chunks(uint64_t regions) {
+    return regions >= 80 * kEncCtas ? 32 : regions >= 20 * kEncCtas ? 16 : 8;
+}
+
 // Compress workspace: [header 1024: status @0, counter @4, nitems @64] [hists]
 // [st_rec] (zero at the start of a call, together: one memset) [jobs] [item0s]
 // [tables] [plan] [st_hist], the per-region arrays (st_rec, plan, st_hist) for
@@ -942,9 +955,11 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
     static_assert(sizeof(HistRegion) <= sizeof(EncRegion), "one array for both");
     HistRegion* hist_regions = reinterpret_cast<HistRegion*>(plan);
 
+    // (per-buffer sizes are the caller's choice too)
+    const uint32_t chunks = cfg->region_chunks || d_region_chunks ? base_chunks(cfg) : default_chunks(L.max_regions);
     if (cudaMemsetAsync(ws, 0, L.st_rec + 8 * (size_t)L.max_regions, st) != cudaSuccess) return HGAP_ERR_CUDA;
-    benc_setup_kernel<<<scan_grid(count), kScanThreads, 0, st>>>(count, d_inputs, d_sizes, d_region_chunks, base_chunks(cfg), jobs,
-                                                  item0s, hist_regions, nitems, L.max_regions, status);
+    benc_setup_kernel<<<scan_grid(count), kScanThreads, 0, st>>>(count, d_inputs, d_sizes, d_region_chunks, chunks, jobs,
+                                                                 item0s, hist_regions, nitems, L.max_regions, status);
     if (cudaGetLastError() != cudaSuccess) return HGAP_ERR_CUDA;
 
     HistStArgs h;
