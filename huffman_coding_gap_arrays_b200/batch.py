@@ -37,7 +37,7 @@ class LaunchConfig:
     hist_ctas_per_sm: int = 0   # persistent grids: CTAs per SM (0 = occupancy maximum)
     enc_ctas_per_sm: int = 0
     dec_ctas_per_sm: int = 0
-    dec_tile_segs: int = 0      # decoder tile: 256 or 512 segments (0 = 512; always 256 for books with a 1-bit code)
+    dec_tile_segs: int = 0      # decoder tile: 256 or 512 segments (0 = by the batch; hgap.h)
     dec_class_mask: int = 0     # decoder classes to launch (0 = all 8; see decoder_class_mask)
 
     def cstruct(self) -> BatchConfig:

@@ -1022,7 +1022,7 @@ hgap_status hgap_batch_decompress(uint32_t count, const hgap_batch_entry* d_entr
     // (the workspace's room tells the buffers' average size: a tile for every 2048 bytes)
     const uint32_t tile_segs = cfg->dec_tile_segs ? cfg->dec_tile_segs
                                : L.tiles_cap < 32 * (uint64_t)count ? kDecTileSmall
-                                                                    : 0;
+                                                                    : kDecTileBatch;
     if (cudaMemsetAsync(ws, 0, L.records + 8 * (size_t)L.tiles_cap, st) != cudaSuccess) return HGAP_ERR_CUDA;
     bdec_table_kernel<<<table_grid(count), kTableThreads, 0, st>>>(count, d_entries, d_bits, d_gaps, d_outputs,
                                                                    tile_segs, cfg->dec_class_mask, wtables, cls, jobs,

@@ -5,9 +5,9 @@
 // segment is decoded ONCE (the reference decodes it twice: a counting pass,
 // then a writing pass, decoder.cu:529-569,672-725).
 //
-// A persistent CTA of W decoding warps (8 or 16) and one more warp takes tiles
-// of 32 W consecutive segments of one stream.  A decoding warp owns 32 of
-// them, one per lane, and everything that is large is its own (no other warp
+// A persistent CTA of W decoding warps (8, 15 or 16) and one more warp takes tiles
+// of 32 W S consecutive segments of one stream.  A decoding warp owns 32 S
+// of them, S per lane, and everything that is large is its own (no other warp
 // reads or writes it), so a tile costs the CTA one barrier:
 //   1. decode: a lane has its segment's words in registers (loaded a tile
 //      ahead: one 16-byte load, the next segment's first word from the
@@ -642,11 +642,16 @@ static int launch_decode_r(const DecArgs& a, const DecTable& t, int ctas_per_sm,
 
 template <int R, bool COMPLETE, bool PAIRS>
 static int launch_decode_s(const DecArgs& a, const DecTable& t, int k, uint32_t tile_segs, cudaStream_t st) {
-    if (dec_tile_segs_for(R, tile_segs) == 512) {
-        if (R >= 16) return launch_decode_r<R, (R >= 32 ? 8 : 16), 1, COMPLETE, PAIRS>(a, t, k, st);
-        return launch_decode_r<R, 8, (R >= 16 ? 1 : 2), COMPLETE, PAIRS>(a, t, k, st);
+    const int segs = dec_tile_segs_for(R, tile_segs);
+    if (segs == 256) return launch_decode_r<R, 8, 1, COMPLETE, PAIRS>(a, t, k, st);
+    if (segs == 480) {
+        // a batch's complete books (it decodes the incomplete ones with 32 rows)
+        if constexpr (R == 16 && COMPLETE && PAIRS) return launch_decode_r<16, 15, 1, true, true>(a, t, k, st);
+        return cudaErrorInvalidValue;
     }
-    return launch_decode_r<R, 8, 1, COMPLETE, PAIRS>(a, t, k, st);
+    constexpr int W = R == 16 ? 16 : 8, S = R >= 16 ? 1 : 2;
+    static_assert(DecCfg<R, W, S>::kSegs == dec_tile_segs(R), "the tile's shape");
+    return launch_decode_r<R, W, S, COMPLETE, PAIRS>(a, t, k, st);
 }
 
 template <bool COMPLETE, bool PAIRS>

@@ -222,20 +222,28 @@ HGAP_HD constexpr int dec_stage_rows(uint32_t min_len) {
 }
 // Segments per decoder tile for a stage of R rows: 512, for which the tile's
 // fixed work (claim, look-back, barrier) counts least (256 MiB at 256 -> 512
-// segments: Zipf(1.2), R = 16, 401 -> 376 us; mixed, R = 11, 546 -> 428; BF16
-// mantissa, R = 8, 576 -> 385); 256 for 32 rows, whose 512-segment tile would
-// leave one CTA per SM.
+// segments: mixed, R = 11, 546 -> 428 us; BF16 mantissa, R = 8, 576 -> 385); 256
+// for 32 rows, whose 512-segment tile would leave one CTA per SM.
 HGAP_HD constexpr int dec_tile_segs(int R) { return R >= 32 ? 256 : 512; }
 // The same with a launch-shape override of 256 or 512 segments (0: the
-// default; 32 rows keep 256), or kDecTileSmall for a batch of small buffers,
-// whose last tiles are mostly empty: 256 for 16 rows (4096 buffers of 4-64 KiB:
-// that class 81 -> 67 us; 11 rows 58 -> 61 and 8 rows 12.7 -> 11.7, left alone).
-constexpr uint32_t kDecTileSmall = 1;
+// default; 32 rows keep 256), or what a batch takes for 16 rows by itself:
+//   kDecTileBatch  480: 15 warps of one segment a lane and the extra one, three
+//   kDecTileBatch  480: 15 warps of one segment a lane and the extra one, three
+//     CTAs and 48 warps an SM where 512 leaves two and 34 (batches of 10 to 80 MB
+//     within 2 %, 291 MB 420 -> 413 us, 593 MB 766 -> 754, 256 buffers of 1 MiB of
+//     Zipf(1.2) 410 -> 394).  Not for the single-buffer calls, whose every CTA
+//     makes its own table: 256 MiB take the same time, 16 MiB 71 -> 79 us a call.
+//     (8 and 11 rows are better off with two segments a lane: mixed 256 MiB
+//     400 us, with 15 warps of one 444.)
+//   kDecTileSmall  256, for small buffers, whose last tiles are mostly empty (4096
+//     buffers of 4-64 KiB: that class 81 -> 67 us with 512 -> 256; 11 rows 58 -> 61
+//     and 8 rows 12.7 -> 11.7, left alone).
+constexpr uint32_t kDecTileBatch = ~0u, kDecTileSmall = ~1u;
 HGAP_HD constexpr int dec_tile_segs_for(int R, uint32_t override_segs) {
-    return override_segs == kDecTileSmall && R == 16                 ? 256
-           : R >= 32                                                 ? 256
-           : (override_segs == 256 || override_segs == 512)          ? (int)override_segs
-                                                                     : dec_tile_segs(R);
+    if (R >= 32) return 256;
+    if (override_segs == kDecTileBatch) return R == 16 ? 480 : dec_tile_segs(R);
+    if (override_segs == kDecTileSmall) return R == 16 ? 256 : dec_tile_segs(R);
+    return override_segs == 256 ? 256 : dec_tile_segs(R);
 }
 constexpr int kDecT2Cap = 2560;  // >= the largest complete 16-bit book (see host.cpp)
 constexpr uint16_t kDecInvalid = 0x4000;

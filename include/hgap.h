@@ -280,9 +280,9 @@ typedef struct hgap_batch_config {
     uint32_t hist_ctas_per_sm; /* persistent grids, CTAs per SM (0 = occupancy maximum) */
     uint32_t enc_ctas_per_sm;
     uint32_t dec_ctas_per_sm;
-    uint32_t dec_tile_segs;    /* decoder tile, 256 or 512 segments (0 = 512, or for books whose
-                                  shortest code has 2 bits 256 in a batch whose buffers average
-                                  under 64 KiB); books with a 1-bit code always take 256 */
+    uint32_t dec_tile_segs;    /* decoder tile, 256 or 512 segments; 0 = 512, but for books whose
+                                  shortest code has 2 bits 480, and 256 in a batch whose buffers
+                                  average under 64 KiB; books with a 1-bit code always take 256 */
     uint32_t dec_class_mask;   /* decoder classes hgap_batch_decompress launches: bit k as
                                   hgap_batch_decoder_class numbers them; 0 = all 8.  For callers
                                   that know their books on the host: an empty class then costs
