@@ -228,7 +228,6 @@ HGAP_HD constexpr int dec_tile_segs(int R) { return R >= 32 ? 256 : 512; }
 // The same with a launch-shape override of 256 or 512 segments (0: the
 // default; 32 rows keep 256), or what a batch takes for 16 rows by itself:
 //   kDecTileBatch  480: 15 warps of one segment a lane and the extra one, three
-//   kDecTileBatch  480: 15 warps of one segment a lane and the extra one, three
 //     CTAs and 48 warps an SM where 512 leaves two and 34 (batches of 10 to 80 MB
 //     within 2 %, 291 MB 420 -> 413 us, 593 MB 766 -> 754, 256 buffers of 1 MiB of
 //     Zipf(1.2) 410 -> 394).  Not for the single-buffer calls, whose every CTA
