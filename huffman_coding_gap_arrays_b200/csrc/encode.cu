@@ -595,7 +595,8 @@ __global__ void __launch_bounds__(kEncThreads, 2)
                     const uint32_t j0 = pa >> 5;
                     uint32_t j1 = ends ? (pz + 31) >> 5 : pz >> 5;
                     if (edge) {
-                        if (lane == 0 && off < R.lo) img[j0] &= ~0u >> (pa & 31);
+                        // (the job starts in the first half: the second one's first word holds the first's last bits)
+                        if (lane == 0 && !half && off < R.lo) img[j0] &= ~0u >> (pa & 31);
                         if (lane == 31 && ends && (pz & 31)) img[pz >> 5] &= ~(~0u >> (pz & 31));
                         __syncwarp();
                     }
