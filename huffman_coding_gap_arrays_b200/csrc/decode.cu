@@ -60,6 +60,8 @@ namespace hgap {
 // each of them more than the round trips it saves (Zipf(1.2) 256 MiB at 32 / 64 /
 // 128 records: 443 / 453 / 479 us, BF16 mantissa 371 / 378 / 392).
 constexpr int kDecLookK = 1;
+// In place of a warp's symbol count: one of its waits gave up.
+constexpr uint32_t kGaveUp = ~0u;
 
 // R: stage rows of 4 symbols per segment (at most 4R symbols per segment); W: decoding warps;
 // S: segments per lane of a tile.
@@ -388,14 +390,17 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
     }
     __syncthreads();
     if (slot[0].nseg == 0) return;
-    // Waits between the warps of the CTA: each side's work between them is itself bounded.
-    auto wait = [&](uint64_t* bar, uint32_t i) { return mbar_wait(&bar[i & 1], (i >> 1) & 1, a.status, false); };
+    // Waits between the warps of the CTA: false for a lane that gave up (so did a look-back
+    // somewhere, or this took longer than any look-back should).
+    auto wait = [&](uint64_t* bar, uint32_t i) {
+        return mbar_wait(&bar[i & 1], (i >> 1) & 1, a.status, true, kCtaWaitLimitNs);
+    };
 
     if (warp == W) {
         // ---- the extra warp -------------------------------------------------------
         // (the second tile is claimed only now, when the other CTAs have their first: a CTA that
         // held two consecutive tiles would keep all later ones waiting for its second)
-        uint32_t claim = 0;
+        uint32_t claim = 0, copies = a.jobs ? 1 : 0;  // table copies issued
         if (lane == 0) {
             fill_slot(1, atomicAdd(a.counter, 1u));
             mbar_arrive(&filled[1]);
@@ -404,11 +409,16 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
         for (uint32_t i = 0; slot[i & 3].nseg != 0; ++i) {
             const DecSlot& T = slot[i & 3];
             const DecSlot& N = slot[(i + 1) & 3];
-            if (!wait(published, i)) break;  // tile i is decoded: the table is free
-            const uint32_t Ct = __reduce_add_sync(kFull, lane < (uint32_t)W ? tot[i & 1][lane] : 0u);
+            if (!__all_sync(kFull, wait(published, i))) break;  // tile i is decoded: the table is free
+            const uint32_t t = lane < (uint32_t)W ? tot[i & 1][lane] : 0u;
+            if (__any_sync(kFull, t == kGaveUp)) break;
+            const uint32_t Ct = __reduce_add_sync(kFull, t);
             if (lane == 0 && N.nseg) {
                 claim = atomicAdd(a.counter, 1u);  // (its answer is needed only after the look-back)
-                if (a.jobs && N.job_id != T.job_id) copy_table(N);
+                if (a.jobs && N.job_id != T.job_id) {
+                    copy_table(N);
+                    ++copies;
+                }
             }
             const uint64_t O = lookback_resolve<kDecLookK>(a.lookback, T.rec, Ct, T.first, a.status, lane,
                                                            wait_limit(a.hook), T.rec + 1 != a.hook.hold_plus1);
@@ -423,6 +433,8 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
             }
             __syncwarp();
         }
+        // never leave the CTA with a copy still in flight into its shared memory
+        if (lane == 0 && copies) mbar_wait(&tbar, (copies - 1) & 1, a.status, false);
         return;
     }
 
@@ -460,9 +472,18 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
         }
     };
     prefetch(slot[0]);
-    // (a wait that gives up leaves no table to decode with: nothing is decoded from then on)
-    uint32_t copies = a.jobs ? 1 : 0;  // table copies so far
-    bool alive = !copies || mbar_wait(&tbar, 0, a.status, false);
+    uint32_t copies = 0;  // table copies waited for
+    auto table_landed = [&] {
+        return __all_sync(kFull, mbar_wait(&tbar, copies++ & 1, a.status, true, kCtaWaitLimitNs));
+    };
+    // A warp whose wait gave up may not go alone: the others' barrier of the next tile, number i,
+    // counts all W.  It says so there, and all leave after that barrier, the extra warp with them.
+    auto give_up = [&](uint32_t i) {
+        if (lane == 0) tot[i & 1][warp] = kGaveUp;
+        named_barrier(1, 32 * W);
+        if (tid == 0) mbar_arrive(&published[i & 1]);
+    };
+    if (a.jobs && !table_landed()) return give_up(0);
 
     uint32_t prev_m = 0, prev_before = 0;  // the warp's symbols of the tile before, and those before them in it
     for (uint32_t i = 0;; ++i) {
@@ -499,7 +520,7 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
                     if (end != 32 + gap) atomicOr(a.status, kDevCorrupt);
                 }
             };
-            if (u < T.nseg && alive) {
+            if (u < T.nseg) {
                 if (COMPLETE && T.index.first_long != kDecWide) segment(std::integral_constant<bool, false>());
                 else segment(std::integral_constant<bool, true>());
             }
@@ -513,11 +534,12 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
         const uint32_t sums = __shfl_sync(kFull, incl, 31);
         const uint32_t sum0 = S > 1 ? sums & 0xffffu : sums, m = S > 1 ? sum0 + (sums >> 16) : sums;  // the warp's symbols
         uint32_t before = 0;
-        bool reload = false;
+        bool reload = false, together = true, ok = true;  // together: no warp gave up before this tile's barrier
         if (have) {
             if (lane == 0) tot[i & 1][warp] = m;
             named_barrier(1, 32 * W);  // the counts are in place, the table is free
             const uint32_t t = lane < (uint32_t)W ? tot[i & 1][lane] : 0u;
+            together = t != kGaveUp;
             before = __reduce_add_sync(kFull, lane < warp ? t : 0u);
             if (warp == 0) {
                 // the aggregate first: nothing that this CTA waits for may hold it back
@@ -528,14 +550,22 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
                 }
             }
             const DecSlot& N = slot[(i + 1) & 3];
-            if (!wait(filled, i + 1)) break;
-            reload = a.jobs && N.nseg && N.job_id != T.job_id;
-            prefetch(N);
+            ok = wait(filled, i + 1);
+            if (ok) {
+                reload = a.jobs && N.nseg && N.job_id != T.job_id;
+                prefetch(N);
+            }
+        } else {
+            named_barrier_arrive(1, 32 * W);  // for a warp that gave up and knows of no end
+        }
+        if (prev) ok = wait(placed, i - 1) && ok;
+        if (!__all_sync(kFull, ok && together)) {
+            if (have && __all_sync(kFull, together)) give_up(i + 1);
+            break;
         }
 
         // ---- 2. write out the tile before -----------------------------------------------
         if (prev) {
-            if (!wait(placed, i - 1)) break;
             uint8_t* const out = dst[(i & 1) ^ 1] + prev_before;
             const uint32_t left = room[(i & 1) ^ 1];
             uint32_t m = left > prev_before ? left - prev_before : 0u;
@@ -613,10 +643,7 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
                 if (n[k]) atomicOr(to[k] + full[k], rest[k]);
             __syncwarp();
         }
-        if (reload) {
-            alive = mbar_wait(&tbar, copies & 1, a.status, false) && alive;
-            ++copies;
-        }
+        if (reload && !table_landed()) return give_up(i + 1);
     }
 }
 

@@ -12,6 +12,9 @@ namespace hgap {
 constexpr unsigned kFull = 0xffffffffu;
 // A wait gives up after this long (ns of %globaltimer) and flags kDevTimeout.
 constexpr uint64_t kWaitLimitNs = 500ull * 1000 * 1000;
+// The same for a warp that waits for another one's look-back: that has kWaitLimitNs for
+// every record that is late, so it may rightly take longer than one of them.
+constexpr uint64_t kCtaWaitLimitNs = 20 * kWaitLimitNs;
 
 __device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
     uint4 v;
@@ -94,6 +97,11 @@ __device__ __forceinline__ void named_barrier(uint32_t id, uint32_t threads) {
     asm volatile("barrier.sync.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Counts towards that barrier without waiting for it.
+__device__ __forceinline__ void named_barrier_arrive(uint32_t id, uint32_t threads) {
+    asm volatile("barrier.arrive.aligned %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 __device__ __forceinline__ void bulk_load(void* dst_smem, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
                  ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
@@ -117,15 +125,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // Waits for the phase of `bar` with the given parity to complete.  Bounded:
-// after kWaitLimitNs it flags kDevTimeout and returns false; with `bail`, it
-// also gives up as soon as a timeout is already flagged (the kernel's output
-// is void then, and it only has to finish).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* status, bool bail) {
+// after limit_ns it flags kDevTimeout and returns false; with `bail`, a wait
+// of more than kBailNs also gives up as soon as a timeout is already flagged
+// (the kernel's output is void then, and it only has to finish).  The lanes of
+// a warp give up each on its own clock.
+constexpr uint64_t kBailNs = 200000;
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* status, bool bail,
+                                          uint64_t limit_ns = kWaitLimitNs) {
     if (mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = global_timer_ns();
     for (;;) {
         if (mbar_try_wait(bar, parity)) return true;
-        if (global_timer_ns() - t0 > kWaitLimitNs || (bail && (ld_relaxed_u32(status) & kDevTimeout))) {
+        const uint64_t waited = global_timer_ns() - t0;
+        if (waited > limit_ns || (bail && waited > kBailNs && (ld_relaxed_u32(status) & kDevTimeout))) {
             atomicOr(status, kDevTimeout);
             return false;
         }
