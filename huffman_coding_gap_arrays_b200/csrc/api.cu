@@ -65,6 +65,7 @@ hgap_status encode_layout(const void* d_in, uint64_t n, void* d_workspace, size_
     a->status = reinterpret_cast<uint32_t*>(ws);
     a->counter = reinterpret_cast<uint32_t*>(ws) + 1;
     a->nitems_dev = reinterpret_cast<uint64_t*>(ws + 8);
+    a->plan_counter = reinterpret_cast<uint32_t*>(ws + 16);
     a->tag = reinterpret_cast<const uint64_t*>(ws + w.tag);
     a->st_rec = reinterpret_cast<uint64_t*>(ws + w.st_rec);
     a->plan = reinterpret_cast<hgap::EncRegion*>(ws + w.plan);

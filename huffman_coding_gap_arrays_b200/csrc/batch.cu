@@ -807,7 +807,7 @@ uint32_t default_chunks(uint64_t regions) {
     return regions >= 80 * kEncCtas ? 32 : regions >= 20 * kEncCtas ? 16 : 8;
 }
 
-// Compress workspace: [header 1024: status @0, counter @4, nitems @64] [hists]
+// Compress workspace: [header 1024: status @0, counters @4 (three), nitems @64] [hists]
 // [st_rec] (zero at the start of a call, together: one memset) [jobs] [item0s]
 // [tables] [plan] [st_hist], the per-region arrays (st_rec, plan, st_hist) for
 // as many regions as the workspace holds.
@@ -991,6 +991,7 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
     a.st_rec = st_rec;
     a.st_hist = st_hist;
     a.counter = status + 1;
+    a.plan_counter = status + 3;
     a.status = status;
     EncTable unused;
     std::memset(&unused, 0, sizeof(unused));

@@ -124,8 +124,9 @@ constexpr int kPlanLookK = 1;
 // CTA's eight regions first, and the look-back runs over these groups (over
 // single regions it took 13 us for the 1171 regions of 256 MiB, here 8): a
 // group in which a job starts publishes the sum from there on as an inclusive
-// prefix.  Groups of one CTA ascend, so a look-back only ever waits for CTAs
-// that are running.
+// prefix.  Groups are claimed in order, and the next one only when the current
+// one's sum is published: a look-back only ever waits for CTAs that run, however
+// many of the grid's CTAs the GPU has room for beside other work.
 // All the regions' dependent loads overlap here, where one warp of a persistent
 // encoder CTA went through them between two regions: encoder and plan of 1024
 // buffers in 64 KiB regions 659 -> 543 us, of 4096 small buffers 170 -> 126, of
@@ -150,9 +151,11 @@ __global__ void __launch_bounds__(kPlanThreads) enc_plan_kernel(const __grid_con
         if (!fits) return;
     }
     __shared__ uint64_t s_agg[kPlanWarps], s_excl;
-    __shared__ uint32_t s_first[kPlanWarps];
+    __shared__ uint32_t s_first[kPlanWarps], s_next;
     const uint32_t warp = tid >> 5;
-    for (uint64_t g = blockIdx.x; g * kPlanWarps < nitems; g += gridDim.x) {
+    if (tid == 0) s_next = atomicAdd(a.plan_counter, 1u);
+    __syncthreads();
+    for (uint64_t g = s_next; g * kPlanWarps < nitems; g = s_next) {
         const uint64_t item = g * kPlanWarps + warp;
         const bool valid = item < nitems;  // uniform over the warp
         uint32_t job = 0;
@@ -194,9 +197,14 @@ __global__ void __launch_bounds__(kPlanThreads) enc_plan_kernel(const __grid_con
             const uint32_t from = starts ? 31 - __clz(starts) : 0u;
             const uint64_t sum = warp_sum_u64(lane >= from ? mine : 0);
             if (lane == 0 && !held) lookback_publish(a.st_rec, g, sum, starts != 0);
+            uint32_t claim = 0;
+            if (lane == 0) claim = atomicAdd(a.plan_counter, 1u);
             const uint64_t e = lookback_resolve<kPlanLookK>(a.st_rec, g, sum, (starts & 1u) != 0, a.status, lane,
                                                             wait_limit(a.hook), !held && starts == 0);
-            if (lane == 0) s_excl = e;
+            if (lane == 0) {
+                s_excl = e;
+                s_next = claim;
+            }
         }
         // the job's bits before this region: in the group, and before it unless the job starts in it
         const uint32_t upto = starts & ((2u << warp) - 1u);

@@ -78,7 +78,8 @@ constexpr uint64_t kEncCtas = 296;
 constexpr uint64_t kEncStOverhead = 1;  // chunks
 
 // Encoder workspace for nst super-tiles:
-//   [status u32][counter u32][super-tiles to encode u64][st_rec u64 x nst]  cleared by every call
+//   [status u32][counter u32][super-tiles to encode u64][plan counter u32, 12 bytes of padding]
+//   [st_rec u64 x nst]                                                      cleared by every call
 //   [tag: n u64, input u64][scratch histogram u32 x 256]                    and these by the histogram pass
 //   [plan EncRegion x nst][st_hist u32 x 256 x nst]
 struct EncWorkspace {
@@ -163,7 +164,7 @@ constexpr uint32_t kRegionVec = 4u;    // output words are 16-byte aligned
 
 inline EncWorkspace encode_workspace(uint64_t nst) {
     EncWorkspace w;
-    w.st_rec = 16;
+    w.st_rec = 32;
     w.tag = (w.st_rec + 8 * (size_t)nst + 15) & ~(size_t)15;
     w.scratch = w.tag + 16;
     w.plan = w.scratch + 1024;
@@ -184,7 +185,8 @@ struct EncArgs {
     uint64_t* st_rec;           // [nitems] look-back records over regions
     const uint32_t* st_hist;    // [nitems][256] per-region histograms
     const uint64_t* tag;        // single path: {n, input address} written by the histogram pass
-    uint32_t* counter;
+    uint32_t* counter;          // regions claimed by the encoder
+    uint32_t* plan_counter;     // groups of regions claimed by the plan
     uint32_t* status;
     LookbackHook hook;
 };
