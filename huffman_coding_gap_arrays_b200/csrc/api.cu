@@ -66,7 +66,7 @@ hgap_status encode_layout(const void* d_in, uint64_t n, void* d_workspace, size_
     a->counter = reinterpret_cast<uint32_t*>(ws) + 1;
     a->nitems_dev = reinterpret_cast<uint64_t*>(ws + 8);
     a->plan_counter = reinterpret_cast<uint32_t*>(ws + 16);
-    a->tag = reinterpret_cast<const uint64_t*>(ws + w.tag);
+    a->tag = reinterpret_cast<const uint64_t*>(ws + hgap::kEncWsTag);
     a->st_rec = reinterpret_cast<uint64_t*>(ws + w.st_rec);
     a->plan = reinterpret_cast<hgap::EncRegion*>(ws + w.plan);
     a->st_hist = reinterpret_cast<const uint32_t*>(ws + w.st_hist);
@@ -74,7 +74,7 @@ hgap_status encode_layout(const void* d_in, uint64_t n, void* d_workspace, size_
     h->nitems = nst;
     h->hist = reinterpret_cast<uint32_t*>(ws + w.scratch);
     h->st_hist = const_cast<uint32_t*>(a->st_hist);
-    h->tag = reinterpret_cast<uint64_t*>(ws + w.tag);
+    h->tag = reinterpret_cast<uint64_t*>(ws + hgap::kEncWsTag);
     return HGAP_OK;
 }
 
@@ -96,10 +96,19 @@ hgap_status encode_outputs(const hgap_codebook* cb, uint32_t* d_bits, uint64_t w
     return HGAP_OK;
 }
 
-// Clears what a call starts from; with `tag_too` also the tag and the scratch histogram.
+// Clears what a call starts from; with `tag_too` also what a histogram pass does.
 hgap_status encode_clear(const hgap::EncArgs& a, bool tag_too, cudaStream_t st) {
     const hgap::EncWorkspace w = hgap::encode_workspace(a.nitems);
-    return cudaMemsetAsync(a.status, 0, tag_too ? w.plan : w.tag, st) == cudaSuccess ? HGAP_OK : HGAP_ERR_CUDA;
+    return cudaMemsetAsync(a.status, 0, tag_too ? w.plan : hgap::kEncWsTag, st) == cudaSuccess ? HGAP_OK : HGAP_ERR_CUDA;
+}
+
+// A prepared call's launches.  (Should the encoder not start, the plan's records stay: no further call may use them.)
+hgap_status encode_launch_prepared(const hgap::EncArgs& a, const hgap::EncTable& t, cudaStream_t st) {
+    const hgap_status s = encode_clear(a, false, st);
+    if (s != HGAP_OK) return s;
+    const int e = hgap::launch_encode(a, t, 0, st);
+    if (e != 0) cudaMemsetAsync(const_cast<uint64_t*>(a.tag), 0, 16, st);
+    return cuda_status(e);
 }
 
 }  // namespace
@@ -134,10 +143,7 @@ hgap_status hgap_encode_prepared(const void* d_in, uint64_t n, const hgap_codebo
     if (s != HGAP_OK) return s;
     hgap::EncTable t;
     hgap::make_enc_table(*cb, &t);
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    s = encode_clear(a, false, st);
-    if (s != HGAP_OK) return s;
-    return cuda_status(hgap::launch_encode(a, t, 0, stream));
+    return encode_launch_prepared(a, t, reinterpret_cast<cudaStream_t>(stream));
 }
 
 hgap_status hgap_encode_part_prepared(const void* d_in, uint64_t n, const hgap_codebook* cb, uint64_t bit0,
@@ -164,10 +170,7 @@ hgap_status hgap_encode_part_prepared(const void* d_in, uint64_t n, const hgap_c
     J.bit0 = bit0;
     hgap::EncTable t;
     hgap::make_enc_table(*cb, &t);
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    s = encode_clear(a, false, st);
-    if (s != HGAP_OK) return s;
-    return cuda_status(hgap::launch_encode(a, t, 0, stream));
+    return encode_launch_prepared(a, t, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

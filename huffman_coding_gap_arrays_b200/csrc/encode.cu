@@ -420,6 +420,11 @@ __global__ void __launch_bounds__(kEncThreads, 2)
     };
     // warp 0: region `item` of the plan to reg[slot], and a job's codes to next_codes, asynchronously
     const uint64_t nitems = *a.nitems_dev;
+    // the plan is made: its records are zero again when a prepared call follows (st_rec, hgap_internal.h)
+    if (!a.jobs) {
+        const uint64_t stride = (uint64_t)gridDim.x * kEncThreads;
+        for (uint64_t g = (uint64_t)blockIdx.x * kEncThreads + tid; g * kPlanWarps < nitems; g += stride) a.st_rec[g] = 0;
+    }
     auto fetch_region = [&](uint32_t slot, uint64_t item) {
         EncRegion* const to = &sh.reg[slot];
         if (item < nitems) {

@@ -79,11 +79,15 @@ constexpr uint64_t kEncStOverhead = 1;  // chunks
 
 // Encoder workspace for nst super-tiles:
 //   [status u32][counter u32][super-tiles to encode u64][plan counter u32, 12 bytes of padding]
-//   [st_rec u64 x nst]                                                      cleared by every call
-//   [tag: n u64, input u64][scratch histogram u32 x 256]                    and these by the histogram pass
+//                                                         cleared by every call
+//   [tag: n u64, input u64][st_rec u64 x nst][scratch histogram u32 x 256]
+//                                                         these by the histogram pass, and st_rec by
+//                                                         the encoder again, for the next prepared call
 //   [plan EncRegion x nst][st_hist u32 x 256 x nst]
+// The tag's place depends on no input: a histogram pass over any other one writes over it.
+constexpr size_t kEncWsTag = 32;
 struct EncWorkspace {
-    size_t st_rec, tag, scratch, plan, st_hist, bytes;
+    size_t st_rec, scratch, plan, st_hist, bytes;
 };
 inline uint64_t encode_chunks(uint64_t n) { return (n + 15 + kEncChunkBytes - 1) / kEncChunkBytes; }
 // An upper bound of the super-tile count of every input of up to n bytes (at any
@@ -164,9 +168,8 @@ constexpr uint32_t kRegionVec = 4u;    // output words are 16-byte aligned
 
 inline EncWorkspace encode_workspace(uint64_t nst) {
     EncWorkspace w;
-    w.st_rec = 32;
-    w.tag = (w.st_rec + 8 * (size_t)nst + 15) & ~(size_t)15;
-    w.scratch = w.tag + 16;
+    w.st_rec = kEncWsTag + 16;
+    w.scratch = (w.st_rec + 8 * (size_t)nst + 15) & ~(size_t)15;
     w.plan = w.scratch + 1024;
     w.st_hist = w.plan + sizeof(EncRegion) * (size_t)nst;
     w.bytes = w.st_hist + 1024 * (size_t)nst;
