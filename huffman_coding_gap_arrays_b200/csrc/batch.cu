@@ -146,8 +146,22 @@ __device__ __forceinline__ uint64_t block_sum_u64(uint64_t v, uint64_t* s_warp) 
     return t;
 }
 
+// The region size when the caller names none: 8 chunks, and larger ones where the
+// batch still gives every encoder CTA (296) many of them, since each region costs
+// its histogram fold, its plan and a last step that is partly empty.
+// Compress in us at 8 / 16 / 32 chunks, by regions of 8 chunks: 4 KiB - 4 MiB
+// buffers, 4725 regions 390 / 396 / 431, 9644: 717 / 693 / 723, 19678: 1383 /
+// 1321 / 1329, 39879: 2734 / 2591 / 2558; buffers of 1 MiB, 4352: 358 / 344 /
+// 351, 17408: 1209 / 1146 / 1130; of 256 KiB, 2560: 212 / 210 / 223, 10240: 653 /
+// 619 / 618.  (12 and 24 chunks lie between or above.)  By the batch's own regions:
+// the workspace may be one kept for larger batches.  Returns log2(chunks / 8).
+__device__ __forceinline__ uint32_t default_shift(uint64_t regions) {
+    return regions >= 80 * kEncCtas ? 2u : regions >= 20 * kEncCtas ? 1u : 0u;
+}
+
 // Numbers the regions, starts the encoder jobs and writes every region for the
 // histogram pass (so that no CTA searches for a region's buffer there).
+// base_chunks: the smallest region size, 0: default_shift.
 __global__ void __launch_bounds__(kScanThreads) benc_setup_kernel(uint32_t count, const uint8_t* const* inputs,
                                                                   const uint64_t* sizes,
                                                                   const uint8_t* region_chunks,
@@ -164,13 +178,14 @@ __global__ void __launch_bounds__(kScanThreads) benc_setup_kernel(uint32_t count
         uint64_t n, nst;
         uint32_t lo, st;
     };
+    uint32_t base = base_chunks;
     auto load = [&](uint64_t j) {
         Buf b = {nullptr, 0, 0, 0, 0};
         if (j < count) {
             b.n = sizes[j];
             b.in = inputs[j];
-            uint32_t rc = region_chunks ? region_chunks[j] : base_chunks;
-            if (rc < base_chunks) rc = base_chunks;
+            uint32_t rc = region_chunks ? region_chunks[j] : base;
+            if (rc < base) rc = base;
             if (rc > 32) rc = 32;
             b.lo = (uint32_t)(reinterpret_cast<uintptr_t>(b.in) & 15);
             b.st = rc * (uint32_t)kEncChunkBytes;
@@ -181,7 +196,24 @@ __global__ void __launch_bounds__(kScanThreads) benc_setup_kernel(uint32_t count
     const uint64_t run = scan_run(count), first = blockIdx.x * run;
     const uint64_t end = first + run < count ? first + run : count;
     uint64_t sum = 0;
-    for (uint64_t j = threadIdx.x; j < first && j < count; j += kScanThreads) sum += load(j).nst;
+    if (base) {
+        for (uint64_t j = threadIdx.x; j < first && j < count; j += kScanThreads) sum += load(j).nst;
+    } else {  // the regions of 8 chunks in all buffers, and of every size before this CTA's run
+        uint64_t all = 0, before[3] = {};
+        for (uint64_t j = threadIdx.x; j < count; j += kScanThreads) {
+            const uint64_t n = sizes[j], end = n ? n + (reinterpret_cast<uintptr_t>(inputs[j]) & 15) : 0;
+#pragma unroll
+            for (uint32_t k = 0; k < 3; ++k) {
+                const uint32_t st = (8u << k) * kEncChunkBytes;
+                const uint64_t nst = (end + st - 1) / st;
+                if (k == 0) all += nst;
+                if (j < first) before[k] += nst;
+            }
+        }
+        const uint32_t k = default_shift(block_sum_u64(all, s_warp));
+        base = 8u << k;
+        sum = k == 0 ? before[0] : k == 1 ? before[1] : before[2];
+    }
     uint64_t carry = block_sum_u64(sum, s_warp);
     for (uint64_t base = first; base < end; base += kScanThreads) {
         const uint64_t j = base + threadIdx.x;
@@ -794,19 +826,6 @@ uint32_t base_chunks(const hgap_batch_config* cfg) {
     return rc > 32 ? 32 : rc;
 }
 
-// The region size when the caller names none: 8 chunks, and larger ones where the
-// batch still gives every encoder CTA (296) many of them, since each region costs
-// its histogram fold, its plan and a last step that is partly empty.  The host
-// knows the sizes only as what the workspace holds, counted in 8-chunk regions.
-// Compress in us at 8 / 16 / 32 chunks, by regions of 8 chunks: 4 KiB - 4 MiB
-// buffers, 4725 regions 390 / 396 / 431, 9644: 717 / 693 / 723, 19678: 1383 /
-// 1321 / 1329, 39879: 2734 / 2591 / 2558; buffers of 1 MiB, 4352: 358 / 344 /
-// 351, 17408: 1209 / 1146 / 1130; of 256 KiB, 2560: 212 / 210 / 223, 10240: 653 /
-// 619 / 618.  (12 and 24 chunks lie between or above.)
-uint32_t default_chunks(uint64_t regions) {
-    return regions >= 80 * kEncCtas ? 32 : regions >= 20 * kEncCtas ? 16 : 8;
-}
-
 // Compress workspace: [header 1024: status @0, counters @4 (three), nitems @64] [hists]
 // [st_rec] (zero at the start of a call, together: one memset) [jobs] [item0s]
 // [tables] [plan] [st_hist], the per-region arrays (st_rec, plan, st_hist) for
@@ -956,7 +975,7 @@ hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, 
     HistRegion* hist_regions = reinterpret_cast<HistRegion*>(plan);
 
     // (per-buffer sizes are the caller's choice too)
-    const uint32_t chunks = cfg->region_chunks || d_region_chunks ? base_chunks(cfg) : default_chunks(L.max_regions);
+    const uint32_t chunks = cfg->region_chunks || d_region_chunks ? base_chunks(cfg) : 0;
     if (cudaMemsetAsync(ws, 0, L.st_rec + 8 * (size_t)L.max_regions, st) != cudaSuccess) return HGAP_ERR_CUDA;
     benc_setup_kernel<<<scan_grid(count), kScanThreads, 0, st>>>(count, d_inputs, d_sizes, d_region_chunks, chunks, jobs,
                                                                  item0s, hist_regions, nitems, L.max_regions, status);

@@ -276,7 +276,7 @@ typedef struct hgap_batch_entry {
 /* Launch shape; every choice leaves the output format unchanged. */
 typedef struct hgap_batch_config {
     uint32_t region_chunks;    /* encoder region = region_chunks x 8 KiB (1..32); 0: 8, or 16 / 32 for
-                                  a workspace of 5920 / 23680 regions of 8 and more */
+                                  a batch of 5920 / 23680 regions of 8 and more */
     uint32_t hist_ctas_per_sm; /* persistent grids, CTAs per SM (0 = occupancy maximum) */
     uint32_t enc_ctas_per_sm;
     uint32_t dec_ctas_per_sm;
