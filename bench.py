@@ -66,7 +66,7 @@ def parse():
                    help="buffers of the batched workload (fewer only for profiling captures)")
     p.add_argument("--plain-buffers", type=int, default=4096,
                    help="buffers of the batch timed through the plain per-buffer path")
-    p.add_argument("--no-tune", action="store_true", help="skip tuning: fixed default launch shape")
+    p.add_argument("--no-tune", action="store_true", help="skip tuning: the library's default launch shape")
     p.add_argument("--shard", action="store_true",
                    help="N > 1: split one batch across the ranks by bytes (strong scaling) instead of "
                         "giving every rank its own batch (weak scaling)")
@@ -703,8 +703,8 @@ def run_batch(args, rank, world, dev, pg):
     tuning = {}
     learned = None
     if args.no_tune:
-        cfg = B.LaunchConfig()
-        tuning["method"] = "fixed default"
+        cfg = B.LaunchConfig(region_chunks=0)
+        tuning["method"] = "library default"
     else:
         t0 = time.time()
         learned = train_learned_tuner(dev)
@@ -714,7 +714,7 @@ def run_batch(args, rank, world, dev, pg):
         t0 = time.time()
         res = T.Autotuner(reps=2, warmup=1).tune(ins, outs, feats, plan=plan)
         tuning["autotuner_seconds"] = round(time.time() - t0, 2)
-        picks = {"default": B.LaunchConfig(), "autotuner": res.config}
+        picks = {"default": B.LaunchConfig(region_chunks=0), "autotuner": res.config}
         if learned.usable:
             picks["mlp"] = learned.choose(feats)
         measured = {}

@@ -32,7 +32,11 @@ DECOMPRESS_KERNELS = 8
 
 @dataclass
 class LaunchConfig:
-    """Launch shape of the batched kernels; no choice changes the output."""
+    """Launch shape of the batched kernels; no choice changes the output.
+
+    ``LaunchConfig()`` is one fixed shape for every batch, with regions of 8
+    chunks.  ``region_chunks=0`` takes the region size by the batch, as
+    ``BatchCodec`` does without a config: name it beside any other field."""
     region_chunks: int = 8      # encoder region = region_chunks x 8 KiB (1..32; 0 = by the batch's size)
     hist_ctas_per_sm: int = 0   # persistent grids: CTAs per SM (0 = occupancy maximum)
     enc_ctas_per_sm: int = 0

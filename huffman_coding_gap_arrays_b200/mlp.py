@@ -13,10 +13,11 @@ move with the launch shape.
 
 It is trained on the autotuner's own records (``tuner.Autotuner``).
 ``LearnedTuner.choose`` scores every candidate shape with a forward pass of an
-ensemble of networks (one per seed) and keeps the default shape unless a
-candidate that every network predicts faster has a mean predicted gain above
-a margin -- the exhaustive autotuner's pick without its measurements.  It only chooses launch shapes, which leave the
-output format unchanged.  Untrained, or with a held-out error above its
+ensemble of networks (one per seed) and keeps the default shape -- the
+library's own, whose regions go by the batch -- unless a candidate that every
+network predicts faster has a mean predicted gain above a margin: the
+exhaustive autotuner's pick without its measurements.  It only chooses launch
+shapes, which leave the output format unchanged.  Untrained, or with a held-out error above its
 limit, it falls back to running the autotuner.
 """
 from __future__ import annotations
@@ -29,7 +30,7 @@ import torch
 from ._lib import MLP_IN, MLP_OUT, MLP_PARAMS, check, lib
 from .batch import LaunchConfig
 from .codec import _stream
-from .tuner import DEC_SPACE, Autotuner, compress_space, with_dec
+from .tuner import DEC_SPACE, Autotuner, compress_space, default_chunks, with_dec
 
 SHAPES = [(32, 10), (32,), (32, 32), (32,), (2, 32), (2,)]
 # CTAs per SM that "0" (the occupancy maximum) means for each grid on B200
@@ -39,8 +40,9 @@ MAX_CTAS = {"hist": 4, "enc": 2, "dec": 5}  # what 0 (the occupancy maximum) sta
 TILE_CODE = {0: 0.0, 256: -1.0, 512: 1.0}
 
 
-def config_vector(cfg: LaunchConfig) -> np.ndarray:
-    return np.array([math.log2(max(cfg.region_chunks, 1)),
+def config_vector(cfg: LaunchConfig, features) -> np.ndarray:
+    """A shape as the networks take it, for an input with these features."""
+    return np.array([math.log2(cfg.region_chunks or default_chunks(features)),
                      cfg.hist_ctas_per_sm or MAX_CTAS["hist"],
                      cfg.enc_ctas_per_sm or MAX_CTAS["enc"],
                      cfg.dec_ctas_per_sm or MAX_CTAS["dec"],
@@ -51,7 +53,7 @@ def records_to_xy(records, relative: bool = True):
     """Autotuner records -> (X n x 10, T n x 2 log-ms targets, NaN = not
     measured).  With `relative`, each target is taken relative to the mean
     log time of the records with the same features (one tuned input)."""
-    X = np.stack([np.concatenate([r.features, config_vector(r.config)]) for r in records]).astype(np.float32)
+    X = np.stack([np.concatenate([r.features, config_vector(r.config, r.features)]) for r in records]).astype(np.float32)
     T = np.stack([[math.log(r.compress_ms) if r.compress_ms == r.compress_ms else np.nan,
                    math.log(r.decompress_ms) if r.decompress_ms == r.decompress_ms else np.nan]
                   for r in records]).astype(np.float64)
@@ -152,7 +154,7 @@ class LearnedTuner:
         self.max_rmse = max_rmse
         self.margin = margin
         self.dec_margin = dec_margin  # the decoder grid moves decompress time little: be stricter
-        self.default = default or LaunchConfig()
+        self.default = default or LaunchConfig(region_chunks=0)
         self.holdout_rmse = float("inf")
         self._memo = {}  # choices by features rounded to 1/8: a serving loop asks about the same sizes
 
@@ -188,7 +190,7 @@ class LearnedTuner:
         """Among the candidates that every member of the ensemble predicts
         faster than the default, the one with the best mean prediction --
         taken only if that mean gain exceeds the margin."""
-        X = np.stack([np.concatenate([f, config_vector(c)]) for c in list(cands) + [default]])
+        X = np.stack([np.concatenate([f, config_vector(c, f)]) for c in list(cands) + [default]])
         P = np.stack([m.predict(X)[:, out] for m in self.mlps])  # members x (candidates + default)
         rel = P[:, :-1] - P[:, -1:]                               # log time relative to the default
         mean = np.where((rel < 0).all(axis=0), rel.mean(axis=0), np.inf)
@@ -226,11 +228,9 @@ class LearnedTuner:
         feats = np.concatenate([keys[:, None], np.tile(rest, (len(keys), 1))], axis=1).astype(np.float32)
         nf = len(feats)
 
-        def rows(cfg_vecs):  # every feature row against every config row (per feature, in order)
-            k = cfg_vecs.shape[-2]
-            F = np.repeat(feats, k, axis=0)
-            Cv = cfg_vecs.reshape(-1, cfg_vecs.shape[-1]) if cfg_vecs.ndim == 3 else np.tile(cfg_vecs, (nf, 1))
-            return np.concatenate([F, Cv], axis=1)
+        def rows(cfg_vecs):  # every feature row against its config rows, in order
+            F = np.repeat(feats, cfg_vecs.shape[1], axis=0)
+            return np.concatenate([F, cfg_vecs.reshape(-1, cfg_vecs.shape[-1])], axis=1)
 
         def best(P, k, margin):  # per feature row: the candidate index, or k (the default)
             rel = P[:, :, :k] - P[:, :, k:k + 1]
@@ -240,12 +240,12 @@ class LearnedTuner:
 
         # stage 1: the compress shape for every size at once
         cands = comp + [base]
-        V = np.stack([config_vector(c) for c in cands])
+        V = np.stack([np.stack([config_vector(c, f) for c in cands]) for f in feats])
         P = np.stack([m.predict(rows(V))[:, 0] for m in self.mlps]).reshape(len(self.mlps), nf, len(cands))
         picks = [cands[i] for i in best(P, len(comp), self.margin)]
         # stage 2: the decoder grid for each size's compress shape
         dec = [[with_dec(c, d) for d in self.dec_space] + [with_dec(c, d0dec)] for c in picks]
-        V = np.stack([np.stack([config_vector(c) for c in row]) for row in dec])
+        V = np.stack([np.stack([config_vector(c, f) for c in row]) for f, row in zip(feats, dec)])
         nd = len(self.dec_space) + 1
         P = np.stack([m.predict(rows(V))[:, 1] for m in self.mlps]).reshape(len(self.mlps), nf, nd)
         for j, i in enumerate(best(P, nd - 1, self.dec_margin)):

@@ -200,7 +200,7 @@ class Server:
         # work dominates), and shapes the tuner predicts faster on the GPU measured slower in
         # service: such batches keep the tuner's default shape
         self.tuner_min_bytes = int(tuner_min_bytes)
-        self.config = config or LaunchConfig()
+        self.config = config or LaunchConfig(region_chunks=0)
         self.budget = float(hbm_budget)
         self.max_batch = int(max_batch)
         self.max_inflight = int(max_inflight)

@@ -27,7 +27,7 @@ import torch
 
 from .batch import BatchCodec, LaunchConfig
 
-REGIONS = (1, 2, 4, 8, 16, 32)
+REGIONS = (1, 2, 4, 8, 16, 32)  # (0, by the batch, is one of the last three)
 HIST_CTAS = (2, 4)
 ENC_CTAS = (1, 2)
 # decoder CTAs per SM; each decoder is clamped to what fits it (5 for 256-segment tiles, 4 for
@@ -35,6 +35,15 @@ ENC_CTAS = (1, 2)
 DEC_CTAS = (1, 2, 3, 4, 0)
 DEC_TILES = (0, 256, 512)  # decoder tile: the default (0), or 256 / 512 segments
 DEC_SPACE = tuple(itertools.product(DEC_CTAS, DEC_TILES))  # (CTAs per SM, tile) pairs
+
+
+def default_chunks(features) -> int:
+    """The region size that ``region_chunks=0`` stands for, in chunks, for a
+    batch with these features: the library's rule (by the regions of 8 chunks:
+    16 from 5920, 32 from 23680), each buffer's last region half full."""
+    f = np.asarray(features, np.float64)
+    regions = 2.0 ** f[0] / 65536 + (2.0 ** f[4] / 2 if f.size > 4 else 0.5)
+    return 32 if regions >= 23680 else 16 if regions >= 5920 else 8
 
 
 def with_dec(cfg: LaunchConfig, dec) -> LaunchConfig:
@@ -158,7 +167,7 @@ class Autotuner:
         device status."""
         sizes = [int(t.numel()) for t in inputs]
         if plan is None:
-            base = min(c.region_chunks for c in self.space)
+            base = min(c.region_chunks or 8 for c in self.space)
             plan = BatchCodec(sizes, LaunchConfig(region_chunks=base))
             plan.bind(inputs, outputs)
         feats = features if features is not None else np.zeros(4, np.float32)
@@ -186,5 +195,5 @@ class Autotuner:
 
 
 __all__ = ["Autotuner", "TuneResult", "Record", "compress_space", "buffer_features", "batch_features",
-           "features_from_hist", "with_dec",
+           "features_from_hist", "default_chunks", "with_dec",
            "REGIONS", "HIST_CTAS", "ENC_CTAS", "DEC_CTAS", "DEC_TILES", "DEC_SPACE"]
