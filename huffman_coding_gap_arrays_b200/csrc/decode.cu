@@ -55,11 +55,6 @@
 
 namespace hgap {
 
-// Look-back window = 32 * kDecLookK tiles per round trip.  One load a lane: the
-// extra warps of all CTAs read the same few lines, and a wider window costs
-// each of them more than the round trips it saves (Zipf(1.2) 256 MiB at 32 / 64 /
-// 128 records: 443 / 453 / 479 us, BF16 mantissa 371 / 378 / 392).
-constexpr int kDecLookK = 1;
 // In place of a warp's symbol count: one of its waits gave up.
 constexpr uint32_t kGaveUp = ~0u;
 
@@ -420,8 +415,8 @@ __global__ void __launch_bounds__(DecCfg<R, W, S>::kThreads, DecCfg<R, W, S>::kM
                     ++copies;
                 }
             }
-            const uint64_t O = lookback_resolve<kDecLookK>(a.lookback, T.rec, Ct, T.first, a.status, lane,
-                                                           wait_limit(a.hook), T.rec + 1 != a.hook.hold_plus1);
+            const uint64_t O = lookback_resolve(a.lookback, T.rec, Ct, T.first, a.status, lane, wait_limit(a.hook),
+                                                T.rec + 1 != a.hook.hold_plus1);
             if (lane == 0) {
                 if (T.last && O + Ct < T.n) atomicOr(a.status, kDevSize);
                 dst[i & 1] = T.out + O;

@@ -166,11 +166,11 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, uint32_t lane) {
 
 // Single-pass decoupled look-back (the reference's scheme,
 // encoder/src/encoder.cu:222-263, decoder/src/decoder.cu:601-638) run by one
-// full warp, with a window of 32*K predecessors per round trip: load j of lane
-// l is the tile at window position 32*j + l, counted from the nearest, so that a
-// load of the warp covers 256 consecutive bytes (with K consecutive records a
-// lane, 2 loads took twice the sectors and the decoder 4 % more time).  The inclusive-prefix frontier advances at most one window per L2
-// round trip, so the window must exceed the tiles started per round trip.
+// full warp, with a window of 32 predecessors per round trip, one a lane, the
+// nearest in lane 0.  One load a lane: all look-backs read the same few lines,
+// and a wider window costs each of them more than the round trips it saves
+// (decoder, 32 / 64 / 128 records: Zipf(1.2) 256 MiB 443 / 453 / 479 us, BF16
+// mantissa 371 / 378 / 392).
 // Only the records between the tile and the nearest inclusive prefix matter.
 // The window is loaded without blocking; records in front of the nearest
 // unpublished one are summed at once and left behind, and the next window
@@ -189,7 +189,6 @@ __device__ __forceinline__ void lookback_publish(uint64_t* rec, uint64_t tile, u
 
 // `limit_ns` bounds the wait for each record; `publish` = false keeps the
 // inclusive prefix unpublished (the bounded-wait test hook only: LookbackHook).
-template <int K>
 __device__ __forceinline__ uint64_t lookback_resolve(uint64_t* rec, uint64_t tile, uint64_t agg, bool first,
                                                      uint32_t* status, uint32_t lane, uint64_t limit_ns,
                                                      bool publish = true) {
@@ -197,26 +196,13 @@ __device__ __forceinline__ uint64_t lookback_resolve(uint64_t* rec, uint64_t til
     uint64_t excl = 0, t0 = 0;
     int64_t top = (int64_t)tile - 1;
     for (;;) {
-        uint64_t v[K];
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            const int64_t i = top - (int64_t)(32 * j + lane);
-            v[j] = i >= 0 ? ld_relaxed_u64(rec + i) : kFlagP;
-        }
-        int gp = 32 * K, gz = 32 * K;  // the window's nearest inclusive prefix / unpublished record
-#pragma unroll
-        for (int j = K - 1; j >= 0; --j) {
-            const uint32_t pmask = __ballot_sync(kFull, (v[j] & kFlagP) != 0);
-            const uint32_t zmask = __ballot_sync(kFull, v[j] == 0);
-            if (pmask) gp = 32 * j + __ffs(pmask) - 1;
-            if (zmask) gz = 32 * j + __ffs(zmask) - 1;
-        }
-        const int take = gz < gp ? gz : gp < 32 * K ? gp + 1 : 32 * K;  // records to sum
-        uint64_t sum = 0;
-#pragma unroll
-        for (int j = 0; j < K; ++j)
-            if ((int)(32 * j + lane) < take) sum += v[j] & kValueMask;
-        excl += warp_sum_u64(sum);
+        const int64_t i = top - (int64_t)lane;
+        const uint64_t v = i >= 0 ? ld_relaxed_u64(rec + i) : kFlagP;
+        // the window's nearest inclusive prefix / unpublished record
+        const uint32_t pmask = __ballot_sync(kFull, (v & kFlagP) != 0), zmask = __ballot_sync(kFull, v == 0);
+        const int gp = pmask ? __ffs(pmask) - 1 : 32, gz = zmask ? __ffs(zmask) - 1 : 32;
+        const int take = gz < gp ? gz : gp < 32 ? gp + 1 : 32;  // records to sum
+        excl += warp_sum_u64((int)lane < take ? v & kValueMask : 0);
         if (gp < gz) break;
         top -= take;
         if (take) {

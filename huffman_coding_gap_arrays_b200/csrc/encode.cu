@@ -116,7 +116,6 @@ __device__ __forceinline__ uint64_t region_end(const EncJob& J, uint64_t st) {
 
 constexpr int kPlanThreads = 256;
 constexpr int kPlanWarps = kPlanThreads / 32;  // regions of a group
-constexpr int kPlanLookK = 1;
 
 // One warp per region: its bit count (its histogram times the code lengths),
 // its first output bit, and by re-encoding a few bytes backwards from there
@@ -199,8 +198,8 @@ __global__ void __launch_bounds__(kPlanThreads) enc_plan_kernel(const __grid_con
             if (lane == 0 && !held) lookback_publish(a.st_rec, g, sum, starts != 0);
             uint32_t claim = 0;
             if (lane == 0) claim = atomicAdd(a.plan_counter, 1u);
-            const uint64_t e = lookback_resolve<kPlanLookK>(a.st_rec, g, sum, (starts & 1u) != 0, a.status, lane,
-                                                            wait_limit(a.hook), !held && starts == 0);
+            const uint64_t e = lookback_resolve(a.st_rec, g, sum, (starts & 1u) != 0, a.status, lane, wait_limit(a.hook),
+                                                !held && starts == 0);
             if (lane == 0) {
                 s_excl = e;
                 s_next = claim;
@@ -214,7 +213,7 @@ __global__ void __launch_bounds__(kPlanThreads) enc_plan_kernel(const __grid_con
         if (!upto) excl += s_excl;
         // (test hook: the regions after a held one in its own group wait for it, too)
         if (held && item >= a.hook.hold_plus1)
-            lookback_resolve<1>(a.st_rec, g + 1, 0, false, a.status, lane, wait_limit(a.hook), false);
+            lookback_resolve(a.st_rec, g + 1, 0, false, a.status, lane, wait_limit(a.hook), false);
         const uint64_t vfirst = st * (uint64_t)J.st_bytes;  // first byte of this region
         const uint64_t G = J.bit0 + excl;
         uint32_t head = 0, gap_head = 0;
