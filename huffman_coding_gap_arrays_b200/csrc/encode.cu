@@ -134,6 +134,8 @@ __global__ void __launch_bounds__(kPlanThreads) enc_plan_kernel(const __grid_con
                                                                 const __grid_constant__ EncTable tab) {
     __shared__ EncTable s_tab;
     const uint32_t tid = threadIdx.x, lane = tid & 31;
+    uint32_t claim = 0;
+    if (tid == 0) claim = atomicAdd(a.plan_counter, 1u);  // (beside the loads below)
     uint64_t nitems = a.nitems;
     if (a.jobs) {
         nitems = *a.nitems_dev;
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(kPlanThreads) enc_plan_kernel(const __grid_con
     __shared__ uint64_t s_agg[kPlanWarps], s_excl;
     __shared__ uint32_t s_first[kPlanWarps], s_next;
     const uint32_t warp = tid >> 5;
-    if (tid == 0) s_next = atomicAdd(a.plan_counter, 1u);
+    if (tid == 0) s_next = claim;
     __syncthreads();
     for (uint64_t g = s_next; g * kPlanWarps < nitems; g = s_next) {
         const uint64_t item = g * kPlanWarps + warp;
@@ -196,7 +198,6 @@ __global__ void __launch_bounds__(kPlanThreads) enc_plan_kernel(const __grid_con
             const uint32_t from = starts ? 31 - __clz(starts) : 0u;
             const uint64_t sum = warp_sum_u64(lane >= from ? mine : 0);
             if (lane == 0 && !held) lookback_publish(a.st_rec, g, sum, starts != 0);
-            uint32_t claim = 0;
             if (lane == 0) claim = atomicAdd(a.plan_counter, 1u);
             const uint64_t e = lookback_resolve(a.st_rec, g, sum, (starts & 1u) != 0, a.status, lane, wait_limit(a.hook),
                                                 !held && starts == 0);
