@@ -15,7 +15,8 @@ It is trained on the autotuner's own records (``tuner.Autotuner``).
 ``LearnedTuner.choose`` scores every candidate shape with a forward pass of an
 ensemble of networks (one per seed) and keeps the default shape -- the
 library's own, whose regions go by the batch -- unless a candidate that every
-network predicts faster has a mean predicted gain above a margin: the
+network predicts faster has a mean predicted gain above a margin, which after
+training is at least the networks' own error on the held-out records: the
 exhaustive autotuner's pick without its measurements.  It only chooses launch
 shapes, which leave the output format unchanged.  Untrained, or with a held-out error above its
 limit, it falls back to running the autotuner.
@@ -167,11 +168,21 @@ class LearnedTuner:
             m.fit(X, T, steps=steps)
             mlps.append(m)
         t = cls(mlps, **kw)
-        Xh, Th = records_to_xy(holdout) if holdout else (X, T)
-        P = t.predict(Xh)
-        ok = np.isfinite(Th)
-        t.holdout_rmse = float(np.sqrt(np.mean((P[ok] - Th[ok]) ** 2))) if ok.any() else float("inf")
+        t.hold_out(holdout if holdout else records, raise_margins="margin" not in kw and "dec_margin" not in kw)
         return t
+
+    def hold_out(self, records, raise_margins: bool = True) -> None:
+        """Measures the ensemble's error on records it was not trained on.  A
+        predicted gain below that error says nothing, so the margins are raised to it."""
+        X, T = records_to_xy(records)
+        D = self.predict(X) - T
+        ok = np.isfinite(D)
+        self.holdout_rmse = float(np.sqrt(np.mean(D[ok] ** 2))) if ok.any() else float("inf")
+        if raise_margins:
+            rms = [float(np.sqrt(np.mean(d[np.isfinite(d)] ** 2))) if np.isfinite(d).any() else 0.0 for d in D.T]
+            self.margin = max(self.margin, 1.0 - math.exp(-rms[0]))
+            self.dec_margin = max(self.dec_margin, 1.0 - math.exp(-rms[1]))
+        self._memo.clear()
 
     def set_default(self, cfg: LaunchConfig) -> None:
         """The shape kept unless a candidate is predicted faster by the margin

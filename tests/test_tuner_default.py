@@ -46,3 +46,23 @@ def test_autotuner_space_may_hold_the_default():
     r = T.Record(_features(24000, 64), LIBRARY, 1.0, float("nan"))
     X, _ = M.records_to_xy([r])
     assert X.shape == (1, 10) and X[0, 5] == 5.0
+
+
+@pytest.mark.parametrize("error,kept", [(0.0, False), (0.1, False), (0.3, True)])
+def test_a_gain_below_the_held_out_error_is_no_reason(error, kept):
+    """The network predicts 0.2 (log) between two region sizes; its held-out records say +- `error`."""
+    f = _features(3000, 64)
+    t = M.LearnedTuner([_Net(4.0)])  # 16 chunks best, the default stands for 8
+    recs = []
+    for i, r in enumerate((1, 2, 4, 8, 16, 32)):
+        cfg = LaunchConfig(region_chunks=r)
+        p = float(t.predict(np.concatenate([f, M.config_vector(cfg, f)])[None])[0, 0])
+        recs.append(T.Record(f, cfg, float(np.exp(p + (error if i % 2 else -error))), float("nan")))
+    mean = np.mean([np.log(r.compress_ms) for r in recs])
+    net = _Net(4.0)
+    net.predict = lambda X, g=_Net(4.0).predict: g(X) - np.array([mean, 0.0])  # targets are relative to their mean
+    t = M.LearnedTuner([net])
+    t.hold_out(recs)
+    assert abs(t.holdout_rmse - error) < 1e-6 and t.dec_margin == 0.05
+    assert abs(t.margin - max(0.03, 1 - np.exp(-error))) < 1e-6
+    assert t.choose(f).region_chunks == (0 if kept else 16)
