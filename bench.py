@@ -99,7 +99,7 @@ def peak_hbm():
 def traffic_ratios():
     """DRAM bytes per uncompressed byte per kernel, from the committed ncu summary."""
     out = {}
-    for name in ("dram_traffic_mixed_1g.txt", "dram_traffic_batch1024.txt"):
+    for name in ("dram_traffic_mixed_1g.txt", "dram_traffic_batch4096.txt"):
         path = os.path.join(ROOT, "profiles", name)
         if not os.path.exists(path):
             continue

@@ -40,11 +40,13 @@
 // and by instruction issue (72 %), not by HBM: fewer wavefronts at three more
 // instructions a step measured slower (Last, below).  Measured (B200, 256 MiB,
 // call without the status read), against a kernel with four CTA barriers a tile, a
-// branch to a second table level and byte-wise compaction: Zipf(1.2) 524 -> 376
-// us, mixed 489 -> 393, BF16 mantissa 422 -> 363, BF16 exponents 324 -> 266,
-// clamped Gaussians of sigma 1 / 3 431 -> 306 / 321 -> 261; 1024 buffers of
-// 4 KiB - 4 MiB (593 MB) 1047 -> 785 us.  Of that the branch-free table gives
-// Zipf(1.2) 439 -> 401 us and the batch 896 -> 858.
+// branch to a second table level and byte-wise compaction: Zipf(1.2) 524 -> 383
+// us, mixed 489 -> 403, BF16 mantissa 422 -> 370, BF16 exponents 324 -> 267,
+// clamped Gaussians of sigma 1 / 3 431 -> 247 / 321 -> 264; 1024 buffers of
+// 4 KiB - 4 MiB (593 MB) 1047 -> 792 us.  (The kernel alone: Zipf(1.2) 362 us,
+// mixed 383, mantissa 348, exponents 247.)  The branch-free table gave Zipf(1.2)
+// 439 -> 401 us and the batch 896 -> 858; that no warp leaves alone when its wait
+// gives up costs 0 to 1.2 % of a call (mixed 1 GiB 1494 -> 1511 us, the others less).
 #include <cuda_runtime.h>
 
 #include <type_traits>

@@ -50,10 +50,10 @@
 //
 // Measured (B200, kernel alone), against a loop that packed two codes at a time
 // into one image of the CTA with two barriers per 8 KiB: 256 MiB of Zipf(1.2)
-// 344 -> 237 us, of the mixed stream 409 -> 243, of BF16 sign|mantissa bytes
-// 353 -> 282, of BF16 exponents 335 -> 234; 1024 buffers of 4 KiB - 4 MiB
-// (593 MB) in 64 KiB regions 879 -> 654 us, in 256 KiB regions 791 -> 568.
-// 0.73 warp instructions per byte (1.12 before) at 71 % of the issue slots.
+// 344 -> 239 us, of the mixed stream 409 -> 243, of BF16 sign|mantissa bytes
+// 353 -> 254, of BF16 exponents 335 -> 237; 1024 buffers of 4 KiB - 4 MiB
+// (593 MB) in 64 KiB regions 879 -> 525 us, in 256 KiB regions 791 -> 546.
+// 0.74 warp instructions per byte (1.12 before) at 74 % of the issue slots.
 #include <cuda_runtime.h>
 
 #include "device_util.cuh"
@@ -121,15 +121,15 @@ constexpr int kPlanWarps = kPlanThreads / 32;  // regions of a group
 // its first output bit, and by re-encoding a few bytes backwards from there
 // what precedes it in its first word and gap byte.  The counts are summed over a
 // CTA's eight regions first, and the look-back runs over these groups (over
-// single regions it took 13 us for the 1171 regions of 256 MiB, here 8): a
+// single regions it took 13 us for the 1171 regions of 256 MiB, here 7): a
 // group in which a job starts publishes the sum from there on as an inclusive
 // prefix.  Groups are claimed in order, and the next one only when the current
 // one's sum is published: a look-back only ever waits for CTAs that run, however
 // many of the grid's CTAs the GPU has room for beside other work.
 // All the regions' dependent loads overlap here, where one warp of a persistent
 // encoder CTA went through them between two regions: encoder and plan of 1024
-// buffers in 64 KiB regions 659 -> 543 us, of 4096 small buffers 170 -> 126, of
-// one 16 MiB buffer 25 -> 26; one 256 MiB buffer pays its 8 us (237 -> 249).
+// buffers in 64 KiB regions 659 -> 542 us, of 4096 small buffers 170 -> 126, of
+// one 16 MiB buffer 25 -> 26; one 256 MiB buffer pays its 7 us (237 -> 246).
 __global__ void __launch_bounds__(kPlanThreads) enc_plan_kernel(const __grid_constant__ EncArgs a,
                                                                 const __grid_constant__ EncTable tab) {
     __shared__ EncTable s_tab;

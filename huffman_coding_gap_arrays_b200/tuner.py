@@ -30,8 +30,8 @@ from .batch import BatchCodec, LaunchConfig
 REGIONS = (1, 2, 4, 8, 16, 32)  # (0, by the batch, is one of the last three)
 HIST_CTAS = (2, 4)
 ENC_CTAS = (1, 2)
-# decoder CTAs per SM; each decoder is clamped to what fits it (5 for 256-segment tiles, 4 for
-# 512-segment ones, 3 for 32 stage rows), and 0 takes that maximum
+# decoder CTAs per SM; each decoder is clamped to what fits it (256-segment tiles 5, for 32 stage rows
+# 3; 512-segment tiles 4, for 16 rows 2; 480-segment tiles 3), and 0 takes that maximum
 DEC_CTAS = (1, 2, 3, 4, 0)
 DEC_TILES = (0, 256, 512)  # decoder tile: the default (0), or 256 / 512 segments
 DEC_SPACE = tuple(itertools.product(DEC_CTAS, DEC_TILES))  # (CTAs per SM, tile) pairs

@@ -281,8 +281,10 @@ typedef struct hgap_batch_config {
     uint32_t enc_ctas_per_sm;
     uint32_t dec_ctas_per_sm;
     uint32_t dec_tile_segs;    /* decoder tile, 256 or 512 segments; 0 = 512, but for books whose
-                                  shortest code has 2 bits 480, and 256 in a batch whose buffers
-                                  average under 64 KiB; books with a 1-bit code always take 256 */
+                                  shortest code has 2 bits 480, and 256 where the workspace is for
+                                  buffers of under 64 KiB on the average (as asked by the query:
+                                  a larger one counts as for larger buffers); books with a 1-bit
+                                  code always take 256 */
     uint32_t dec_class_mask;   /* decoder classes hgap_batch_decompress launches: bit k as
                                   hgap_batch_decoder_class numbers them; 0 = all 8.  For callers
                                   that know their books on the host: an empty class then costs
@@ -306,7 +308,7 @@ uint64_t hgap_batch_gaps_capacity(uint32_t count, const uint64_t* sizes);  /* wo
 /* d_inputs / d_sizes: device arrays of count input pointers and sizes.
  * d_region_chunks: optional device array of per-buffer region sizes (in 8 KiB
  * chunks, raised to cfg->region_chunks at least); NULL = cfg for all.
- * Workspace 16-byte aligned, from hgap_batch_compress_workspace_bytes with
+ * Workspace 256-byte aligned, from hgap_batch_compress_workspace_bytes with
  * the same sizes and cfg. */
 hgap_status hgap_batch_compress(uint32_t count, const uint8_t* const* d_inputs, const uint64_t* d_sizes,
                                 const uint8_t* d_region_chunks, uint32_t* d_bits, uint64_t bits_capacity,
